@@ -462,3 +462,45 @@ def test_host_transfers_from_two_threads_on_one_context():
     for t in ts:
         t.join(300)
     assert not errors, errors
+
+
+def _jumps(n, seed=3):
+    """Lines of 200..9000 values with jumps of up to 2^40, noise widths 0..34 bits and a phase that is no
+    multiple of the partition sizes: candidates of every size win, and residuals pass 32 bits."""
+    rng = np.random.default_rng(seed)
+    v = np.empty(n, np.int64)
+    pos = 0
+    while pos < n:
+        run = min(n - pos, int(rng.integers(200, 9000)))
+        w = int(rng.integers(0, 35))
+        v[pos:pos + run] = int(rng.integers(0, 1 << 40)) + int(rng.integers(0, 5000)) * np.arange(run) + rng.integers(0, 1 << w, run)
+        pos += run
+    return v
+
+
+def _shifted_line(n, seed=3):
+    """One line with a single early jump: the walk from 0 is out of step with every later range's first
+    block, so it leaves the starts that the range walks visit."""
+    v = 7 * np.arange(n, dtype=np.int64) + np.random.default_rng(seed).integers(0, 1 << 10, n)
+    v[5 * 128:] += 1 << 30
+    return v
+
+
+# 8,388,608 values (65,536 blocks) is the longest column whose starts are all evaluated; longer ones walk
+@pytest.mark.parametrize("kind,n", [("jumps", 8_388_608), ("jumps", 8_388_609), ("jumps", 9_000_001), ("shifted", 8_700_000),
+                                    ("i64_ns", 8_500_001), ("i32_linear", 9_000_127), ("i64_negwalk", 8_400_000)])
+def test_variable_partitions_around_the_walk_limit(oracle, glc_ctx, kind, n):
+    v = _jumps(n) if kind == "jumps" else _shifted_line(n) if kind == "shifted" else _data(kind, n, seed=7)
+    ds, de = glc.partition_variable(glc_ctx, v)
+    s, e = oracle.partition_variable(v)
+    assert np.array_equal(ds, s) and np.array_equal(de, e)
+
+
+@pytest.mark.parametrize("n", [127, 128, 129, 3711, 3712, 3713, 29 * 8 * 128 - 1, 29 * 8 * 128, 29 * 8 * 128 + 1, 100_003])
+def test_variable_partitions_of_jumps(oracle, glc_ctx, n):
+    for seed in (3, 4):
+        v = _jumps(n, seed)
+        for w in (v, -v, v.astype(np.uint64), (v & 0x7FFFFFFF).astype(np.int32), (v & 0xFFFFFFFF).astype(np.uint32)):
+            ds, de = glc.partition_variable(glc_ctx, w)
+            s, e = oracle.partition_variable(w)
+            assert np.array_equal(ds, s) and np.array_equal(de, e)
