@@ -281,14 +281,6 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
   c->sync_free = true;
   int32_t* tmp_s = nullptr;
   int32_t* tmp_e = nullptr;
-  long long* part_err = nullptr;  // variable partitions: each partition's max |delta|, measured by the partitioner
-  struct StreamFree {  // returned to the pool after the stream's work so far, on every exit
-    void** p;
-    cudaStream_t s;
-    ~StreamFree() {
-      if (*p) cudaFreeAsync(*p, s);
-    }
-  } part_err_free{reinterpret_cast<void**>(&part_err), s};
   if (mode == GLC_PART_FIXED) {
     c->P = (n + fixed_len - 1) / fixed_len;
     c->fixed_len = fixed_len;
@@ -299,14 +291,16 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
     c->P = P;
     c->fixed_len = 0;
   } else {
-    std::string perr;
-    int64_t P = 0;
-    cudaError_t e = launch_partition_variable(ctx, dtype, dev_values, n, &tmp_s, &tmp_e, &P, s, &perr, &part_err);
-    if (e != cudaSuccess) return perr.empty() ? cuda_fail(ctx, e, "variable partitioner") : fail(ctx, GLC_ERR_CUDA, perr);
-    c->P = P;
     c->fixed_len = 0;
+    std::string perr;
+    PartOut po;  // the partitions come fitted
+    po.column = c;
+    po.alloc = alloc_meta;
+    po.stats = ctx->d_stats;
+    cudaError_t e = launch_partition_variable(ctx, dtype, dev_values, n, po, s, &perr);
+    if (e != cudaSuccess) return perr.empty() ? cuda_fail(ctx, e, "variable partitioner") : fail(ctx, GLC_ERR_CUDA, perr);
   }
-  CK(alloc_meta(c, s), "compress: metadata allocation");
+  if (mode != GLC_PART_VARIABLE) CK(alloc_meta(c, s), "compress: metadata allocation");
   if (mode == GLC_PART_FIXED && fixed_compress_supported(n, fixed_len)) {
     // one read of the values: fit, widths and words of every tile (into scratch slots), a scan of
     // the tiles' bits; then, with the total known, the words placed into an exact-size array
@@ -334,18 +328,21 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
   }
   if (mode == GLC_PART_FIXED) {
     CK(launch_fixed_partitions(c->d_start, c->d_end, n, fixed_len, c->P, s), "compress: fixed partitions");
-  } else {
+  } else if (mode == GLC_PART_VARIABLE_V6) {
     CK(cudaMemcpyAsync(c->d_start, tmp_s, 4 * c->P, cudaMemcpyDeviceToDevice, s), "compress: partition copy");
     CK(cudaMemcpyAsync(c->d_end, tmp_e, 4 * c->P, cudaMemcpyDeviceToDevice, s), "compress: partition copy");
     cudaFreeAsync(tmp_s, s);
     cudaFreeAsync(tmp_e, s);
   }
-  const size_t sb = fit_scratch_bytes(nullptr, n, c->P);
-  void* scratch = nullptr;
-  CK(pool_alloc(ctx, &scratch, sb, s), "compress: scratch allocation");
-  cudaError_t e = launch_fit(dtype, dev_values, c, scratch, sb, ctx->d_stats, s, part_err);
+  cudaError_t e = cudaSuccess;
+  if (mode != GLC_PART_VARIABLE) {
+    const size_t sb = fit_scratch_bytes(nullptr, n, c->P);
+    void* scratch = nullptr;
+    CK(pool_alloc(ctx, &scratch, sb, s), "compress: scratch allocation");
+    e = launch_fit(dtype, dev_values, c, scratch, sb, ctx->d_stats, s);
+    cudaFreeAsync(scratch, s);
+  }
   if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-  cudaFreeAsync(scratch, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "compress: fit");
   if (ctx->h_stats[2] != DEVERR_NONE) return fail(ctx, GLC_ERR_TIMEOUT, "compress: a device-side wait of the fit gave up");
@@ -444,8 +441,12 @@ static glc_status partition_only(glc_ctx* ctx, glc_dtype dtype, const void* valu
   int64_t P = 0;
   std::string perr;
   std::unique_lock<std::mutex> stats_lock(ctx->stats_mu);  // partition counts come back through h_stats
+  PartOut po;
+  po.starts = &ds;
+  po.ends = &de;
+  po.P = &P;
   cudaError_t e = v6_base > 0 ? launch_partition_v6(ctx, dtype, dev_values, n, v6_base, &ds, &de, &P, s)
-                              : launch_partition_variable(ctx, dtype, dev_values, n, &ds, &de, &P, s, &perr);
+                              : launch_partition_variable(ctx, dtype, dev_values, n, po, s, &perr);
   if (staged) cudaFreeAsync(staged, s);
   if (e != cudaSuccess) return perr.empty() ? cuda_fail(ctx, e, "partition") : fail(ctx, GLC_ERR_CUDA, perr);
   *num_partitions = P;

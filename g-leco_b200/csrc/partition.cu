@@ -20,10 +20,9 @@
 // second pass over the values.
 //
 // Merge.  The reference absorbs right neighbours left to right while the merged cost is lower
-// (CpuPartitioner.cuh:198-242).  Here merging runs in rounds: every adjacent pair is scored,
-// and the profitable pairs with (index + round) even merge, so the chosen pairs never overlap;
-// rounds stop when no pair is profitable (at most 64 rounds).  A pair whose two partitions did
-// not change keeps its score from the previous round.
+// (CpuPartitioner.cuh:198-242).  Here merging runs in rounds: the profitable adjacent pairs
+// with (index + round) even merge, so the chosen pairs never overlap; rounds stop when no pair is
+// profitable (at most 64 rounds).
 //
 // Fits use exact 128-bit sums from a prefix over 128-value blocks (every boundary here is a
 // multiple of 128 or n), so each candidate's line costs O(1) and only its max |delta| needs a
@@ -49,8 +48,6 @@ constexpr int kWalksPerSM = 7;  // range walks (one warp each) whose reaches fit
 // its longest chain: 3M timestamps took 3070 us of walks of 2048 blocks and take 141 us this way;
 // 200M values would take 26 times the evaluations of the walks.
 constexpr int64_t kAllStartsBlocks = 65536;
-constexpr int kMaxMergeRounds = 64;
-constexpr int kPairChunk = 4096;
 constexpr int32_t kUnknown = -1;  // best end of a start not evaluated
 
 struct SumPair {  // trivially constructible: SumPair() value-initialises to zero
@@ -65,27 +62,40 @@ struct SumPair {  // trivially constructible: SumPair() value-initialises to zer
 };
 
 // ---- block sums -----------------------------------------------------------------------
-template <typename T> __global__ void block_sums_kernel(const T* __restrict__ v, int64_t n, int64_t nb, SumPair* __restrict__ out) {
-  const int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (j >= nb) return;
-  i128 sy = 0, siy = 0;
+// Eight lanes per block, 16 values each (all loads in flight before the sums), from 64-bit partials of
+// the values' halves with the index inside the block.  ovf (uint64 only): the block holds a value
+// above 2^53, so its partition is copied.
+template <typename T> __global__ void __launch_bounds__(256)
+block_sums_kernel(const T* __restrict__ v, int64_t n, int64_t nb, SumPair* __restrict__ out, uint8_t* __restrict__ ovf) {
+  const int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const int l = threadIdx.x & 7;
+  const int64_t i0 = j * kMinPart;
+  T y[16];
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int64_t i = j * kMinPart + k * 32 + lane;
-    if (i < n) {
-      const i128 y = (i128)__ldg(v + i);
-      sy += y;
-      siy += (i128)i * y;
+  for (int k = 0; k < 16; k++) y[k] = i0 + 8 * k + l < n ? __ldg(v + i0 + 8 * k + l) : (T)0;
+  HalfSums<T> h;
+  bool over = false;
+#pragma unroll
+  for (int k = 0; k < 16; k++) {
+    h.add(y[k], 8 * k + l);
+    over |= overflows_double<T>(y[k]);
+  }
+#pragma unroll
+  for (int m = 4; m > 0; m >>= 1) {  // (a block's sums of halves and of index * half stay inside 64 bits)
+    h.s_lo += __shfl_xor_sync(FULL_MASK, h.s_lo, m);
+    h.x_lo += __shfl_xor_sync(FULL_MASK, h.x_lo, m);
+    if (sizeof(T) == 8) {
+      h.s_hi += __shfl_xor_sync(FULL_MASK, h.s_hi, m);
+      h.x_hi += __shfl_xor_sync(FULL_MASK, h.x_hi, m);
     }
   }
-  sy = warp_sum_i128(sy);
-  siy = warp_sum_i128(siy);
-  if (lane == 0) {
+  const unsigned any = __ballot_sync(FULL_MASK, over);
+  if (l == 0 && j < nb) {
     SumPair s;
-    s.y = sy;
-    s.iy = siy;
+    s.y = h.sy();
+    s.iy = h.sxy() + (i128)i0 * s.y;
     out[j] = s;
+    if (!TypeTraits<T>::is_signed && sizeof(T) == 8) ovf[j] = ((any >> (threadIdx.x & 24)) & 0xffu) != 0;
   }
 }
 
@@ -159,8 +169,9 @@ __device__ __forceinline__ uint32_t high_bits(long long y) {
 //   kExact   the format's saturating integer arithmetic.
 enum : int { kNonNeg = 0, kOffset = 1, kSigned = 2, kExact = 3 };
 
-template <typename T> __device__ __forceinline__ int line_form(double t0, double t1, int len, double& d) {
-  const double xa = __fma_rn(t1, 0.0, t0), xb = __fma_rn(t1, (double)(len - 1), t0);  // monotone between
+// (over offsets [o0, o1]: the prediction argument is monotone between them)
+template <typename T> __device__ __forceinline__ int line_form(double t0, double t1, int64_t o0, int64_t o1, double& d) {
+  const double xa = __fma_rn(t1, (double)o0, t0), xb = __fma_rn(t1, (double)o1, t0);
   d = 0.0;
   if (pred_fp64_safe<T>(xa) && pred_fp64_safe<T>(xb)) return xa >= -0.25 && xb >= -0.25 ? kNonNeg : kSigned;
   if constexpr (sizeof(T) == 8) {
@@ -257,7 +268,7 @@ template <typename T, bool SMEM, bool LIMITED>
 __device__ __forceinline__ long long scan_line(const T* __restrict__ vs, int len, double t0, double t1, long long lim,
                                                int lane) {
   double d;
-  const int form = line_form<T>(t0, t1, len, d);
+  const int form = line_form<T>(t0, t1, 0, len - 1, d);
   if ((form == kNonNeg || (sizeof(T) == 8 && form == kOffset)) && (!LIMITED || lim < 0x7fffffffll)) {
     bool fits;
     const uint32_t m = form == kNonNeg
@@ -616,175 +627,436 @@ chain_emit_kernel(const int32_t* __restrict__ nb_next, const long long* __restri
   }
 }
 
-// ---- costs of partitions ---------------------------------------------------------------
-struct LineJob {  // one range whose max |delta| is needed
-  int32_t a, b;
-  double t0, t1;
-  double sum;  // pairs: the two partitions' costs (a merge must cost less); partitions: +inf
-};
-
-// chunks of each job (0 for jobs that are cached)
-// known (partitions only): a max |delta| already measured (the split evaluation of the
-// partition's start, same line and values), or -1.  A pair kept from the previous round (cached)
-// keeps its max |delta| too (cached_err).
-__global__ void job_setup_kernel(const int32_t* __restrict__ ps, const int32_t* __restrict__ pe, int64_t m, int pairs,
-                                 const uint8_t* __restrict__ cached, const long long* __restrict__ cached_err,
-                                 const long long* __restrict__ known, const double* __restrict__ pc, RangeSums rs,
-                                 LineJob* __restrict__ jobs, int64_t* __restrict__ nch, long long* __restrict__ err) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t njobs = pairs ? m - 1 : m;
-  if (k >= njobs) return;
-  LineJob jb;
-  jb.a = ps[k];
-  jb.b = pairs ? pe[k + 1] : pe[k];
-  rs.line(jb.a, jb.b, jb.t0, jb.t1);
-  jb.sum = pairs ? __dadd_rn(pc[k], pc[k + 1]) : __longlong_as_double(0x7ff0000000000000ll);
-  jobs[k] = jb;
-  const long long kn = known ? known[k] : -1;
-  const bool kept = cached && cached[k];
-  err[k] = kn >= 0 ? kn : (kept ? cached_err[k] : 0);
-  const bool skip = kept || kn >= 0;
-  nch[k] = skip ? 0 : ((int64_t)jb.b - jb.a + kPairChunk - 1) / kPairChunk;
+// ---- merge rounds ------------------------------------------------------------------------
+// Max |residual| of the line over offsets [o0, o1) of the values at vs, by one warp (every lane returns
+// it); above lim it only says so.  Any length; eight loads per lane in flight.
+template <typename T, int FORM>
+__device__ __forceinline__ uint32_t range_narrow(const T* __restrict__ vs, int64_t o0, int64_t o1, double t0, double t1,
+                                                 double d, uint32_t lim, int lane, bool& fits) {
+  constexpr long long kHalf = 1ll << 31;
+  constexpr int kDeep = 16;
+  const long long add = kMagicBits + kHalf - (FORM == kOffset ? (long long)d : 0);
+  uint32_t mx = (uint32_t)kHalf, mn = (uint32_t)kHalf, wide = 0;
+  double od = (double)(o0 + lane);
+  auto take = [&](T y, double o) {  // as in scan_narrow
+    const double x = __fma_rn(t1, o, t0);
+    const double m = FORM == kNonNeg ? __dadd_rz(__dadd_rn(x, 0x1.fffffffffffffp-2), kMagic)
+                                     : __dadd_rd(__dadd_rn(__dsub_rn(x, d), 0.5), kMagic);
+    const unsigned long long r = (unsigned long long)(long long)y - (unsigned long long)__double_as_longlong(m) +
+                                 (unsigned long long)add;
+    wide |= (uint32_t)(r >> 32);
+    mx = max(mx, (uint32_t)r);
+    mn = min(mn, (uint32_t)r);
+  };
+  const T* p = vs + o0 + lane;
+  int64_t left = o1 - o0;
+  for (; left >= 32 * kDeep; left -= 32 * kDeep, p += 32 * kDeep) {
+    T y[kDeep];
+#pragma unroll
+    for (int u = 0; u < kDeep; u++) y[u] = __ldg(p + 32 * u);
+#pragma unroll
+    for (int u = 0; u < kDeep; u++, od = __dadd_rn(od, 32.0)) take(y[u], od);
+    if (__any_sync(FULL_MASK, max(mx - (uint32_t)kHalf, (uint32_t)kHalf - mn) > lim || wide != 0)) {
+      left = 0;
+      break;
+    }
+  }
+  for (int64_t o = lane; o < left; o += 32, p += 32, od = __dadd_rn(od, 32.0)) take(__ldg(p), od);
+  fits = !__any_sync(FULL_MASK, wide != 0);
+  return __reduce_max_sync(FULL_MASK, max(mx - (uint32_t)kHalf, (uint32_t)kHalf - mn));
 }
 
-// Max |delta| of a job's line over chunk q of the job (256 threads, no CTA barrier: warps may
-// skip a chunk independently), folded into *errk by each warp.
+// The same in the format's own arithmetic, or in FP64 where every quantity is an exact integer.
 template <typename T>
-__device__ __forceinline__ void job_chunk(const T* __restrict__ v, const LineJob& jb, int64_t q, long long* errk) {
-  const int64_t off0 = q * kPairChunk;
-  const int64_t len = (int64_t)jb.b - jb.a;
-  const int64_t off1 = off0 + kPairChunk < len ? off0 + kPairChunk : len;
-  long long mm = 0;
-  bool exact = true;
-  if (off1 > off0 && line_fp64_safe<T>(jb.t0, jb.t1, off0, off1 - 1)) {  // exact in FP64 (glc_device.cuh)
-    static_assert(kPairChunk == 16 * 256, "16 values per thread");
-    T ys[16];
-#pragma unroll
-    for (int u = 0; u < 16; u++) {  // all loads in flight before the arithmetic
-      const int64_t o = off0 + threadIdx.x + u * 256;
-      ys[u] = o < off1 ? __ldg(v + jb.a + o) : (T)0;
-    }
-    double md = 0.0;
-    bool ok = true;
-#pragma unroll
-    for (int u = 0; u < 16; u++) {
-      const int64_t o = off0 + threadIdx.x + u * 256;
-      if (o < off1) {
-        ok &= value_fp64_safe<T>(ys[u]);
-        md = fmax(md, abs_resid_fp64((double)(long long)ys[u], __fma_rn(jb.t1, (double)o, jb.t0)));
+__device__ __noinline__ long long range_exact(const T* __restrict__ vs, int64_t o0, int64_t o1, double t0, double t1,
+                                              long long lim, int lane) {
+  long long m = 0;
+  for (int64_t b = o0; b < o1; b += 256) {
+    const int64_t e = b + 256 < o1 ? b + 256 : o1;
+    if (line_fp64_safe<T>(t0, t1, b, e - 1)) {
+      double md = 0.0;
+      bool ok = true;
+      for (int64_t o = b + lane; o < e; o += 32) {
+        const T y = __ldg(vs + o);
+        ok &= value_fp64_safe<T>(y);
+        md = fmax(md, abs_resid_fp64((double)(long long)y, __fma_rn(t1, (double)o, t0)));
+      }
+      if (__all_sync(FULL_MASK, ok)) {
+        m = max(m, (long long)md);
+        if (__any_sync(FULL_MASK, m > lim)) break;
+        continue;
       }
     }
-    if (ok) {  // this thread's values were all inside the exact range
-      mm = (long long)md;
-      exact = false;
-    }
+    for (int64_t o = b + lane; o < e; o += 32)
+      m = max(m, abs_ref(calc_delta<T>(__ldg(vs + o), predict<T>(t0, t1, o))));
+    if (__any_sync(FULL_MASK, m > lim)) break;
   }
-  if (exact)
-    for (int64_t o = off0 + threadIdx.x; o < off1; o += 256) {
-      const long long d = abs_ref(calc_delta<T>(__ldg(v + jb.a + o), predict<T>(jb.t0, jb.t1, o)));
-      mm = d > mm ? d : mm;
-    }
-  mm = warp_max_ll(mm);
-  if ((threadIdx.x & 31) == 0 && mm > 0) atomicMax(errk, mm);
+  return warp_max_ll(m);
 }
 
-// A pair whose partial max |delta| already makes the merge cost at least the two partitions'
-// costs is not merged whatever the rest of it holds (the score stays unprofitable, also when it
-// is kept for the next round), so its remaining chunks are skipped.  One warp decides.
-__device__ __forceinline__ bool job_settled(const LineJob& jb, const long long* errk) {
-  long long e = 0;
-  if ((threadIdx.x & 31) == 0) e = *(const volatile long long*)errk;
-  e = __shfl_sync(FULL_MASK, e, 0);
-  return !(part_cost((int64_t)jb.b - jb.a, bits_for(e)) < jb.sum);
+template <typename T>
+__device__ __forceinline__ long long range_line(const T* __restrict__ vs, int64_t o0, int64_t o1, double t0, double t1,
+                                                long long lim, int lane) {
+  double d;
+  const int form = line_form<T>(t0, t1, o0, o1 - 1, d);
+  if (form == kNonNeg || (sizeof(T) == 8 && form == kOffset)) {
+    bool fits;
+    const uint32_t l32 = lim < 0x7fffffffll ? (uint32_t)lim : 0x7fffffffu;
+    const uint32_t m = form == kNonNeg ? range_narrow<T, kNonNeg>(vs, o0, o1, t0, t1, d, l32, lane, fits)
+                                       : range_narrow<T, kOffset>(vs, o0, o1, t0, t1, d, l32, lane, fits);
+    if (fits && m <= 0x7fffffffu) return (long long)m;
+    if (lim < 0x7fffffffll) return lim + 1;
+  }
+  return range_exact<T>(vs, o0, o1, t0, t1, lim, lane);
 }
 
-// Max |delta| of every job still to measure: persistent CTAs, one job at a time, its chunks in
-// order (each warp stops at the first chunk after which the pair is settled).
-template <typename T> __global__ void __launch_bounds__(256, 4)
-job_err_kernel(const T* __restrict__ v, const LineJob* __restrict__ jobs, const int64_t* __restrict__ nch,
-               int64_t njobs, long long* __restrict__ err) {
-  for (int64_t k = blockIdx.x; k < njobs; k += gridDim.x) {
-    const int64_t nc = nch[k];  // 0: kept from the previous round
-    if (nc == 0) continue;
-    const LineJob jb = jobs[k];
-    for (int64_t q = 0; q < nc; q++) {
-      if (q > 0 && job_settled(jb, err + k)) break;
-      job_chunk<T>(v, jb, q, err + k);
+// The largest max |delta| with which a partition of len values costs less than `sum` (-1: none).
+__device__ __forceinline__ long long err_below_cost(int64_t len, double sum) {
+  int b = 64;
+  const double est = (sum - kModelBytes) * 8.0 / (double)len;  // real number of bits at equality
+  if (est < 64.0) b = est < 0.0 ? 0 : (int)est + 1;
+  while (b >= 0 && !(part_cost(len, b) < sum)) b--;
+  return b < 0 ? -1 : b < 2 ? 0 : b >= 64 ? 0x7fffffffffffffffll : (1ll << (b - 1)) - 1;
+}
+
+// One version of the partition list.
+struct PartList {
+  int32_t* start;
+  int32_t* end;
+  double* cost;
+  long long* err;     // max |delta| of the partition's line, bit 63 set when a value is above 2^53
+  uint8_t* rejected;  // the pair (this, next) was scored and is not worth merging
+};
+constexpr long long kOverflowBit = (long long)0x8000000000000000ull;
+
+struct MergeArgs {
+  PartList a, b;         // a holds the split's partitions (cost and rejected not set)
+  const uint8_t* ovf;    // per block (uint64)
+  int64_t n;
+  int32_t m;             // partitions in a
+  int32_t unit;          // values of a pair that one warp scans
+  uint8_t* selected;     // pair (k, k + 1) merges this round
+  long long* pair_err;
+  double* pair_t;        // line of a pair in the unit queue
+  long long* pair_lim;
+  uint2* queue;          // (left part, unit) of pairs longer than one unit
+  int32_t* cta_heads;    // per CTA
+  unsigned* counters;    // kMergeCounters, zero
+  int64_t* out;          // [0] partitions left, [1] 1 when they are in b, [2] DEVERR_*
+};
+constexpr int kMaxMergeRounds = 64;
+constexpr int kMergeThreads = 512;
+constexpr int kMergeUnitMost = 4096;  // values of a pair that one warp scans, at most
+// counters: [0] grid barrier, then per round: pairs taken, queue length, pairs rejected
+constexpr int kMergeCounters = 4 + 4 * kMaxMergeRounds;
+
+// Barrier of all CTAs of a cooperative launch (a counter that only grows); false when the bounded wait
+// gave up.
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned& arrived, int64_t* status) {
+  __shared__ int s_ok;
+  __syncthreads();
+  arrived += gridDim.x;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(bar, 1u);
+    long long spins = 0;
+    unsigned seen;
+    do {
+      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+    } while ((int)(seen - arrived) < 0 && ++spins < kSpinLimit);
+    s_ok = (int)(seen - arrived) >= 0;
+    if (!s_ok) atomicExch((unsigned long long*)status, (unsigned long long)DEVERR_TIMEOUT);
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// All merge rounds in one cooperative launch (one CTA per SM; nine launches and a host round trip per
+// round before: 15 rounds on 200M piecewise values).  In round r the pairs (k, k + 1) with k + r even
+// can merge, so only those are scored, every value read once per round (scoring all pairs read it
+// twice).  A pair that is not worth merging stays so until one of its partitions changes (rejected).
+// A warp scores a pair: lines of up to eight pairs at once by its lanes, 32 spread residuals, then the
+// values in order until one residual is above what the merge allows.  Pairs longer than a unit put
+// their further units in a queue that all warps empty together after the others.
+//
+// 200M piecewise uint64 values: 3343 us of error passes and ~450 us of bookkeeping launches -> 1320 us;
+// 3M int64 timestamps: 57 + ~170 -> 120 us.  Bound by the values read (about four passes at 5 TB/s) and,
+// on short columns, by the barriers.  Units of 32,768 values measured 1829 us (the last warps of a
+// round scan alone), 8192: 1420, 4096: 1346; 1024 threads with eight loads in flight per lane 1925
+// (64 registers: spills).
+template <typename T> __global__ void __launch_bounds__(kMergeThreads)
+merge_kernel(const T* __restrict__ v, RangeSums rs, MergeArgs a) {
+  __shared__ int32_t s_scan[kMergeThreads / 32];
+  __shared__ int32_t s_base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t tid = (int64_t)blockIdx.x * kMergeThreads + threadIdx.x, nthreads = (int64_t)gridDim.x * kMergeThreads;
+  const int nwarps = (int)(nthreads >> 5), gwarp = (int)(tid >> 5);
+  unsigned arrived = 0;
+  PartList cur = a.a, nxt = a.b;
+  int m = a.m;
+  // costs of the split's partitions: their max |delta| came with the split (-1: fewer than 128 values)
+  for (int64_t k = tid; k < m; k += nthreads) {
+    const int64_t s = cur.start[k], e = cur.end[k];
+    long long err = cur.err[k];
+    if (err < 0) {
+      double t0, t1;
+      rs.line(s, e, t0, t1);
+      err = 0;
+      for (int64_t o = 0; o < e - s; o++) err = max(err, abs_ref(calc_delta<T>(v[s + o], predict<T>(t0, t1, o))));
     }
+    cur.cost[k] = part_cost(e - s, bits_for(err));
+    cur.rejected[k] = 0;
+    if (!TypeTraits<T>::is_signed && sizeof(T) == 8) {
+      bool over = false;
+      for (int64_t b = s / kMinPart; b * kMinPart < e; b++) over |= a.ovf[b] != 0;
+      if (over) err |= kOverflowBit;
+    }
+    cur.err[k] = err;
+  }
+  if (!grid_barrier(a.counters, arrived, a.out + 2)) return;
+  bool flipped = false;
+  for (int round = 0; round < kMaxMergeRounds && m >= 2; round++) {
+    unsigned* taken = a.counters + 4 + 4 * round;
+    unsigned* queued = taken + 1;
+    unsigned* nrej = taken + 2;
+    const int odd = round & 1, pairs = (m - odd) / 2;  // k = 2 q + odd, k + 1 < m
+    // ---- score ----
+    int per = pairs / (nwarps * 8);
+    per = per < 1 ? 1 : per > 4 ? 4 : per;
+    for (;;) {
+      unsigned q0 = lane == 0 ? atomicAdd(taken, (unsigned)per) : 0u;
+      q0 = __shfl_sync(FULL_MASK, q0, 0);
+      if (q0 >= (unsigned)pairs) break;
+      const int mine = (int)q0 + lane;
+      const bool have = lane < per && mine < pairs;
+      const int kk = 2 * mine + odd;
+      int64_t s = 0, e = 0;
+      double t0 = 0.0, t1 = 0.0;
+      long long lim = -1;
+      bool todo = false;
+      if (have) {
+        a.selected[kk] = 0;
+        todo = cur.rejected[kk] == 0;
+        if (todo) {
+          s = cur.start[kk];
+          e = cur.end[kk + 1];
+          rs.line(s, e, t0, t1);
+          lim = err_below_cost(e - s, __dadd_rn(cur.cost[kk], cur.cost[kk + 1]));
+          if (lim < 0) {
+            cur.rejected[kk] = 1;
+            todo = false;
+          }
+        }
+      }
+      unsigned work = __ballot_sync(FULL_MASK, todo);
+      while (work) {
+        const int src = __ffs((int)work) - 1;
+        work &= work - 1;
+        const int k = __shfl_sync(FULL_MASK, kk, src);
+        const int64_t ps = __shfl_sync(FULL_MASK, s, src), len = __shfl_sync(FULL_MASK, e, src) - ps;
+        const double u0 = __shfl_sync(FULL_MASK, t0, src), u1 = __shfl_sync(FULL_MASK, t1, src);
+        const long long lk = __shfl_sync(FULL_MASK, lim, src);
+        const T* vs = v + ps;
+        const int64_t o = len >= 64 ? lane * (len >> 5) + (len >> 6) : lane < len ? lane : 0;
+        long long err = warp_max_ll(abs_ref(calc_delta<T>(__ldg(vs + o), predict<T>(u0, u1, o))));
+        const bool longer = len > a.unit;
+        if (err <= lk) err = range_line<T>(vs, 0, longer ? a.unit : len, u0, u1, lk, lane);
+        if (longer && err <= lk) {  // the rest of it by all warps
+          const unsigned units = (unsigned)((len + a.unit - 1) / a.unit) - 1;
+          unsigned at = lane == 0 ? atomicAdd(queued, units) : 0u;
+          at = __shfl_sync(FULL_MASK, at, 0);
+          for (unsigned u = lane; u < units; u += 32) a.queue[at + u] = make_uint2((unsigned)k, u + 1);
+          if (lane == 0) {
+            a.pair_t[2 * k] = u0;
+            a.pair_t[2 * k + 1] = u1;
+            a.pair_lim[k] = lk;
+          }
+        }
+        if (lane == 0) {
+          a.pair_err[k] = err;
+          const bool merge = err <= lk;
+          a.selected[k] = merge;
+          if (!merge) cur.rejected[k] = 1;
+        }
+      }
+    }
+    if (!grid_barrier(a.counters, arrived, a.out + 2)) return;
+    const unsigned nq = *(volatile unsigned*)queued;
+    if (nq) {
+      for (unsigned i = gwarp; i < nq; i += nwarps) {
+        const uint2 w = a.queue[i];
+        const int k = (int)w.x;
+        const long long lk = a.pair_lim[k];
+        long long seen = lane == 0 ? *(volatile long long*)(a.pair_err + k) : 0;
+        if (__shfl_sync(FULL_MASK, seen, 0) > lk) continue;  // settled by another unit
+        const int64_t ps = cur.start[k], len = cur.end[k + 1] - ps;
+        const int64_t o0 = (int64_t)w.y * a.unit, o1 = o0 + a.unit < len ? o0 + a.unit : len;
+        const long long err = range_line<T>(v + ps, o0, o1, a.pair_t[2 * k], a.pair_t[2 * k + 1], lk, lane);
+        if (lane == 0) {
+          atomicMax(a.pair_err + k, err);
+          if (err > lk) {
+            a.selected[k] = 0;
+            cur.rejected[k] = 1;
+          }
+        }
+      }
+      if (!grid_barrier(a.counters, arrived, a.out + 2)) return;
+    }
+    // ---- compact: a CTA takes a stretch of the list ----
+    const int seg = (m + gridDim.x - 1) / gridDim.x, k0 = min(m, (int)blockIdx.x * seg), k1 = min(m, k0 + seg);
+    auto merges = [&](int k) { return k >= odd && ((k + round) & 1) == 0 && k + 1 < m && a.selected[k]; };
+    int heads = 0;
+    for (int k = k0 + threadIdx.x; k < k1; k += kMergeThreads) heads += !merges(k - 1);
+    heads = __reduce_add_sync(FULL_MASK, heads);
+    if (lane == 0) s_scan[warp] = heads;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int t = 0;
+      for (int w = 0; w < kMergeThreads / 32; w++) t += s_scan[w];
+      a.cta_heads[blockIdx.x] = t;
+    }
+    if (!grid_barrier(a.counters, arrived, a.out + 2)) return;
+    // heads before this CTA, and all of them
+    int before = 0, all = 0;
+    for (int c = threadIdx.x; c < (int)gridDim.x; c += kMergeThreads) {
+      const int h = *(volatile int32_t*)(a.cta_heads + c);
+      all += h;
+      if (c < (int)blockIdx.x) before += h;
+    }
+    before = __reduce_add_sync(FULL_MASK, before);
+    all = __reduce_add_sync(FULL_MASK, all);
+    __shared__ int32_t s_before[kMergeThreads / 32], s_all[kMergeThreads / 32];
+    if (lane == 0) {
+      s_before[warp] = before;
+      s_all[warp] = all;
+    }
+    __syncthreads();
+    before = all = 0;
+    for (int w = 0; w < kMergeThreads / 32; w++) {
+      before += s_before[w];
+      all += s_all[w];
+    }
+    if (threadIdx.x == 0) s_base = before;
+    int rej = 0;
+    for (int kb = k0; kb < k1; kb += kMergeThreads) {
+      const int k = kb + (int)threadIdx.x;
+      const bool head = k < k1 && !merges(k - 1);
+      const unsigned bal = __ballot_sync(FULL_MASK, head);
+      __syncthreads();  // s_base set; the last step's s_scan read
+      if (lane == 0) s_scan[warp] = __popc(bal);
+      __syncthreads();
+      int d = s_base + __popc(bal & ((1u << lane) - 1u)), total = 0;
+      for (int w = 0; w < kMergeThreads / 32; w++) {
+        const int c = s_scan[w];
+        d += w < warp ? c : 0;
+        total += c;
+      }
+      if (head) {
+        const bool sel = merges(k);
+        nxt.start[d] = cur.start[k];
+        const int32_t end = cur.end[sel ? k + 1 : k];
+        nxt.end[d] = end;
+        long long err = cur.err[k];
+        double cost = cur.cost[k];
+        if (sel) {
+          const long long pe = a.pair_err[k];
+          cost = part_cost((int64_t)end - cur.start[k], bits_for(pe));
+          err = pe | ((err | cur.err[k + 1]) & kOverflowBit);
+        }
+        nxt.err[d] = err;
+        nxt.cost[d] = cost;
+        const bool r = !sel && k + 1 < m && cur.rejected[k] && !merges(k + 1);
+        nxt.rejected[d] = r;
+        rej += r;
+      }
+      __syncthreads();  // everyone has read s_base and s_scan
+      if (threadIdx.x == 0) s_base += total;
+    }
+    rej = __reduce_add_sync(FULL_MASK, rej);
+    if (lane == 0 && rej) atomicAdd(nrej, (unsigned)rej);
+    if (!grid_barrier(a.counters, arrived, a.out + 2)) return;
+    const PartList t = cur;
+    cur = nxt;
+    nxt = t;
+    flipped = !flipped;
+    m = all;
+    if (*(volatile unsigned*)nrej == (unsigned)(m - 1)) break;  // no pair is worth merging
+  }
+  if (tid == 0) {
+    a.out[0] = m;
+    a.out[1] = flipped;
   }
 }
 
-// Initial part costs.
-__global__ void part_cost_kernel(const LineJob* __restrict__ jobs, const long long* __restrict__ err, int64_t m,
-                                 double* __restrict__ pc) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m) return;
-  pc[k] = part_cost((int64_t)jobs[k].b - jobs[k].a, bits_for(err[k]));
-}
-
-// Pair scores: merged cost (fresh or cached) and profitability; any profitable -> *any = 1.
-__global__ void pair_score_kernel(const LineJob* __restrict__ jobs, const long long* __restrict__ err,
-                                  const uint8_t* __restrict__ cached, const double* __restrict__ cached_mc,
-                                  const double* __restrict__ pc, int64_t m, double* __restrict__ mc,
-                                  uint8_t* __restrict__ prof, int* __restrict__ any) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m - 1) return;
-  double c;
-  if (cached && cached[k]) c = cached_mc[k];
-  else c = part_cost((int64_t)jobs[k].b - jobs[k].a, bits_for(err[k]));
-  mc[k] = c;
-  const bool p = c < __dadd_rn(pc[k], pc[k + 1]);
-  prof[k] = p ? 1 : 0;
-  if (p) atomicOr(any, 1);
-}
-
-// heads: part k starts a new part unless pair k-1 merges.
-__global__ void merge_heads_kernel(const uint8_t* __restrict__ prof, int64_t m, int round, int64_t* __restrict__ head) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m) return;
-  const bool absorbed = k > 0 && prof[k - 1] && (((k - 1) + round) % 2 == 0);
-  head[k] = absorbed ? 0 : 1;
-}
-
-__device__ __forceinline__ bool selected(const uint8_t* prof, int64_t m, int64_t k, int round) {
-  return k >= 0 && k < m - 1 && prof[k] && ((k + round) % 2 == 0);
-}
-
-__global__ void merge_scatter_kernel(const int32_t* __restrict__ ps, const int32_t* __restrict__ pe,
-                                     const double* __restrict__ pc, const double* __restrict__ mc,
-                                     const uint8_t* __restrict__ prof, const int64_t* __restrict__ head,
-                                     const int64_t* __restrict__ idx, int64_t m, int round,
-                                     int32_t* __restrict__ ps2, int32_t* __restrict__ pe2, double* __restrict__ pc2,
-                                     uint8_t* __restrict__ cached2, double* __restrict__ cmc2,
-                                     const long long* __restrict__ pair_err, const long long* __restrict__ part_err,
-                                     long long* __restrict__ part_err2, long long* __restrict__ cerr2) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m || !head[k]) return;
-  const int64_t d = idx[k];
-  const bool sel = selected(prof, m, k, round);
-  ps2[d] = ps[k];
-  pe2[d] = sel ? pe[k + 1] : pe[k];
-  pc2[d] = sel ? mc[k] : pc[k];
-  part_err2[d] = sel ? pair_err[k] : part_err[k];  // a merged pair was measured in full (never settled early)
-  // the score of (this part, next part) survives when neither changed
-  const int64_t nxt = sel ? k + 2 : k + 1;  // old index of the next head
-  const bool keep = !sel && nxt < m && !selected(prof, m, nxt, round);
-  cached2[d] = keep ? 1 : 0;
-  cmc2[d] = keep ? mc[k] : 0.0;
-  cerr2[d] = keep ? pair_err[k] : 0;
+// ---- the fit of the final partitions ----------------------------------------------------------
+// Line, model, max |delta| and width of each partition, all from the partitioner's exact sums and
+// errors: no pass over the values (the fit's own pass took 307 us on 200M values).
+template <typename T> __global__ void __launch_bounds__(128)
+part_fit_kernel(PartList l, RangeSums rs, int32_t P, int32_t* __restrict__ starts, int32_t* __restrict__ ends,
+                int32_t* __restrict__ types, double* __restrict__ params, int32_t* __restrict__ bits,
+                int64_t* __restrict__ errb, int64_t* __restrict__ widths, unsigned long long* __restrict__ max_bits,
+                unsigned long long* __restrict__ per_tile) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  int b = 0;
+  unsigned k = 0;
+  if (p < P) {
+    const int64_t s = l.start[p], e = l.end[p];
+    const bool copy = l.err[p] < 0;
+    double t0 = 0.0, t1 = 0.0;
+    if (!copy) rs.line(s, e, t0, t1);
+    const long long err = copy ? 0 : l.err[p];
+    b = copy ? (int)sizeof(T) * 8 : bits_for(err);
+    starts[p] = (int32_t)s;
+    ends[p] = (int32_t)e;
+    types[p] = copy ? MODEL_DIRECT_COPY : MODEL_LINEAR;
+    double2* q = reinterpret_cast<double2*>(params + 4 * (int64_t)p);
+    q[0] = make_double2(t0, t1);
+    q[1] = make_double2(0.0, 0.0);
+    bits[p] = b;
+    errb[p] = err;
+    widths[p] = (e - s) * b;
+    if (p < P - 1) k = (unsigned)((kDecodeTile + e - s - 1) / (e - s));
+  }
+  b = (int)__reduce_max_sync(FULL_MASK, (unsigned)b);
+  k = __reduce_max_sync(FULL_MASK, k);
+  if ((threadIdx.x & 31) == 0) {
+    if (b > 0) atomicMax(max_bits, (unsigned long long)b);
+    if (k > 0) atomicMax(per_tile, (unsigned long long)k);
+  }
 }
 
 static inline size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// Two allocations: the split's arrays by the column's blocks, the lists by the partitions it made.
+struct PoolBuf {
+  cudaStream_t s;
+  char* p = nullptr;
+  size_t used = 0;
+  explicit PoolBuf(cudaStream_t st) : s(st) {}
+  ~PoolBuf() {
+    if (p) cudaFreeAsync(p, s);
+  }
+  template <typename V> void want(V** at, size_t count) { fields.push_back({(void**)at, al(sizeof(V) * count)}); }
+  cudaError_t get(glc_ctx* ctx) {
+    for (auto& f : fields) used += f.second;
+    cudaError_t e = pool_alloc(ctx, &p, used, s);
+    if (e != cudaSuccess) {
+      p = nullptr;
+      return e;
+    }
+    char* q = p;
+    for (auto& f : fields) {
+      *f.first = q;
+      q += f.second;
+    }
+    return cudaSuccess;
+  }
+  std::vector<std::pair<void**, size_t>> fields;
+};
+
 template <typename T>
-static cudaError_t partition_typed(glc_ctx* ctx, const T* v, int64_t n, int32_t** out_s, int32_t** out_e, int64_t* outP,
-                                   cudaStream_t s, std::string* err, long long** out_err) {
+static cudaError_t partition_typed(glc_ctx* ctx, const T* v, int64_t n, const PartOut& out, cudaStream_t s, std::string* err) {
   cudaError_t e;
-  *out_s = nullptr;
-  *out_e = nullptr;
-  *outP = 0;
-  if (out_err) *out_err = nullptr;
-  if (n <= 0) return cudaSuccess;
   const int64_t nb = (n + kMinPart - 1) / kMinPart;
   const bool all_starts = nb <= kAllStartsBlocks;
   // all starts: short ranges keep the chains through each short; walks: one wave of ranges (seven
@@ -797,188 +1069,141 @@ static cudaError_t partition_typed(glc_ctx* ctx, const T* v, int64_t n, int32_t*
   const int rb = (int)per * kMaxJumpBlocks;
   const int64_t nr = (nb + rb - 1) / rb;
   const Ranges rg{nb, nr, rb};
-  const int64_t mmax = nb;  // split partitions are >= 128 values except the last
-  size_t bytes = 0;
-  bytes += al(sizeof(SumPair) * (nb + 1));                     // prefix
-  bytes += al(sizeof(SumPair) * (scan_num_tiles(nb) + 1));     // scan tiles (pair)
-  bytes += al(sizeof(int32_t) * nb);                           // nb_next
-  bytes += al(sizeof(int32_t) * nr * kMaxJumpBlocks) * 2;      // exits, counts
-  bytes += al(sizeof(int32_t) * nr) * 3;                       // entries, base, exit_first
-  bytes += al(sizeof(int32_t) * nb) * 3;                       // cexit, ccnt, visit
-  bytes += al(sizeof(long long) * nb);                         // nb_err
-  bytes += al(sizeof(long long) * mmax);                       // kerr
-  bytes += al(sizeof(long long) * mmax) * 4;                   // part_err, part_err2, cerr, cerr2
-  bytes += al(sizeof(int64_t) * (nb + 1)) * 2;                 // flags, idx
-  bytes += al(sizeof(int64_t) * (scan_num_tiles(nb) + 1));     // scan tiles (i64)
-  bytes += al(sizeof(int32_t) * mmax) * 4;                     // ps, pe, ps2, pe2
-  bytes += al(sizeof(double) * mmax) * 5;                      // pc, pc2, mc, cmc, cmc2
-  bytes += al(sizeof(uint8_t) * mmax) * 3;                     // prof, cached, cached2
-  bytes += al(sizeof(LineJob) * mmax);                         // jobs
-  bytes += al(sizeof(int64_t) * (mmax + 1));                   // nch
-  bytes += al(sizeof(long long) * mmax);                       // err
-  bytes += al(sizeof(int64_t) * 4);                            // device scalars
-  char* buf = nullptr;
-  if ((e = pool_alloc(ctx, &buf, bytes, s)) != cudaSuccess) return e;
-  char* sp = buf;
-  auto take = [&](size_t b) { char* r = sp; sp += al(b); return (void*)r; };
-  SumPair* pre = (SumPair*)take(sizeof(SumPair) * (nb + 1));
-  SumPair* ptiles = (SumPair*)take(sizeof(SumPair) * (scan_num_tiles(nb) + 1));
-  int32_t* nb_next = (int32_t*)take(sizeof(int32_t) * nb);
-  int32_t* exits = (int32_t*)take(sizeof(int32_t) * nr * kMaxJumpBlocks);
-  int32_t* cnts = (int32_t*)take(sizeof(int32_t) * nr * kMaxJumpBlocks);
-  int32_t* entries = (int32_t*)take(sizeof(int32_t) * nr);
-  int32_t* base = (int32_t*)take(sizeof(int32_t) * nr);
-  int32_t* exit_first = (int32_t*)take(sizeof(int32_t) * nr);
-  int32_t* cexit = (int32_t*)take(sizeof(int32_t) * nb);
-  int32_t* ccnt = (int32_t*)take(sizeof(int32_t) * nb);
-  int32_t* visit = (int32_t*)take(sizeof(int32_t) * nb);
-  long long* nb_err = (long long*)take(sizeof(long long) * nb);
-  long long* kerr = (long long*)take(sizeof(long long) * mmax);
-  long long* part_err = (long long*)take(sizeof(long long) * mmax);
-  long long* part_err2 = (long long*)take(sizeof(long long) * mmax);
-  long long* cerr = (long long*)take(sizeof(long long) * mmax);
-  long long* cerr2 = (long long*)take(sizeof(long long) * mmax);
-  int64_t* flags = (int64_t*)take(sizeof(int64_t) * (nb + 1));
-  int64_t* idx = (int64_t*)take(sizeof(int64_t) * (nb + 1));
-  int64_t* itiles = (int64_t*)take(sizeof(int64_t) * (scan_num_tiles(nb) + 1));
-  int32_t* ps = (int32_t*)take(sizeof(int32_t) * mmax);
-  int32_t* pe = (int32_t*)take(sizeof(int32_t) * mmax);
-  int32_t* ps2 = (int32_t*)take(sizeof(int32_t) * mmax);
-  int32_t* pe2 = (int32_t*)take(sizeof(int32_t) * mmax);
-  double* pc = (double*)take(sizeof(double) * mmax);
-  double* pc2 = (double*)take(sizeof(double) * mmax);
-  double* mc = (double*)take(sizeof(double) * mmax);
-  double* cmc = (double*)take(sizeof(double) * mmax);
-  double* cmc2 = (double*)take(sizeof(double) * mmax);
-  uint8_t* prof = (uint8_t*)take(mmax);
-  uint8_t* cached = (uint8_t*)take(mmax);
-  uint8_t* cached2 = (uint8_t*)take(mmax);
-  LineJob* jobs = (LineJob*)take(sizeof(LineJob) * mmax);
-  int64_t* nch = (int64_t*)take(sizeof(int64_t) * (mmax + 1));
-  long long* perr = (long long*)take(sizeof(long long) * mmax);
-  int64_t* dsc = (int64_t*)take(sizeof(int64_t) * 4);  // [0] unused, [1] m, [2] any (int), [3] walk fail
+  PoolBuf split(s), lists(s);
+  SumPair *pre, *ptiles;
+  int32_t *nb_next, *exits, *cnts, *entries, *base, *exit_first, *cexit = nullptr, *ccnt = nullptr, *visit = nullptr;
+  long long* nb_err;
+  uint8_t* ovf;
+  int64_t* dsc;        // [1] partitions of the split, [3] first range the walks did not cover (-1: none);
+                       // [4] partitions left, [5] list, [6] DEVERR_*
+  unsigned* counters;  // right after dsc: cleared together
+  split.want(&pre, nb + 1);
+  split.want(&ptiles, scan_num_tiles(nb) + 1);
+  split.want(&nb_next, nb);
+  split.want(&nb_err, nb);
+  split.want(&ovf, sizeof(T) == 8 && !TypeTraits<T>::is_signed ? nb : 1);
+  split.want(&exits, nr * kMaxJumpBlocks);
+  split.want(&cnts, nr * kMaxJumpBlocks);
+  split.want(&entries, nr);
+  split.want(&base, nr);
+  split.want(&exit_first, nr);
+  if (!all_starts) {
+    split.want(&cexit, nb);
+    split.want(&ccnt, nb);
+    split.want(&visit, nb);
+  }
+  split.want(&dsc, 32);
+  split.want(&counters, kMergeCounters);
+  if ((e = split.get(ctx)) != cudaSuccess) return e;
   RangeSums rs{pre, n, nb};
-
-  auto fail = [&](cudaError_t ee) { cudaFreeAsync(buf, s); return ee; };
-  static PerDeviceFlag link_attr;
-  if (const int dev = current_device(); !link_attr.test(dev)) {
+  static PerDeviceFlag attrs;
+  if (const int dev = current_device(); !attrs.test(dev)) {
     if ((e = cudaFuncSetAttribute(chain_link_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLinkSmem)) != cudaSuccess ||
         (e = cudaFuncSetAttribute(chain_link_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLinkSmem)) != cudaSuccess)
-      return fail(e);
-    link_attr.set(dev);
+      return e;
+    attrs.set(dev);
   }
   auto grid = [](int64_t x, int b) { return (unsigned)((x + b - 1) / b); };
 
-  block_sums_kernel<T><<<grid(nb * 32, 256), 256, 0, s>>>(v, n, nb, pre);
-  if ((e = exclusive_scan<SumPair>(pre, pre, nb, pre + nb, ptiles, s)) != cudaSuccess) return fail(e);
-  if ((e = cudaMemsetAsync(nb_next, 0xff, sizeof(int32_t) * nb, s)) != cudaSuccess) return fail(e);
-  // dsc[1] = partitions, dsc[3] = first range the walks did not cover (-1: none)
-  auto emit = [&]() -> cudaError_t {
-    chain_emit_kernel<<<(unsigned)nr, 32, (sizeof(int32_t) + sizeof(uint16_t)) * rb, s>>>(nb_next, nb_err, entries, base,
-                                                                                           rg, n, ps, pe, kerr);
+  if ((e = cudaMemsetAsync(dsc, 0, (size_t)((char*)(counters + kMergeCounters) - (char*)dsc), s)) != cudaSuccess) return e;
+  block_sums_kernel<T><<<grid(nb * 8, 256), 256, 0, s>>>(v, n, nb, pre, ovf);
+  if ((e = exclusive_scan<SumPair>(pre, pre, nb, pre + nb, ptiles, s)) != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(nb_next, 0xff, sizeof(int32_t) * nb, s)) != cudaSuccess) return e;
+  auto linked = [&]() -> cudaError_t {
     cudaError_t ee = cudaGetLastError();
-    if (ee == cudaSuccess)
-      ee = cudaMemcpyAsync(ctx->h_stats, dsc + 1, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+    if (ee == cudaSuccess) ee = cudaMemcpyAsync(ctx->h_stats, dsc + 1, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
     return ee == cudaSuccess ? cudaStreamSynchronize(s) : ee;
   };
   auto every_start = [&]() -> cudaError_t {
     split_kernel<T><<<grid(nb, 8), 256, 0, s>>>(v, rs, nb_next, nb_err);
     chain_exit_kernel<<<(unsigned)nr, 32, sizeof(int32_t) * rb, s>>>(nb_next, rg, exits, cnts);
     chain_link_kernel<false><<<1, 1024, kLinkSmem, s>>>(exits, cnts, rg, entries, base, dsc + 1);
-    return emit();
+    return linked();
   };
   if (all_starts) {
-    if ((e = every_start()) != cudaSuccess) return fail(e);
+    if ((e = every_start()) != cudaSuccess) return e;
   } else {  // the walk from 0: first only the starts that the walks of the ranges visit
-    if ((e = cudaMemsetAsync(cexit, 0xff, sizeof(int32_t) * nb, s)) != cudaSuccess) return fail(e);
+    if ((e = cudaMemsetAsync(cexit, 0xff, sizeof(int32_t) * nb, s)) != cudaSuccess) return e;
     const WalkOut w{nb_next, nb_err, cexit, ccnt, visit, exit_first};
     walk_kernel<T, true><<<(unsigned)nr, 32, 0, s>>>(v, rs, rg, w);
     walk_kernel<T, false><<<(unsigned)nr, 32, 0, s>>>(v, rs, rg, w);
     chain_link_kernel<true><<<1, 1024, kLinkSmem, s>>>(cexit, ccnt, rg, entries, base, dsc + 1);
-    if ((e = emit()) != cudaSuccess) return fail(e);
-    if (ctx->h_stats[2] >= 0 && (e = every_start()) != cudaSuccess) return fail(e);  // it left the visited starts
+    if ((e = linked()) != cudaSuccess) return e;
+    if (ctx->h_stats[2] >= 0 && (e = every_start()) != cudaSuccess) return e;  // it left the visited starts
   }
-  int64_t m = ctx->h_stats[0];
-  if (m <= 0 || m > mmax) {
+  const int64_t m = ctx->h_stats[0];
+  if (m <= 0 || m > nb) {
     if (err) *err = "partitioner produced an invalid split";
-    cudaFreeAsync(buf, s);
     return cudaErrorUnknown;
   }
 
-  // max |delta| of each job's line (partitions, or adjacent pairs of the merge rounds)
-  auto run_jobs = [&](int64_t cnt, int pairs, const uint8_t* cache, const long long* known) -> cudaError_t {
-    job_setup_kernel<<<grid(cnt, 256), 256, 0, s>>>(ps, pe, m, pairs, cache, cerr, known, pc, rs, jobs, nch, perr);
-    const int64_t resident = (int64_t)ctx->num_sms * 4;  // 256-thread CTAs, four per SM
-    job_err_kernel<T><<<(unsigned)(cnt < resident ? cnt : resident), 256, 0, s>>>(v, jobs, nch, cnt, perr);
-    return cudaGetLastError();
-  };
-  // costs of the split partitions: their max |delta| came with the split evaluation
-  if ((e = run_jobs(m, 0, nullptr, kerr)) != cudaSuccess) return fail(e);
-  part_cost_kernel<<<grid(m, 256), 256, 0, s>>>(jobs, perr, m, pc);
-  // each partition's max |delta| travels with it through the merge rounds (for the fit)
-  if ((e = cudaMemcpyAsync(part_err, perr, sizeof(long long) * m, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-    return fail(e);
-  if ((e = cudaMemsetAsync(cached, 0, mmax, s)) != cudaSuccess) return fail(e);
+  MergeArgs ma;
+  for (PartList* l : {&ma.a, &ma.b}) {
+    lists.want(&l->start, m);
+    lists.want(&l->end, m);
+    lists.want(&l->cost, m);
+    lists.want(&l->err, m);
+    lists.want(&l->rejected, m);
+  }
+  lists.want(&ma.selected, m);
+  lists.want(&ma.pair_err, m);
+  lists.want(&ma.pair_t, 2 * m);
+  lists.want(&ma.pair_lim, m);
+  // units small enough that a short column's pairs reach every warp
+  ma.unit = 512;
+  while (ma.unit < kMergeUnitMost && n / ma.unit > 2ll * ctx->num_sms * (kMergeThreads / 32)) ma.unit *= 2;
+  lists.want(&ma.queue, n / ma.unit + m + 1);
+  lists.want(&ma.cta_heads, ctx->num_sms);
+  int64_t *widths, *wtiles;
+  lists.want(&widths, m + 1);
+  lists.want(&wtiles, scan_num_tiles(m) + 1);
+  if ((e = lists.get(ctx)) != cudaSuccess) return e;
+  ma.ovf = ovf;
+  ma.n = n;
+  ma.m = (int32_t)m;
+  ma.counters = counters;
+  ma.out = dsc + 4;
+  chain_emit_kernel<<<(unsigned)nr, 32, (sizeof(int32_t) + sizeof(uint16_t)) * rb, s>>>(nb_next, nb_err, entries, base, rg, n,
+                                                                                         ma.a.start, ma.a.end, ma.a.err);
+  // one CTA per SM, all resident; fewer when the list is short (a cheaper barrier)
+  const int64_t ctas = std::min<int64_t>(ctx->num_sms, std::max<int64_t>(1, (m + 15) / 16));
+  void* kargs[] = {(void*)&v, (void*)&rs, (void*)&ma};
+  if ((e = cudaLaunchCooperativeKernel((const void*)merge_kernel<T>, dim3((unsigned)ctas), dim3(kMergeThreads), kargs, 0, s)) !=
+          cudaSuccess ||
+      (e = cudaMemcpyAsync(ctx->h_stats, dsc + 4, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+      (e = cudaStreamSynchronize(s)) != cudaSuccess)
+    return e;
+  const int64_t P = ctx->h_stats[0];
+  if (ctx->h_stats[2] != DEVERR_NONE || P <= 0 || P > m) {
+    if (err) *err = ctx->h_stats[2] == DEVERR_TIMEOUT ? "a device-side wait of the partitioner gave up" : "partitioner produced an invalid merge";
+    return cudaErrorUnknown;
+  }
+  const PartList fin = ctx->h_stats[1] ? ma.b : ma.a;
 
-  for (int round = 0; round < kMaxMergeRounds && m >= 2; round++) {
-    if ((e = run_jobs(m - 1, 1, cached, nullptr)) != cudaSuccess) return fail(e);
-    if ((e = cudaMemsetAsync(dsc + 2, 0, sizeof(int64_t), s)) != cudaSuccess) return fail(e);
-    pair_score_kernel<<<grid(m - 1, 256), 256, 0, s>>>(jobs, perr, cached, cmc, pc, m, mc, prof, (int*)(dsc + 2));
-    merge_heads_kernel<<<grid(m, 256), 256, 0, s>>>(prof, m, round, flags);
-    if ((e = exclusive_scan<int64_t>(flags, idx, m, dsc + 1, itiles, s)) != cudaSuccess) return fail(e);
-    merge_scatter_kernel<<<grid(m, 256), 256, 0, s>>>(ps, pe, pc, mc, prof, flags, idx, m, round, ps2, pe2, pc2,
-                                                       cached2, cmc2, perr, part_err, part_err2, cerr2);
-    if ((e = cudaGetLastError()) != cudaSuccess) return fail(e);
-    if ((e = cudaMemcpyAsync(ctx->h_stats, dsc + 1, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-      return fail(e);
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail(e);
-    const int64_t m2 = ctx->h_stats[0];
-    const int any = (int)(ctx->h_stats[1] & 0xffffffff);
-    if (!any) break;  // nothing merged: the lists are unchanged
-    std::swap(ps, ps2);
-    std::swap(pe, pe2);
-    std::swap(pc, pc2);
-    std::swap(cached, cached2);
-    std::swap(cmc, cmc2);
-    std::swap(part_err, part_err2);
-    std::swap(cerr, cerr2);
-    m = m2;
+  if (out.column) {  // the column's arrays, fitted
+    glc_column* c = out.column;
+    c->P = P;
+    if ((e = out.alloc(c, s)) != cudaSuccess || (e = cudaMemsetAsync(out.stats, 0, 4 * sizeof(int64_t), s)) != cudaSuccess) return e;
+    part_fit_kernel<T><<<grid(P, 128), 128, 0, s>>>(fin, rs, (int32_t)P, c->d_start, c->d_end, c->d_types, c->d_params,
+                                                    c->d_bits, c->d_err, widths, (unsigned long long*)(out.stats + 1),
+                                                    (unsigned long long*)(out.stats + 3));
+    return exclusive_scan<int64_t>(widths, c->d_offs, P, out.stats, wtiles, s);
   }
-
-  int32_t* rs_out = nullptr;
-  int32_t* re_out = nullptr;
-  if ((e = pool_alloc(ctx, &rs_out, sizeof(int32_t) * m, s)) != cudaSuccess) return fail(e);
-  if ((e = pool_alloc(ctx, &re_out, sizeof(int32_t) * m, s)) != cudaSuccess) {
-    cudaFreeAsync(rs_out, s);
-    return fail(e);
-  }
-  cudaMemcpyAsync(rs_out, ps, sizeof(int32_t) * m, cudaMemcpyDeviceToDevice, s);
-  cudaMemcpyAsync(re_out, pe, sizeof(int32_t) * m, cudaMemcpyDeviceToDevice, s);
-  if (out_err) {
-    long long* er_out = nullptr;
-    if ((e = pool_alloc(ctx, &er_out, sizeof(long long) * m, s)) != cudaSuccess) {
-      cudaFreeAsync(rs_out, s);
-      cudaFreeAsync(re_out, s);
-      return fail(e);
-    }
-    cudaMemcpyAsync(er_out, part_err, sizeof(long long) * m, cudaMemcpyDeviceToDevice, s);
-    *out_err = er_out;
-  }
-  cudaFreeAsync(buf, s);
-  *out_s = rs_out;
-  *out_e = re_out;
-  *outP = m;
-  return cudaGetLastError();
+  *out.P = P;
+  if ((e = pool_alloc(ctx, out.starts, sizeof(int32_t) * P, s)) != cudaSuccess) return e;
+  if ((e = pool_alloc(ctx, out.ends, sizeof(int32_t) * P, s)) == cudaSuccess &&
+      (e = cudaMemcpyAsync(*out.starts, fin.start, sizeof(int32_t) * P, cudaMemcpyDeviceToDevice, s)) == cudaSuccess)
+    e = cudaMemcpyAsync(*out.ends, fin.end, sizeof(int32_t) * P, cudaMemcpyDeviceToDevice, s);
+  return e;
 }
 
-cudaError_t launch_partition_variable(glc_ctx* ctx, glc_dtype dt, const void* values, int64_t n, int32_t** d_starts,
-                                      int32_t** d_ends, int64_t* P, cudaStream_t s, std::string* err,
-                                      long long** d_err) {
+cudaError_t launch_partition_variable(glc_ctx* ctx, glc_dtype dt, const void* values, int64_t n, const PartOut& out,
+                                      cudaStream_t s, std::string* err) {
   switch (dt) {
-    case GLC_I32: return partition_typed<int32_t>(ctx, (const int32_t*)values, n, d_starts, d_ends, P, s, err, d_err);
-    case GLC_I64: return partition_typed<int64_t>(ctx, (const int64_t*)values, n, d_starts, d_ends, P, s, err, d_err);
-    case GLC_U64: return partition_typed<uint64_t>(ctx, (const uint64_t*)values, n, d_starts, d_ends, P, s, err, d_err);
-    case GLC_U32: return partition_typed<uint32_t>(ctx, (const uint32_t*)values, n, d_starts, d_ends, P, s, err, d_err);
+    case GLC_I32: return partition_typed<int32_t>(ctx, (const int32_t*)values, n, out, s, err);
+    case GLC_I64: return partition_typed<int64_t>(ctx, (const int64_t*)values, n, out, s, err);
+    case GLC_U64: return partition_typed<uint64_t>(ctx, (const uint64_t*)values, n, out, s, err);
+    case GLC_U32: return partition_typed<uint32_t>(ctx, (const uint32_t*)values, n, out, s, err);
   }
   return cudaErrorInvalidValue;
 }
