@@ -626,10 +626,38 @@ glc_status glc_serialize(glc_ctx* ctx, const glc_column* c, void* blob, uint64_t
   uint8_t* b = (uint8_t*)blob;
   const cudaMemcpyKind k = host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
   const uint64_t P = c->P;
+  static_assert(sizeof(BlobHeader) == 4 * kSerHeaderWords, "header words");
   struct Piece { uint64_t off; const void* src; uint64_t bytes; } pieces[8] = {
       {h.start_off, c->d_start, 4 * P}, {h.end_off, c->d_end, 4 * P},     {h.types_off, c->d_types, 4 * P},
       {h.params_off, c->d_params, 32 * P}, {h.bits_off, c->d_bits, 4 * P}, {h.offsets_off, c->d_offs, 8 * P},
       {h.errb_off, c->d_err, 8 * P},     {h.delta_off, words_begin(c), h.delta_size}};
+  // A device blob and column of this context's device: one kernel.  Blobs elsewhere (host memory,
+  // another device) and odd addresses are copied piece by piece.
+  bool one_launch = !host && c->ctx && c->ctx->device == ctx->device && ((uintptr_t)b & 3) == 0;
+  for (const Piece& pc : pieces) one_launch = one_launch && ((uintptr_t)pc.src & 3) == 0;
+  if (one_launch) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, b) != cudaSuccess) {
+      cudaGetLastError();  // clear the error of an unknown pointer
+      one_launch = false;
+    } else {
+      one_launch = at.type == cudaMemoryTypeDevice && at.device == ctx->device;
+    }
+  }
+  if (one_launch) {
+    SerializeArgs a;
+    a.dst = b;
+    a.total = total;
+    std::memcpy(a.header, &h, sizeof a.header);
+    for (int k = 0; k < kSerPieces; k++) {
+      a.src[k] = pieces[k].src;
+      a.off[k] = pieces[k].off;
+      a.bytes[k] = pieces[k].bytes;
+    }
+    CK(launch_serialize(a, ctx->num_sms, s), "serialize");
+    CK(cudaStreamSynchronize(s), "serialize: sync");  // the blob is complete when the call returns
+    return GLC_OK;
+  }
   // zero the gaps (alignment padding and the tail), then the header, then the arrays
   uint64_t cursor = sizeof(BlobHeader);
   for (const Piece& pc : pieces) {

@@ -236,6 +236,19 @@ cudaError_t launch_choose_lengths(glc_dtype dt, const CfColumn* cols, const int3
 cudaError_t launch_place_prepacked(glc_dtype dt, const CfColumn* cols, const int32_t* owner, int64_t nitems,
                                    void* scratch, PartDesc* tdesc, long long* terr, unsigned long long* status,
                                    int num_sms, cudaStream_t s);
+// serialize.cu: a blob written to device memory.  Piece k (the seven metadata arrays, then the
+// bitstream) lies at dst + off[k]; the offsets ascend and, like the total, are multiples of 8; dst
+// and every source are 4-byte aligned.
+constexpr int kSerPieces = 8;
+constexpr int kSerHeaderWords = 30;
+struct SerializeArgs {
+  void* dst;
+  uint64_t total;
+  const void* src[kSerPieces];
+  uint64_t off[kSerPieces], bytes[kSerPieces];
+  uint32_t header[kSerHeaderWords];
+};
+cudaError_t launch_serialize(const SerializeArgs& a, int num_sms, cudaStream_t s);
 cudaError_t launch_validate(const glc_column* c, int* d_bad, cudaStream_t s);
 cudaError_t launch_max_bits(const glc_column* c, int64_t* d_out, cudaStream_t s);
 // pack.cu: one column's arrays for the packer

@@ -504,3 +504,28 @@ def test_variable_partitions_of_jumps(oracle, glc_ctx, n):
             ds, de = glc.partition_variable(glc_ctx, w)
             s, e = oracle.partition_variable(w)
             assert np.array_equal(ds, s) and np.array_equal(de, e)
+
+
+@pytest.mark.parametrize("kind,n,mode", [("i32_linear", 1, "fixed"), ("u32_const", 5_000, "fixed"), ("u32_noise", 4097, "var"),
+                                         ("i64_walk", 100_003, "fixed"), ("u64_piecewise", 300_001, "var"),
+                                         ("i64_extreme", 40_961, "fixed")])
+@pytest.mark.parametrize("offset", [0, 4, 8, 12, 2, 1])
+def test_serialize_into_device_memory(oracle, glc_ctx, kind, n, mode, offset):
+    """A blob written at any address of a device buffer (the launch at 4-byte aligned ones, the copies at the
+    others) equals the oracle's, and the bytes around it stay as they were."""
+    import ctypes
+    torch = pytest.importorskip("torch")
+    v = _data(kind, n)
+    code = {"int32": glc.I32, "int64": glc.I64, "uint64": glc.U64, "uint32": glc.U32}[v.dtype.name]
+    col = glc.compress_device(glc_ctx, code, v.ctypes.data, n, glc.FIXED if mode == "fixed" else glc.VARIABLE,
+                              fixed_len=1000, host=True)
+    blob = oracle.serialize(oracle.compress(v, "fixed", 1000) if mode == "fixed" else oracle.compress(v, "variable"))
+    buf = torch.full((len(blob) + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    size = ctypes.c_uint64()
+    glc_ctx.check(glc_ctx.lib.glc_serialize(glc_ctx.handle, col.handle, buf.data_ptr() + offset, len(blob), 0, 0,
+                                            ctypes.byref(size), None))
+    got = buf.cpu().numpy().tobytes()
+    assert size.value == len(blob) and got[offset:offset + len(blob)] == blob
+    assert set(got[:offset] + got[offset + len(blob):]) == {0xA5}
+    col.free()
