@@ -41,6 +41,28 @@ struct __align__(32) PartDesc {
   int32_t bits_type;
 };
 
+// 32 bytes (one DRAM sector) at a 32-byte aligned address in one access (sm_100).
+struct Bytes32 {
+  unsigned long long q[4];
+};
+__device__ __forceinline__ Bytes32 load32_nc(const void* p) {  // read-only data
+  Bytes32 r;
+  asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(r.q[0]), "=l"(r.q[1]), "=l"(r.q[2]), "=l"(r.q[3]) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ Bytes32 load32(const void* p) {
+  Bytes32 r;
+  asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(r.q[0]), "=l"(r.q[1]), "=l"(r.q[2]), "=l"(r.q[3])
+               : "l"(p)
+               : "memory");
+  return r;
+}
+__device__ __forceinline__ void store32(void* p, const Bytes32& r) {
+  asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(r.q[0]), "l"(r.q[1]), "l"(r.q[2]), "l"(r.q[3])
+               : "memory");
+}
+
 template <typename T> struct TypeTraits;
 template <> struct TypeTraits<int32_t>  { static constexpr bool is_signed = true;  };
 template <> struct TypeTraits<int64_t>  { static constexpr bool is_signed = true;  };
@@ -240,6 +262,7 @@ __device__ __forceinline__ double i128_to_double(i128 v) {
 
 // n(n^2-1)/6 exactly, without 128-bit division.
 __device__ __forceinline__ i128 den6_exact(int64_t n) {
+  if (n <= (1 << 20)) return (i128)((uint64_t)n * ((uint64_t)n * (uint64_t)n - 1) / 6);  // n^3 fits 64 bits
   int64_t a = n - 1, b = n, c = n + 1;
   if (a % 3 == 0) a /= 3; else if (b % 3 == 0) b /= 3; else c /= 3;
   if ((a & 1) == 0) a /= 2; else if ((b & 1) == 0) b /= 2; else c /= 2;

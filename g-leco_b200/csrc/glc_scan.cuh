@@ -1,7 +1,11 @@
 // glc_scan.cuh -- device-wide exclusive prefix sum (reduce-then-scan) for any trivially
 // copyable value type with operator+ (int64, 128-bit integers, pairs of them).
 //
-// Three launches: each 1024-thread CTA scans a tile of 4096 items and writes the tile total;
+// Up to 16384 items of 8 bytes: one CTA, one launch (the totals of a column's tiles or partitions
+// are usually that few, and each launch of a chain costs 3 to 5 us, its gap included: 13,725
+// widths took 14 us in three launches, 5 us in one).  More than that, where one SM's loads would
+// bound it, or wider items:
+// three launches: each 1024-thread CTA scans a tile of 4096 items and writes the tile total;
 // one CTA scans the tile totals (looping with a carry, so any count works); each CTA then adds
 // its tile's base.  The bit offsets of the bitstream are this scan over len * bits
 // (the reference computes each offset with an O(P) loop per partition,
@@ -119,6 +123,85 @@ scan_add_kernel(V* __restrict__ out, int64_t count, const V* __restrict__ tile_b
     if (base + k < count) out[base + k] = out[base + k] + b;
 }
 
+// The whole scan in one CTA: up to four chunks of 4 items per thread, all of them loaded before the
+// barriers and stored after them (in and out may alias).  The chunks' warp scans are independent,
+// and warp c scans the warp totals of chunk c, so four chunks cost two barriers like one.  A
+// thread's four 8-byte items are one 32-byte access where in and out allow it (one SM writes a
+// sector per cycle: 13,725 items in 8-byte stores took 11 us).
+constexpr int kScanOneChunks = 4;
+constexpr int kScanOneMax = kScanTile * kScanOneChunks;
+
+template <typename V> __global__ void __launch_bounds__(kScanThreads)
+scan_one_kernel(const V* in, V* out, int count, V* grand_total) {
+  __shared__ V s_warp[kScanOneChunks][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int chunk = (int)blockDim.x * kScanItems;
+  static_assert(sizeof(V) * kScanItems == 32, "a thread's items of a chunk are one 32-byte access");
+  const bool vec_in = (reinterpret_cast<uintptr_t>(in) & 31) == 0, vec_out = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
+  V items[kScanOneChunks][kScanItems], sum[kScanOneChunks], inc[kScanOneChunks];
+#pragma unroll
+  for (int c = 0; c < kScanOneChunks; c++) {
+    const int base = c * chunk + (int)threadIdx.x * kScanItems;
+    sum[c] = V();
+    if (vec_in && base + kScanItems <= count) {
+      const Bytes32 r = load32(in + base);
+      memcpy(items[c], &r, 32);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kScanItems; k++) items[c][k] = (base + k < count) ? in[base + k] : V();
+    }
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) sum[c] = sum[c] + items[c][k];
+    inc[c] = sum[c];
+  }
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+#pragma unroll
+    for (int c = 0; c < kScanOneChunks; c++) {
+      const V y = shfl_up_any(inc[c], d);
+      if (lane >= d) inc[c] = inc[c] + y;
+    }
+  }
+  if (lane == 31) {
+#pragma unroll
+    for (int c = 0; c < kScanOneChunks; c++) s_warp[c][warp] = inc[c];
+  }
+  __syncthreads();
+  for (int c = warp; c < kScanOneChunks; c += nwarps) {
+    V w = lane < nwarps ? s_warp[c][lane] : V();
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const V y = shfl_up_any(w, d);
+      if (lane >= d) w = w + y;
+    }
+    if (lane < nwarps) s_warp[c][lane] = w;  // inclusive
+  }
+  __syncthreads();
+  V before = V();  // the chunks before chunk c
+#pragma unroll
+  for (int c = 0; c < kScanOneChunks; c++) {
+    const int base = c * chunk + (int)threadIdx.x * kScanItems;
+    V ex = before + (warp > 0 ? s_warp[c][warp - 1] : V()) + inc[c] - sum[c];
+    V res[kScanItems];
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+      res[k] = ex;
+      ex = ex + items[c][k];
+    }
+    if (vec_out && base + kScanItems <= count) {
+      Bytes32 r;
+      memcpy(&r, res, 32);
+      store32(out + base, r);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kScanItems; k++)
+        if (base + k < count) out[base + k] = res[k];
+    }
+    before = before + s_warp[c][nwarps - 1];
+  }
+  if (threadIdx.x == 0 && grand_total) *grand_total = before;
+}
+
 inline int64_t scan_num_tiles(int64_t count) { return (count + kScanTile - 1) / kScanTile; }
 
 // Scratch: one V per tile.  in and out may alias.  *grand_total (device) may be null.
@@ -127,6 +210,14 @@ cudaError_t exclusive_scan(const V* in, V* out, int64_t count, V* grand_total, V
   if (count <= 0) {
     if (grand_total) return cudaMemsetAsync(grand_total, 0, sizeof(V), s);
     return cudaSuccess;
+  }
+  if constexpr (sizeof(V) == 8) {
+    if (count <= kScanOneMax) {
+      const int need = (int)((count + kScanItems - 1) / kScanItems + 31) & ~31;
+      const int threads = need < kScanThreads ? need : kScanThreads;
+      scan_one_kernel<V><<<1, threads, 0, s>>>(in, out, (int)count, grand_total);
+      return cudaGetLastError();
+    }
   }
   int64_t nt = scan_num_tiles(count);
   scan_tiles_kernel<V><<<(unsigned)nt, kScanThreads, 0, s>>>(in, out, count, tile_scratch);
