@@ -5,29 +5,19 @@
 // Replaces, for those columns, the separate fit, bit-offset scan, table build and pack passes
 // (fit.cu, glc_scan.cuh, pack.cu; in the reference wprocessPartitionsKernel,
 // setBitOffsetsKernel and packDeltasKernelOptimized, compression/CompressionKernels.cuh:45-372,
-// which read the values four times) with ONE persistent kernel that reads every value once:
-//
-//   producer warp   stages tile t's values in shared memory with cp.async.bulk, three stages
-//                   (full/empty mbarriers, bounded waits that sleep in the barrier);
-//   solver warp     fits the lines of tile k + 1 from its exact sums (one lane per partition, the
-//                   same arithmetic as fit.cu, so the result is identical bit for bit) and picks
-//                   each partition's residual mode, while the compute warps work on tile k;
-//   compute warps   per step, with every partition inside the tile (L divides 4096):
-//     A  exact sums of tile k + 1 per partition from 64-bit partials of 32-bit halves, and the
-//        range flags (direct copy; FP64-safe values); a group of L/16 threads owns a partition,
-//        16 values each;
-//     B  the residual of every value of tile k (fma prediction, round half away from zero,
-//        saturating cast; calculateDelta -- in FP64 without conversion instructions where the
-//        line and the values allow it) and max |residual| per partition -> the bit widths;
-//     C  the tile's words into its own slot of a scratch array (slots of the worst-case size of
-//        a tile, bit offsets relative to the tile), the partitions' descriptors with
-//        tile-relative offsets and their max errors, and the tile's bit count;
-//   then an exclusive scan of the tiles' bit counts gives every tile's first bit, and
-//   fixed_place_kernel (one CTA per tile) copies each tile's words to their place in the column
-//   and writes the metadata arrays from the descriptors.  No tile waits for another.
+// which read the values four times) with ONE kernel that reads every value once.  Every partition
+// lies inside a tile (L divides 4096), so a CTA fits, measures and packs its tile alone: its words
+// go into its own slot of a scratch array (slots of the worst-case size of a tile, bit offsets
+// relative to the tile), with the partitions' descriptors and max errors and the tile's bit count.
+// Then an exclusive scan of the tiles' bit counts gives every tile's first bit, and
+// fixed_place_kernel (one CTA per tile) copies each tile's words to their place in the column
+// and writes the metadata arrays from the descriptors.  No tile waits for another.
 //
 // The column's word array is allocated at its exact size between the two kernels (the scan gives
 // the total); the slots cost one extra write and read of the compressed bits.
+//
+// The partition-length choice of a batch (choose_lengths_kernel) measures three lengths at once in
+// persistent CTAs of producer, solver and compute warps and packs the usual choice, 4096, on the way.
 #include <type_traits>
 #include "glc_internal.h"
 #include "glc_scan.cuh"
@@ -68,15 +58,6 @@ struct FixedCompressArgs {
 };
 
 __device__ __forceinline__ void cf_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kCfThreads) : "memory"); }
-// cf_sync that also returns whether any compute thread passed true.
-__device__ __forceinline__ bool cf_sync_or(bool v) {
-  uint32_t r;
-  asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 1, %2, q;\n selp.u32 %0, 1, 0, p;\n}\n"
-               : "=r"(r)
-               : "r"((uint32_t)v), "n"(kCfThreads)
-               : "memory");
-  return r != 0;
-}
 
 // The producer lane of a launch: stages item blockIdx.x + k * gridDim.x of the work list into stage
 // k % S (its values, from the 16-byte block that holds the first one), with the item, its
@@ -122,7 +103,6 @@ constexpr double kMagic = 6755399441055744.0;        // K = 1.5 * 2^52: the bits
 constexpr double kHalfBias = 0x1.fffffffffffffp-2;    // 0.5 - 2^-54
 constexpr int kFtStride = 129;                        // transposed fields: field f of 32-value group G at f * 129 + G
 constexpr int kFtWords = 32 * kFtStride;
-constexpr int kStgWords = kDecodeTile + kDecodeTile / 32;  // a tile's words, one pad word after every 32
 
 // How a partition's residuals are computed (uniform per partition, so per thread):
 //   CF_DIRECT   direct copy (a uint64 value above 2^53): the field is the value;
@@ -433,16 +413,13 @@ __device__ __forceinline__ void cf_store_resid(const T* xp, long long* rp, int r
   }
 }
 
-// The compress kernel's CTA: eight compute warps, the producer warp and the solver warp.  Per step
+// The length choice's CTA: eight compute warps, the producer warp and the solver warp.  Per step
 // k the compute warps take the sums of tile k + 1 and the residuals, widths and words of tile k,
-// while the solver warp fits the lines of tile k + 1 (one lane per partition) and the producer
-// stages the next tile as soon as a stage is free: the fit's long dependency chain (128-bit
-// arithmetic, two divisions) runs beside the compute warps instead of between two of their
-// barriers.  Every wait is bounded.  The compress kernel runs two stages at three CTAs per SM (64
-// registers; measured 5 % faster than three stages at two CTAs per SM: other CTAs cover the load
-// of the next tile); the length choice, with heavier per-value work, three stages at two (two
-// stages at three CTAs per SM fit its registers too, but measured 3 % slower).
-constexpr int kCfCompressStages = 2;
+// while the solver warp fits the lines of tile k + 1 and the producer stages the next tile as soon
+// as a stage is free: the fit's long dependency chain (128-bit arithmetic, two divisions) runs
+// beside the compute warps instead of between two of their barriers.  Every wait is bounded.  Three
+// stages at two CTAs per SM (two stages at three CTAs per SM fit its registers too, but measured 3 %
+// slower).
 constexpr int kCfChooseStages = 3;
 constexpr int kCfFixCTA = kCfThreads + 64;
 
@@ -450,314 +427,445 @@ template <typename T> __host__ __device__ constexpr int cf_fix_smem_bytes(int st
   return stages * cf_stage_bytes<T>() + (sizeof(T) == 4 ? kCfWorkBytes : 0);
 }
 
-// A tile as a step sees it.
-struct CfGeom {
-  const CfColumn* col;
-  int64_t t, e0;
-  int L, g, W, cnt, np, segs_per_part;
-  int lg_L, lg_g, lg_W;  // L, g and W are powers of two: divisions are shifts
-};
-__device__ __forceinline__ CfGeom cf_geom(const FixedCompressArgs& a, int64_t item, int c) {
-  CfGeom q;
-  q.col = a.cols ? a.cols + c : &a.single;
-  q.t = item - q.col->item_base;
-  q.e0 = q.t * kDecodeTile;
-  const int64_t left = q.col->n - q.e0;
-  q.cnt = (int)(left < kDecodeTile ? left : kDecodeTile);
-  q.L = q.col->L;
-  q.lg_L = 31 - __clz(q.L);
-  q.g = q.L >> 4;
-  q.lg_g = q.lg_L - 4;
-  q.W = q.g < 32 ? q.g : 32;
-  q.lg_W = q.lg_g < 5 ? q.lg_g : 5;
-  q.np = (q.cnt + q.L - 1) >> q.lg_L;
-  q.segs_per_part = q.g >> q.lg_W;
-  return q;
+// ---- the compress kernel ---------------------------------------------------------------------
+// One CTA of 128 threads per 4096-value tile, six CTAs per SM; thread G owns the 32 consecutive values
+// of group G.  A partition is a whole number of groups (L is a multiple of 32), so a group's fields,
+// at the partition's width b, are exactly b whole words: the thread keeps its 32 fields in registers
+// from the residual pass to the packing, and no field passes through shared memory.
+//   load      16-byte asynchronous copies; group G's row starts G * (32 sizeof(T) + 16) bytes into
+//             the stage, so the lanes of a warp read their rows in 16-byte pieces without bank
+//             conflicts (rows without the 16 bytes would put every lane on the same banks);
+//   A         exact sums of y and j y over the group from 32-bit halves, added over the partition;
+//   solve     lane p of warp 0 fits partition p (fit.cu's arithmetic) and picks its residual mode;
+//   B         residuals in 64-bit integers against an FP64 prediction rounded without conversion
+//             instructions; their smallest, largest and a test that all fit 32 bits;
+//   C         widths and offsets (every warp for itself, from the partitions' maxima), fields to
+//             words with the width a compile-time constant (one funnel shift each), words through
+//             shared memory (over the warp's values) to the tile's slot in 16-byte stores.
+// A tile with a width above 31, a direct copy, a general-mode partition or an incomplete group takes
+// the slow path: 64-bit residuals value by value, each group packed in its own row.  Its last group
+// aside, a column of full tiles reaches it where a residual passes 2^30 (a jump inside a partition).
+// What bounds it: instruction issue (56 % of the slots, about 50 instructions per value and lane, the
+// sums' 64-bit additions and the residuals' integer tests first) and the five barriers of a tile,
+// which the other CTAs of the SM cover in part; memory is at 39 %.  200M uint64 values at L = 4096:
+// 903 -> 498 us (3.9 TB/s), against persistent CTAs of 256 compute threads, three per SM,
+// that passed every field through shared memory and packed with half of their threads.
+constexpr int kCgThreads = 128;
+template <typename T> __host__ __device__ constexpr int cg_row_bytes() { return 32 * (int)sizeof(T) + 16; }
+template <typename T> __host__ __device__ constexpr int cg_stage_bytes() { return kCgThreads * cg_row_bytes<T>(); }
+static_assert(cg_row_bytes<int32_t>() >= 4 * 32, "the staged words of a segment fit its rows");
+
+// Byte offset in the stage of value j of the tile.
+template <typename T> __device__ __forceinline__ int cg_at(int j) { return j * (int)sizeof(T) + (j >> 5) * 16; }
+
+template <int BYTES> __device__ __forceinline__ void cp_async(uint32_t dst, const void* src, int valid) {
+  // copies `valid` bytes and zeroes the rest of the BYTES
+  if (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(BYTES), "r"(valid) : "memory");
 }
 
-template <typename T> __global__ void __launch_bounds__(kCfFixCTA, 3)
-fixed_compress_kernel(const __grid_constant__ FixedCompressArgs a) {
-  constexpr int S = kCfCompressStages;
-  extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ __align__(8) uint64_t full[S], empty[S], sums[S], lines[S];
-  __shared__ int64_t s_stile[S];   // work item staged in each stage (-1: the end)
-  __shared__ int s_shead[S];
-  __shared__ int s_scol[S];
-  __shared__ long long s_acc[S][kCfMaxSegs][4];   // per stage: the segments' exact partial sums
-  __shared__ uint32_t s_flag[S][kCfMaxSegs];      // and range flags
-  __shared__ double s_t0[S][kCfMaxParts], s_t1[S][kCfMaxParts], s_c[S][kCfMaxParts];  // the solver's lines
-  __shared__ long long s_ci[S][kCfMaxParts];
-  __shared__ int s_mode[S][kCfMaxParts];
-  __shared__ unsigned long long s_mx[kCfMaxSegs];
-  __shared__ int s_b[kCfMaxParts];
-  __shared__ int s_bl[kCfMaxParts + 1];
-  __shared__ int s_ok;
-
-  if (threadIdx.x == 0) {
-    for (int st = 0; st < S; st++) {
-      mbar_init(&full[st], 1);
-      mbar_init(&empty[st], 1);
-      mbar_init(&sums[st], kCfThreads / 32);
-      mbar_init(&lines[st], 1);
+// The tile's values (cnt of them at src, the rest zero) into the rows of the stage.
+template <typename T> __device__ __forceinline__ void cg_load(uint8_t* stage, const T* src, int cnt, int tid) {
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(stage);
+  constexpr int kPer = 16 / (int)sizeof(T);  // values per 16-byte copy
+  constexpr int kIters = kDecodeTile / kPer / kCgThreads;
+  const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+  if (vec && cnt == kDecodeTile) {  // copies a whole number of rows apart: one address each side, constant steps
+    constexpr int kStep = kCgThreads * kPer;
+    static_assert(kStep % 32 == 0, "a step is a whole number of rows");
+    const T* p = src + tid * kPer;
+    const uint32_t d = base + cg_at<T>(tid * kPer);
+#pragma unroll
+    for (int i = 0; i < kIters; i++) cp_async<16>(d + i * (kStep / 32) * cg_row_bytes<T>(), p + i * kStep, 16);
+  } else if (vec) {
+#pragma unroll 4
+    for (int i = 0; i < kIters; i++) {
+      const int j = (i * kCgThreads + tid) * kPer;
+      const int left = (cnt - j) * (int)sizeof(T);
+      cp_async<16>(base + cg_at<T>(j), left > 0 ? src + j : src, left >= 16 ? 16 : (left > 0 ? left : 0));
     }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  } else {  // values aligned to their own size only
+#pragma unroll 8
+    for (int i = 0; i < kDecodeTile / kCgThreads; i++) {
+      const int j = i * kCgThreads + tid;
+      cp_async<(int)sizeof(T)>(base + cg_at<T>(j), j < cnt ? src + j : src, j < cnt ? (int)sizeof(T) : 0);
+    }
+  }
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+}
+
+// The values of 16 bytes of a row.
+template <typename T> struct CgVec {
+  static constexpr int N = 16 / (int)sizeof(T);
+  T v[N];
+  __device__ __forceinline__ explicit CgVec(const uint8_t* p) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    memcpy(v, &u, 16);
+  }
+};
+
+// Exact sums of a group (values past the column's end are zero): s = sum y_f, x = sum (i0 + f) y_f, by
+// halves.  Every partial is below 32 * 2^12 * 2^32 = 2^49 in magnitude.
+template <typename T>
+__device__ __forceinline__ void cg_sums(const uint8_t* __restrict__ row, int i0, HalfSums<T>& hs, uint32_t& flag) {
+  typedef typename HalfSums<T>::Acc Acc;
+  Acc s_lo = 0, s_hi = 0, t_lo = 0, t_hi = 0;
+#pragma unroll
+  for (int k = 0; k < 32 / CgVec<T>::N; k++) {
+    const CgVec<T> vec(row + 16 * k);
+#pragma unroll
+    for (int u = 0; u < CgVec<T>::N; u++) {
+      const int f = k * CgVec<T>::N + u;
+      const T y = vec.v[u];
+      value_flag<T>(flag, y);
+      if (sizeof(T) == 8) {
+        const uint32_t yl = (uint32_t)(uint64_t)y, yh = (uint32_t)((uint64_t)y >> 32);
+        s_lo = (Acc)madw_u(yl, 1u, (uint64_t)s_lo);
+        if (f) t_lo = (Acc)madw_u(yl, (uint32_t)f, (uint64_t)t_lo);
+        if (TypeTraits<T>::is_signed) {
+          s_hi = (Acc)madw_s((int32_t)yh, 1, (int64_t)s_hi);
+          if (f) t_hi = (Acc)madw_s((int32_t)yh, f, (int64_t)t_hi);
+        } else {
+          s_hi = (Acc)madw_u(yh, 1u, (uint64_t)s_hi);
+          if (f) t_hi = (Acc)madw_u(yh, (uint32_t)f, (uint64_t)t_hi);
+        }
+      } else if (TypeTraits<T>::is_signed) {
+        s_lo = (Acc)madw_s((int32_t)y, 1, (int64_t)s_lo);
+        if (f) t_lo = (Acc)madw_s((int32_t)y, f, (int64_t)t_lo);
+      } else {
+        s_lo = (Acc)madw_u((uint32_t)y, 1u, (uint64_t)s_lo);
+        if (f) t_lo = (Acc)madw_u((uint32_t)y, (uint32_t)f, (uint64_t)t_lo);
+      }
+    }
+  }
+  hs.s_lo = s_lo;
+  hs.s_hi = s_hi;
+  hs.x_lo = (Acc)i0 * s_lo + t_lo;
+  hs.x_hi = (Acc)i0 * s_hi + t_hi;
+}
+
+// The residuals of a full group in one of the fast modes: y - pred as 64-bit integers, pred from the
+// bits of K + pred (or K - pred, K + pred - c).  Keeps their low 32 bits in fl and the largest
+// magnitude; false when some residual does not fit 32 bits (then only the slow path knows them: a
+// difference taken modulo 2^64 that fits 32 bits is the difference, |y - pred| < 2^64 + 2^51 here and
+// within 2^32 of a multiple of 2^64 only near 0).
+template <typename T, int MODE>
+__device__ __forceinline__ bool cg_resid(const uint8_t* __restrict__ row, int i0, double t0, double t1, double c,
+                                         long long ci, uint32_t (&fl)[32], uint32_t& mag) {
+  constexpr long long kBits = 0x4338000000000000ll;  // the bits of K
+  double xd = (double)i0;
+  int mn = 0, mx = 0;
+  uint32_t wide = 0u;
+#pragma unroll
+  for (int k = 0; k < 32 / CgVec<T>::N; k++) {
+    const CgVec<T> vec(row + 16 * k);
+#pragma unroll
+    for (int u = 0; u < CgVec<T>::N; u++) {
+      const int f = k * CgVec<T>::N + u;
+      const double x = __fma_rn(t1, xd, t0);
+      xd = __dadd_rn(xd, 1.0);
+      uint64_t d = TypeTraits<T>::is_signed ? (uint64_t)(long long)vec.v[u] : (uint64_t)vec.v[u];
+      if (MODE == CF_NONNEG) {
+        d -= (uint64_t)(__double_as_longlong(__dadd_rz(__dadd_rn(x, kHalfBias), kMagic)) - kBits);
+      } else if (MODE == CF_NONPOS) {
+        d += (uint64_t)(__double_as_longlong(__dadd_rz(__dsub_rn(kHalfBias, x), kMagic)) - kBits);
+      } else {
+        d -= (uint64_t)ci;
+        d -= (uint64_t)(__double_as_longlong(__dadd_rz(__dadd_rn(__dsub_rn(x, c), 0.5), kMagic)) - kBits);
+      }
+      const int lo = (int)(uint32_t)d;
+      fl[f] = (uint32_t)d;
+      wide |= (uint32_t)(d >> 32) ^ (uint32_t)(lo >> 31);
+      mn = min(mn, lo);
+      mx = max(mx, lo);
+    }
+  }
+  mag = max((uint32_t)mx, 0u - (uint32_t)mn);
+  return wide == 0u;
+}
+
+// One value's residual, or the value itself for direct copy, in 64 bits (the slow path).  The fast
+// modes' formulas are those of cg_resid, exact modulo 2^64 as calc_delta is for signed types; a
+// uint64 partition outside direct copy holds values up to 2^53, where calc_delta does not saturate.
+template <typename T>
+__device__ __forceinline__ long long cg_field(T y, double xi, int mode, double t0, double t1, double c, long long ci) {
+  constexpr long long kBits = 0x4338000000000000ll;
+  const uint64_t v = TypeTraits<T>::is_signed ? (uint64_t)(long long)y : (uint64_t)y;
+  const double x = __fma_rn(t1, xi, t0);
+  if (mode == CF_NONNEG) return (long long)(v - (uint64_t)(__double_as_longlong(__dadd_rz(__dadd_rn(x, kHalfBias), kMagic)) - kBits));
+  if (sizeof(T) == 8 && mode == CF_OFFSET)
+    return (long long)(v - (uint64_t)ci -
+                       (uint64_t)(__double_as_longlong(__dadd_rz(__dadd_rn(__dsub_rn(x, c), 0.5), kMagic)) - kBits));
+  if (TypeTraits<T>::is_signed && mode == CF_NONPOS)
+    return (long long)(v + (uint64_t)(__double_as_longlong(__dadd_rz(__dsub_rn(kHalfBias, x), kMagic)) - kBits));
+  if (mode == CF_DIRECT) return (long long)v;  // the field is the value itself
+  return calc_delta<T>(y, predict_from<T>(x));
+}
+
+// The slow path's packing: the group's values become its words (width b, 1 to 64) in place.  After
+// value f, at most (f + 1) b / 32 words are complete, which end no later than value f does (4-byte
+// types, fields of up to 33 bits: the 33rd word lies in the row's padding).
+template <typename T>
+__device__ __forceinline__ void cg_pack_slow(uint8_t* row, int glen, int i0, int b, int mode, double t0, double t1,
+                                             double c, long long ci) {
+  uint32_t* words = reinterpret_cast<uint32_t*>(row);
+  const uint64_t mask = b >= 64 ? ~0ull : ((1ull << b) - 1ull);
+  uint32_t acc = 0u;  // bits not yet stored: `have` (0 to 31) of them
+  int have = 0, k = 0;
+  double xi = (double)i0;
+#pragma unroll 1
+  for (int f = 0; f < glen; f++) {
+    const T y = *reinterpret_cast<const T*>(row + f * (int)sizeof(T));
+    const uint64_t v = (uint64_t)cg_field<T>(y, xi, mode, t0, t1, c, ci) & mask;
+    xi = __dadd_rn(xi, 1.0);
+    const uint64_t lo = (v << have) | acc;
+    const uint32_t over = have ? (uint32_t)(v >> 32 >> (32 - have)) : 0u;  // the bits past 64
+    int n = have + b;  // 1 to 95 bits in (over, lo)
+    uint32_t w0 = (uint32_t)lo, w1 = (uint32_t)(lo >> 32), w2 = over;
+    if (n >= 32) { words[k++] = w0; w0 = w1; w1 = w2; n -= 32; }
+    if (n >= 32) { words[k++] = w0; w0 = w1; n -= 32; }
+    acc = w0;
+    have = n;
+  }
+  if (have) words[k] = acc;
+}
+
+// Packs a group's 32 fields (width B) into its B words at stg.  acc holds the bits so far at its top
+// and older bits below them: one funnel shift appends a field (whatever lies above its B bits is
+// shifted out), and a word is complete when 32 bits have come in.
+template <int B>
+__device__ __forceinline__ void cg_pack(const uint32_t (&fl)[32], uint32_t* __restrict__ stg) {
+  uint32_t acc = 0u;
+#pragma unroll
+  for (int f = 0; f < 32; f++) {
+    const int sh = (f * B) & 31;  // bits of the open word
+    if (sh + B < 32) {
+      acc = __funnelshift_r(acc, fl[f], B);
+    } else {
+      stg[(f * B) >> 5] = __funnelshift_r(acc, fl[f], 32 - sh);
+      acc = fl[f] << (32 - B);
+    }
+  }
+}
+
+__device__ __forceinline__ void cg_pack_dispatch(int b, const uint32_t (&fl)[32], uint32_t* __restrict__ stg) {
+  switch (b) {
+#define GLC_CG_PACK(B) \
+  case B: cg_pack<B>(fl, stg); break;
+    GLC_CG_PACK(1) GLC_CG_PACK(2) GLC_CG_PACK(3) GLC_CG_PACK(4) GLC_CG_PACK(5) GLC_CG_PACK(6) GLC_CG_PACK(7)
+    GLC_CG_PACK(8) GLC_CG_PACK(9) GLC_CG_PACK(10) GLC_CG_PACK(11) GLC_CG_PACK(12) GLC_CG_PACK(13) GLC_CG_PACK(14)
+    GLC_CG_PACK(15) GLC_CG_PACK(16) GLC_CG_PACK(17) GLC_CG_PACK(18) GLC_CG_PACK(19) GLC_CG_PACK(20)
+    GLC_CG_PACK(21) GLC_CG_PACK(22) GLC_CG_PACK(23) GLC_CG_PACK(24) GLC_CG_PACK(25) GLC_CG_PACK(26)
+    GLC_CG_PACK(27) GLC_CG_PACK(28) GLC_CG_PACK(29) GLC_CG_PACK(30) GLC_CG_PACK(31)
+#undef GLC_CG_PACK
+    default: break;  // width 0: no words
+  }
+}
+
+template <typename T> __global__ void __launch_bounds__(kCgThreads, 6)
+fixed_compress_kernel(const __grid_constant__ FixedCompressArgs a) {
+  extern __shared__ __align__(128) uint8_t stage[];
+  __shared__ long long s_acc[kCfMaxSegs][4];  // the segments' exact partial sums and range flags
+  __shared__ uint32_t s_flag[kCfMaxSegs];
+  __shared__ double s_t0[kCfMaxParts], s_t1[kCfMaxParts], s_c[kCfMaxParts];
+  __shared__ long long s_ci[kCfMaxParts];
+  __shared__ int s_mode[kCfMaxParts];
+  __shared__ unsigned long long s_mx[kCfMaxSegs];
+  const int tid = threadIdx.x, lane = tid & 31;
+
+  const int64_t item = blockIdx.x;
+  const CfColumn& col = a.cols ? a.cols[a.owner ? a.owner[item] : 0] : a.single;
+  const int64_t t = item - col.item_base, e0 = t * kDecodeTile;
+  const int64_t left = col.n - e0;
+  const int cnt = (int)(left < kDecodeTile ? left : kDecodeTile);
+  const int L = col.L, lg = 31 - __clz(L) - 5;  // groups per partition: 2^lg, 8 to 128
+  const int np = (cnt + L - 1) / L;
+  const int p = tid >> lg, i0 = 32 * (tid & ((1 << lg) - 1));  // this group's partition, its first index there
+  const int lgW = lg < 5 ? lg : 5, W = 1 << lgW;               // lanes of a reduction segment
+  const int seg = tid >> lgW, segs = 1 << (lg - lgW);          // segments of a partition: 1, 2 or 4
+  const int glen = cnt - 32 * tid < 32 ? cnt - 32 * tid : 32;  // values of the group (<= 0: none)
+  uint8_t* row = stage + tid * cg_row_bytes<T>();
+
+  cg_load<T>(stage, reinterpret_cast<const T*>(col.values) + e0, cnt, tid);
+  __syncthreads();
+
+  {  // ---- A: exact sums and range flags per segment ----
+    HalfSums<T> hs;
+    uint32_t flag = 0;
+    cg_sums<T>(row, i0, hs, flag);
+    // a warp's sum by 24-bit limbs holds for partials below 2^50 (the high limb below 2^26 a lane)
+    const long long c0 = seg_sum48((long long)hs.s_lo, W);
+    const long long c1 = sizeof(T) == 8 ? seg_sum48((long long)hs.s_hi, W) : 0;
+    const long long c2 = seg_sum48((long long)hs.x_lo, W);
+    const long long c3 = sizeof(T) == 8 ? seg_sum48((long long)hs.x_hi, W) : 0;
+    flag = TypeTraits<T>::is_signed ? seg_or_u32(flag, W) : seg_max_u32(flag, W);
+    if ((tid & (W - 1)) == 0) {
+      s_acc[seg][0] = c0;
+      s_acc[seg][1] = c1;
+      s_acc[seg][2] = c2;
+      s_acc[seg][3] = c3;
+      s_flag[seg] = flag;
+    }
+  }
+  __syncthreads();
+  if (tid < np) {  // ---- the lines ----
+    long long a0 = 0, a1 = 0, a2 = 0, a3 = 0;
+    uint32_t flag = 0;
+    for (int s = tid * segs; s < (tid + 1) * segs; s++) {
+      a0 += s_acc[s][0];
+      a1 += s_acc[s][1];
+      a2 += s_acc[s][2];
+      a3 += s_acc[s][3];
+      flag = TypeTraits<T>::is_signed ? (flag | s_flag[s]) : (s_flag[s] > flag ? s_flag[s] : flag);
+    }
+    const int len = (cnt - tid * L) < L ? (cnt - tid * L) : L;
+    bool ovf = false;  // a uint64 value above 2^53: direct copy
+    if (!TypeTraits<T>::is_signed && sizeof(T) == 8) {
+      ovf = flag > 0x200000u;
+      if (flag == 0x200000u)
+        for (int j = tid * L; j < tid * L + len && !ovf; j++)
+          ovf = (uint64_t)*reinterpret_cast<const T*>(stage + cg_at<T>(j)) > (1ull << 53);
+    }
+    const bool vsafe = sizeof(T) == 4 || flag < 0x80000u;
+    double t0 = 0.0, t1 = 0.0, c = 0.0;
+    long long ci = 0;
+    int mode = CF_DIRECT;
+    if (!ovf) {
+      solve_line(len, (i128)a0 + (i128)a1 * ((i128)1 << 32), (i128)a2 + (i128)a3 * ((i128)1 << 32), t0, t1);
+      mode = cf_mode<T>(t0, t1, len, vsafe, c, ci);
+    }
+    s_t0[tid] = t0;
+    s_t1[tid] = t1;
+    s_c[tid] = c;
+    s_ci[tid] = ci;
+    s_mode[tid] = mode;
   }
   __syncthreads();
 
-  const int tid = threadIdx.x, lane = tid & 31;
-  if (tid >= kCfThreads + 32) {  // ---- solver warp ----
-    for (int k = 0;; k++) {
-      const int st = k % S;
-      int ok = 1;
-      if (lane == 0) {
-        ok = mbar_wait_sleep(&sums[st], (uint32_t)(k / S) & 1u);
-        if (!ok) atomicExch(a.status, (unsigned long long)DEVERR_TIMEOUT);
+  // ---- B: the residuals: low 32 bits kept, max |residual| per segment ----
+  uint32_t fl[32];
+  bool slow = false;
+  {
+    unsigned long long mx = 0;
+    if (glen > 0) {
+      const int mode = s_mode[p];
+      const double t0 = s_t0[p], t1 = s_t1[p];
+      uint32_t mag = 0u;
+      bool ok = glen == 32;
+      if (ok) {
+        if (mode == CF_NONNEG) ok = cg_resid<T, CF_NONNEG>(row, i0, t0, t1, 0.0, 0, fl, mag);
+        else if (TypeTraits<T>::is_signed && mode == CF_NONPOS) ok = cg_resid<T, CF_NONPOS>(row, i0, t0, t1, 0.0, 0, fl, mag);
+        else if (sizeof(T) == 8 && mode == CF_OFFSET) ok = cg_resid<T, CF_OFFSET>(row, i0, t0, t1, s_c[p], s_ci[p], fl, mag);
+        else ok = false;
       }
-      if (!__shfl_sync(FULL_MASK, ok, 0)) return;
-      const int64_t item = s_stile[st];
-      if (item < 0) return;
-      const CfGeom q = cf_geom(a, item, s_scol[st]);
-      if (lane < q.np) {  // lane p fits partition p (fit.cu's arithmetic) and picks its residual mode
-        const int p = lane;
-        long long a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-        uint32_t flag = 0;
-        for (int s = p * q.segs_per_part; s < (p + 1) * q.segs_per_part; s++) {
-          a0 += s_acc[st][s][0];
-          a1 += s_acc[st][s][1];
-          a2 += s_acc[st][s][2];
-          a3 += s_acc[st][s][3];
-          flag = TypeTraits<T>::is_signed ? (flag | s_flag[st][s]) : (s_flag[st][s] > flag ? s_flag[st][s] : flag);
+      mx = mag;
+      slow = !ok;
+      if (slow && mode != CF_DIRECT) {
+        mx = 0;
+const double c = s_c[p];
+        const long long ci = s_ci[p];
+        double xi = (double)i0;
+#pragma unroll 1
+        for (int f = 0; f < glen; f++) {
+          const T y = *reinterpret_cast<const T*>(row + f * (int)sizeof(T));
+          const unsigned long long ad = (unsigned long long)abs_ref(cg_field<T>(y, xi, mode, t0, t1, c, ci));
+          xi = __dadd_rn(xi, 1.0);
+          mx = ad > mx ? ad : mx;
         }
-        const int len = (q.cnt - p * q.L) < q.L ? (q.cnt - p * q.L) : q.L;
-        const T* xp = reinterpret_cast<const T*>(smem + (size_t)st * cf_stage_bytes<T>() + s_shead[st]) + p * q.L;
-        const bool ovf = cf_overflows<T>(flag, xp, len);  // a value above 2^53: direct copy
-        const bool vsafe = sizeof(T) == 4 || flag < 0x80000u;
-        double t0 = 0.0, t1 = 0.0, c = 0.0;
-        long long ci = 0;
-        int mode = CF_DIRECT;
-        if (!ovf) {
-          solve_line(len, (i128)a0 + (i128)a1 * ((i128)1 << 32), (i128)a2 + (i128)a3 * ((i128)1 << 32), t0, t1);
-          mode = cf_mode<T>(t0, t1, len, vsafe, c, ci);
-        }
-        s_t0[st][p] = t0;
-        s_t1[st][p] = t1;
-        s_c[st][p] = c;
-        s_ci[st][p] = ci;
-        s_mode[st][p] = mode;
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&lines[st]);
+    }
+    mx = seg_max_u64(mx, W);
+    if ((tid & (W - 1)) == 0) s_mx[seg] = mx;
+  }
+  slow = __syncthreads_or(slow);
+
+  // ---- widths and tile-relative offsets: lane q of every warp for partition q ----
+  int b = 0, bl = 0, total;
+  {
+    int nb = 0;
+    unsigned long long m = 0;
+    if (lane < np) {
+      for (int s = lane * segs; s < (lane + 1) * segs; s++) m = s_mx[s] > m ? s_mx[s] : m;
+      const bool direct = s_mode[lane] == CF_DIRECT;
+      b = direct ? (int)sizeof(T) * 8 : bits_for((long long)m);
+      if (direct) m = 0;
+      nb = ((cnt - lane * L) < L ? (cnt - lane * L) : L) * b;
+    }
+    int inc = nb;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(FULL_MASK, inc, o);
+      if (lane >= o) inc += v;
+    }
+    bl = inc - nb;
+    total = __shfl_sync(FULL_MASK, inc, 31);
+    const int bmax = (int)__reduce_max_sync(FULL_MASK, (unsigned)b);
+    slow = slow || bmax > 31;
+    if (tid < np) {
+      // the descriptor with the tile-relative offset and the max error; fixed_place_kernel
+      // completes the offset and writes the other metadata arrays from the descriptor
+      const int64_t gp = t * col.parts_per_tile + tid;
+      PartDesc d;
+      d.theta0 = s_t0[tid];
+      d.theta1 = s_t1[tid];
+      d.bit_off = bl;
+      d.start = (int32_t)(e0 + (int64_t)tid * L);
+      d.bits_type = (b & 0xff) | ((s_mode[tid] == CF_DIRECT ? MODEL_DIRECT_COPY : MODEL_LINEAR) << 8);
+      col.desc[gp] = d;
+      col.err[gp] = (long long)m;
+    }
+    if (tid == 0) {
+      a.tile_bits[item] = total;
+      if (bmax > 0) atomicMax(col.stats + 1, (unsigned long long)bmax);
     }
   }
-  if (tid >= kCfThreads) {  // ---- producer ----
-    if (tid == kCfThreads) cf_produce<T, S>(a, smem, full, empty, s_stile, s_shead, s_scol);
+
+  uint32_t* out = a.slots + item * a.slot_words;
+  const int bp = __shfl_sync(FULL_MASK, b, p & 31), blp = __shfl_sync(FULL_MASK, bl, p & 31);
+  if (!slow) {
+    // ---- C: the group's words, staged over its warp's rows (read by no other warp), then to the
+    // slot, a reduction segment at a time: its groups are consecutive words of one partition.  Groups
+    // lie b words apart, or b + 1 for an even b, so that the lanes' stores fall on different banks ----
+    uint32_t* stg = reinterpret_cast<uint32_t*>(stage + (tid & ~31) * cg_row_bytes<T>());
+    __syncwarp();
+    if (glen > 0) cg_pack_dispatch(bp, fl, stg + (lane & ~(W - 1)) * 32 + (lane & (W - 1)) * (bp | 1));
+    __syncwarp();
+    const int o0 = (blp >> 5) + (i0 >> 5) * bp;  // this group's first word in the tile
+    for (int l = 0; l < 32; l += W) {
+      const int bs = __shfl_sync(FULL_MASK, bp, l), os = __shfl_sync(FULL_MASK, o0, l);
+      const int groups = __popc(__ballot_sync(FULL_MASK, glen > 0) >> l & (uint32_t)((1ull << W) - 1ull));
+      const int nw = groups * bs, pad = (bs & 1) ^ 1;
+      const uint32_t mb = bs > 1 ? 0xffffffffu / (uint32_t)bs + 1u : 0u;  // w / b by a multiply-high (w < 2^10)
+      const uint32_t* q = stg + l * 32;
+      uint32_t* ow = out + os;  // 16-byte aligned: a segment holds at least 8 groups
+      for (int w = 4 * lane; w + 3 < nw; w += 128) {
+        uint32_t v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = q[w + u + (pad ? (int)__umulhi((uint32_t)(w + u), mb) : 0)];
+        *reinterpret_cast<uint4*>(ow + w) = make_uint4(v[0], v[1], v[2], v[3]);
+      }
+      const int w = (nw & ~3) + lane;
+      if (w < nw) ow[w] = q[w + (pad ? (int)__umulhi((uint32_t)w, mb) : 0)];
+    }
     return;
   }
-
-  // ---- compute warps ----
-  // the exact sums of the tile in stage st into s_acc[st] / s_flag[st], then each warp arrives on
-  // sums[st] (an end marker is passed on unsummed, so the solver sees the end too)
-  auto stage_sums = [&](int st) {
-    const int64_t item = s_stile[st];
-    if (item >= 0) {
-      const CfGeom q = cf_geom(a, item, s_scol[st]);
-      const int p_me = tid >> q.lg_g, r_me = tid & (q.g - 1);
-      const int my_len = p_me < q.np ? ((q.cnt - p_me * q.L) < q.L ? (q.cnt - p_me * q.L) : q.L) : 0;
-      const T* xp = reinterpret_cast<const T*>(smem + (size_t)st * cf_stage_bytes<T>() + s_shead[st]) + p_me * q.L;
-      HalfSums<T> hs;
-      uint32_t flag = 0;
-      if (my_len == q.L) cf_sums<T, true>(xp, r_me, q.g, q.L, hs, flag);
-      else if (my_len > 0) cf_sums<T, false>(xp, r_me, q.g, my_len, hs, flag);
-      // every partial is below 2^48 in magnitude (16 values, i < 2^12, 32-bit halves)
-      const long long c0 = seg_sum48((long long)hs.s_lo, q.W);
-      const long long c1 = sizeof(T) == 8 ? seg_sum48((long long)hs.s_hi, q.W) : 0;
-      const long long c2 = seg_sum48((long long)hs.x_lo, q.W);
-      const long long c3 = sizeof(T) == 8 ? seg_sum48((long long)hs.x_hi, q.W) : 0;
-      flag = TypeTraits<T>::is_signed ? seg_or_u32(flag, q.W) : seg_max_u32(flag, q.W);
-      if ((tid & (q.W - 1)) == 0) {
-        const int seg = tid >> q.lg_W;
-        s_acc[st][seg][0] = c0;
-        s_acc[st][seg][1] = c1;
-        s_acc[st][seg][2] = c2;
-        s_acc[st][seg][3] = c3;
-        s_flag[st][seg] = flag;
-      }
+  // ---- slow path: each group's words in its own row, then to the slot, one thread per word ----
+  if (glen > 0 && bp > 0) cg_pack_slow<T>(row, glen, i0, bp, s_mode[p], s_t0[p], s_t1[p], s_c[p], s_ci[p]);
+  __syncthreads();
+  for (int q = 0; q < np; q++) {
+    const int bq = __shfl_sync(FULL_MASK, b, q), blq = __shfl_sync(FULL_MASK, bl, q);
+    if (bq <= 0) continue;
+    const int len = (cnt - q * L) < L ? (cnt - q * L) : L;
+    const int nwp = (int)(((long long)len * bq + 31) >> 5);
+    const uint32_t mb = bq > 1 ? 0xffffffffu / (uint32_t)bq + 1u : 0u;  // w / b by a multiply-high (w < 2^13)
+    const uint8_t* rows = stage + (q << lg) * cg_row_bytes<T>();
+    uint32_t* ow = out + (blq >> 5);
+    for (int w = tid; w < nwp; w += kCgThreads) {
+      const int g = bq > 1 ? (int)__umulhi((uint32_t)w, mb) : w;
+      ow[w] = *reinterpret_cast<const uint32_t*>(rows + g * cg_row_bytes<T>() + 4 * (w - g * bq));
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sums[st]);
-  };
-  // tid 0 waits for a phase; every compute thread learns the outcome after the barrier
-  auto wait_all = [&](uint64_t* bar, uint32_t par) {
-    if (tid == 0) {
-      s_ok = mbar_wait_sleep(bar, par);
-      if (!s_ok) atomicExch(a.status, (unsigned long long)DEVERR_TIMEOUT);
-    }
-  };
-
-  if (tid == 0) {
-    s_ok = mbar_wait_sleep(&full[0], 0);
-    if (!s_ok) {
-      atomicExch(a.status, (unsigned long long)DEVERR_TIMEOUT);
-      mbar_wait_bounded(&full[0], 0);  // a copy in flight lands before the CTA exits
-    }
-  }
-  cf_sync();
-  if (!s_ok) return;
-  mbar_try_wait(&full[0], 0);  // the phase is complete: orders this thread's reads after the copy
-  if (s_stile[0] < 0) return;
-  stage_sums(0);
-
-  for (int k = 0;; k++) {
-    const int st = k % S, st1 = (k + 1) % S;
-    const uint32_t par = (uint32_t)(k / S) & 1u, par1 = (uint32_t)((k + 1) / S) & 1u;
-    // the next tile's values and this tile's lines
-    if (tid == 0) {
-      s_ok = mbar_wait_sleep(&full[st1], par1);
-      if (!s_ok) {
-        atomicExch(a.status, (unsigned long long)DEVERR_TIMEOUT);
-        mbar_wait_bounded(&full[st1], par1);  // a copy in flight lands before the CTA exits
-      } else {
-        wait_all(&lines[st], par);
-      }
-    }
-    cf_sync();
-    if (!s_ok) return;
-    mbar_try_wait(&full[st1], par1);
-    mbar_try_wait(&lines[st], par);
-    const int64_t item1 = s_stile[st1];
-    stage_sums(st1);
-
-    const int64_t item = s_stile[st];
-    const CfGeom q = cf_geom(a, item, s_scol[st]);
-    const CfColumn& col = *q.col;
-    const int L = q.L, g = q.g, W = q.W, np = q.np, cnt = q.cnt;
-    const int64_t t = q.t, e0 = q.e0;
-    const int seg = tid >> q.lg_W, segs_per_part = q.segs_per_part;
-    const int p_me = tid >> q.lg_g, r_me = tid & (g - 1);
-    uint8_t* stage = smem + (size_t)st * cf_stage_bytes<T>();
-    T* x = reinterpret_cast<T*>(stage + s_shead[st]);
-    // the fields and staged words of the fast packing: over the stage for 8-byte types (its values
-    // are dead by then), in the work area for 4-byte types
-    uint8_t* work = sizeof(T) == 8 ? stage : smem + (size_t)S * cf_stage_bytes<T>();
-    const int my_len = p_me < np ? ((cnt - p_me * L) < L ? (cnt - p_me * L) : L) : 0;
-    const T* xp = x + p_me * L;
-
-    // ---- B: residual of every value: its low 32 bits kept, max |residual| per partition ----
-    uint32_t fl[kCfPerThread];
-    bool wide;
-    {
-      unsigned long long mx = 0;
-#pragma unroll
-      for (int m = 0; m < kCfPerThread; m++) fl[m] = 0u;
-      if (my_len > 0) {
-        const int mode = s_mode[st][p_me];
-        const double t0 = s_t0[st][p_me], t1 = s_t1[st][p_me];
-        bool general = mode == CF_GENERAL;
-        if (mode == CF_NONNEG) {
-          mx = my_len == L ? cf_resid_sign<T, true, false>(xp, r_me, g, L, t0, t1, fl)
-                           : cf_resid_sign<T, false, false>(xp, r_me, g, my_len, t0, t1, fl);
-        } else if (TypeTraits<T>::is_signed && mode == CF_NONPOS) {
-          mx = my_len == L ? cf_resid_sign<T, true, true>(xp, r_me, g, L, t0, t1, fl)
-                           : cf_resid_sign<T, false, true>(xp, r_me, g, my_len, t0, t1, fl);
-        } else if (sizeof(T) == 8 && mode == CF_OFFSET) {
-          const double c = s_c[st][p_me];
-          const long long ci = s_ci[st][p_me];
-          general = !(my_len == L ? cf_resid_offset<T, true>(xp, r_me, g, L, t0, t1, c, ci, fl, mx)
-                                  : cf_resid_offset<T, false>(xp, r_me, g, my_len, t0, t1, c, ci, fl, mx));
-        }
-        if (general) mx = cf_resid_general<T>(xp, r_me, g, my_len, t0, t1, fl);
-      }
-      mx = seg_max_u64(mx, W);
-      if ((tid & (W - 1)) == 0) s_mx[seg] = mx;
-      // a width above 31 anywhere in the tile (a max |residual| of 2^30 or more, or direct copy)
-      wide = my_len > 0 && (s_mode[st][p_me] == CF_DIRECT || mx >= (1ull << 30));
-    }
-    wide = cf_sync_or(wide);
-    if (tid < 32) {  // widths, tile-relative bit ranges (a warp scan), descriptors, the tile's bits
-      const int p = lane;
-      int b = 0, nb = 0;
-      unsigned long long err = 0;
-      if (p < np) {
-        unsigned long long m = 0;
-        for (int s = p * segs_per_part; s < (p + 1) * segs_per_part; s++) m = s_mx[s] > m ? s_mx[s] : m;
-        const bool direct = s_mode[st][p] == CF_DIRECT;
-        b = direct ? (int)sizeof(T) * 8 : bits_for((long long)m);
-        err = direct ? 0 : m;
-        nb = ((cnt - p * L) < L ? (cnt - p * L) : L) * b;
-      }
-      int inc = nb;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(FULL_MASK, inc, o);
-        if (lane >= o) inc += v;
-      }
-      const int bl = inc - nb;
-      const int bmax = (int)__reduce_max_sync(FULL_MASK, (unsigned)b);
-      const int total = __shfl_sync(FULL_MASK, inc, 31);
-      if (p < np) {
-        s_bl[p] = bl;
-        s_b[p] = b;
-        // the descriptor with the tile-relative offset and the max error; fixed_place_kernel
-        // completes the offset and writes the other metadata arrays from the descriptor
-        const int64_t gp = t * col.parts_per_tile + p;
-        PartDesc d;
-        d.theta0 = s_t0[st][p];
-        d.theta1 = s_t1[st][p];
-        d.bit_off = bl;
-        d.start = (int32_t)(e0 + (int64_t)p * L);
-        d.bits_type = (b & 0xff) | ((s_mode[st][p] == CF_DIRECT ? MODEL_DIRECT_COPY : MODEL_LINEAR) << 8);
-        col.desc[gp] = d;
-        col.err[gp] = (long long)err;
-      }
-      if (lane == 0) {
-        s_bl[np] = total;
-        a.tile_bits[item] = total;
-        if (bmax > 0) atomicMax(col.stats + 1, (unsigned long long)bmax);
-      }
-    }
-    // (the widths are not needed by the field writes or the residual recompute below: they run
-    // beside warp 0's section and one barrier covers both)
-
-    uint32_t* out = a.slots + item * a.slot_words;
-    if (!wide) {
-      // ---- C (every width <= 31): fields transposed, one thread packs each 32-value group into
-      // its `width` words (every partition starts on a word: L is a multiple of 32), staged, then
-      // copied to the slot with coalesced stores ----
-      uint32_t* fT = reinterpret_cast<uint32_t*>(work);
-      uint32_t* stg = fT + kFtWords;
-      if (g >= 32) {  // g a multiple of 32: position j = p_me L + r_me + g m has j % 32 = lane
-        uint32_t* fp = fT + lane * kFtStride + ((p_me * L + r_me) >> 5);
-        const int step = g >> 5;
-#pragma unroll
-        for (int m = 0; m < kCfPerThread; m++) fp[m * step] = fl[m];
-      } else {
-#pragma unroll
-        for (int m = 0; m < kCfPerThread; m++) {
-          const int j = p_me * L + r_me + g * m;  // position in the tile (the threads cover all 4096)
-          fT[(j & 31) * kFtStride + (j >> 5)] = fl[m];
-        }
-      }
-      cf_sync();
-      if (tid < ((cnt + 31) >> 5)) {
-        const int G = tid, p = G >> (q.lg_L - 5);  // L / 32 groups per partition
-        cf_pack_dispatch(s_b[p], fT + G, stg, (s_bl[p] >> 5) + (G - (p << (q.lg_L - 5))) * s_b[p]);
-      }
-      cf_sync();
-      const int nw = (s_bl[np] + 31) >> 5;
-      for (int w = tid; w < nw; w += kCfThreads) out[w] = stg[w + (w >> 5)];
-    } else {
-      // ---- C (a width above 31): the exact 64-bit residuals over the values (8-byte types) or in
-      // the work area, then per partition one thread per word of the slot ----
-      long long* res = sizeof(T) == 8 ? reinterpret_cast<long long*>(x) : reinterpret_cast<long long*>(work);
-      if (my_len > 0)
-        cf_store_resid<T>(xp, res + p_me * L, r_me, g, my_len, s_mode[st][p_me], s_t0[st][p_me], s_t1[st][p_me]);
-      cf_sync();
-      for (int p = 0; p < np; p++)
-        cf_words_dispatch(s_b[p], res + p * L, (cnt - p * L) < L ? (cnt - p * L) : L, out + (s_bl[p] >> 5), tid);
-    }
-    cf_sync();  // every compute thread is done with stage st and the work area
-    if (tid == 0) mbar_arrive(&empty[st]);
-    if (item1 < 0) return;
   }
 }
 
@@ -1222,35 +1330,18 @@ __global__ void __launch_bounds__(kPlaceThreads, 8) fixed_place_kernel(FixedComp
   }
 }
 
-template <typename T> static cudaError_t launch_fixed_compress_t(const FixedCompressArgs& a, int num_sms, cudaStream_t s) {
-  constexpr int smem = cf_fix_smem_bytes<T>(kCfCompressStages);
-  static PerDeviceFlag attr_set;  // per instantiation and device
-  const int dev = current_device();
-  cudaError_t e;
-  if (!attr_set.test(dev)) {
-    if ((e = cudaFuncSetAttribute(fixed_compress_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) !=
-        cudaSuccess)
-      return e;
-    attr_set.set(dev);
-  }
-  int per_sm = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fixed_compress_kernel<T>, kCfFixCTA, smem)) !=
-      cudaSuccess)
-    return e;
-  if (per_sm < 1) per_sm = 1;
-  int64_t grid = (int64_t)per_sm * num_sms;
-  if (grid > a.nitems) grid = a.nitems;
-  if (grid < 1) grid = 1;
-  fixed_compress_kernel<T><<<(unsigned)grid, kCfFixCTA, smem, s>>>(a);
+template <typename T> static cudaError_t launch_fixed_compress_t(const FixedCompressArgs& a, cudaStream_t s) {
+  // (34 KB per CTA for 8-byte types, 18 KB for 4-byte ones: within the default limit)
+  fixed_compress_kernel<T><<<(unsigned)a.nitems, kCgThreads, cg_stage_bytes<T>(), s>>>(a);
   return cudaGetLastError();
 }
 
-static cudaError_t launch_fixed_compress_dt(glc_dtype dt, const FixedCompressArgs& a, int num_sms, cudaStream_t s) {
+static cudaError_t launch_fixed_compress_dt(glc_dtype dt, const FixedCompressArgs& a, cudaStream_t s) {
   switch (dt) {
-    case GLC_I32: return launch_fixed_compress_t<int32_t>(a, num_sms, s);
-    case GLC_I64: return launch_fixed_compress_t<int64_t>(a, num_sms, s);
-    case GLC_U64: return launch_fixed_compress_t<uint64_t>(a, num_sms, s);
-    case GLC_U32: return launch_fixed_compress_t<uint32_t>(a, num_sms, s);
+    case GLC_I32: return launch_fixed_compress_t<int32_t>(a, s);
+    case GLC_I64: return launch_fixed_compress_t<int64_t>(a, s);
+    case GLC_U64: return launch_fixed_compress_t<uint64_t>(a, s);
+    case GLC_U32: return launch_fixed_compress_t<uint32_t>(a, s);
   }
   return cudaErrorInvalidValue;
 }
@@ -1337,14 +1428,14 @@ static void carve(FixedCompressArgs& a, glc_dtype dt, void* scratch) {
 }
 
 // Pass 1 for one launch: fit, residuals and each tile's words into its slot, the tiles' bits, and
-// their exclusive scan (tile_first[nitems] = all the launch's bits).
-static cudaError_t compress_pass(glc_dtype dt, FixedCompressArgs& a, void* scratch, int num_sms, cudaStream_t s) {
+// their exclusive scan (all the launch's bits into *total where it is given).
+static cudaError_t compress_pass(glc_dtype dt, FixedCompressArgs& a, void* scratch, int64_t* total, cudaStream_t s) {
   carve(a, dt, scratch);
   cudaError_t e;
-  if ((e = launch_fixed_compress_dt(dt, a, num_sms, s)) != cudaSuccess) return e;
+  if ((e = launch_fixed_compress_dt(dt, a, s)) != cudaSuccess) return e;
   int64_t* first = const_cast<int64_t*>(a.tile_first);
   int64_t* tmp = first + a.nitems + 1;
-  return exclusive_scan<int64_t>(a.tile_bits, first, a.nitems, first + a.nitems, tmp, s);
+  return exclusive_scan<int64_t>(a.tile_bits, first, a.nitems, total, tmp, s);
 }
 
 static cudaError_t place_pass(const FixedCompressArgs& a, int num_sms, cudaStream_t s) {
@@ -1385,9 +1476,8 @@ cudaError_t launch_fixed_compress(glc_dtype dt, const void* values, glc_column* 
   a.status = stats + 2;
   cudaError_t e;
   if ((e = cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned long long), s)) != cudaSuccess) return e;
-  if ((e = compress_pass(dt, a, scratch, c->ctx ? c->ctx->num_sms : 148, s)) != cudaSuccess) return e;
   // the total: the scan's grand total (the column is the whole launch)
-  return cudaMemcpyAsync(stats, a.tile_first + a.nitems, sizeof(int64_t), cudaMemcpyDeviceToDevice, s);
+  return compress_pass(dt, a, scratch, (int64_t*)stats, s);
 }
 
 // Pass 2 for one column: its words into c->d_words (c->nwords_alloc words), its offsets, descriptors
@@ -1436,7 +1526,7 @@ cudaError_t launch_place_prepacked(glc_dtype dt, const CfColumn* cols, const int
   a.terr = terr;
   carve(a, dt, scratch);
   int64_t* first = const_cast<int64_t*>(a.tile_first);
-  cudaError_t e = exclusive_scan<int64_t>(a.tile_bits, first, a.nitems, first + a.nitems, first + a.nitems + 1, s);
+  cudaError_t e = exclusive_scan<int64_t>(a.tile_bits, first, a.nitems, nullptr, first + a.nitems + 1, s);
   if (e != cudaSuccess) return e;
   return place_pass(a, num_sms, s);
 }
@@ -1453,7 +1543,7 @@ cudaError_t launch_fixed_compress_batch(glc_dtype dt, const CfColumn* cols, cons
   a.nitems = nitems;
   a.status = status;
   cudaError_t e;
-  if ((e = compress_pass(dt, a, scratch, num_sms, s)) != cudaSuccess) return e;
+  if ((e = compress_pass(dt, a, scratch, nullptr, s)) != cudaSuccess) return e;
   return place_pass(a, num_sms, s);
 }
 

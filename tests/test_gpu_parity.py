@@ -529,3 +529,25 @@ def test_serialize_into_device_memory(oracle, glc_ctx, kind, n, mode, offset):
     assert size.value == len(blob) and got[offset:offset + len(blob)] == blob
     assert set(got[:offset] + got[offset + len(blob):]) == {0xA5}
     col.free()
+
+
+@pytest.mark.parametrize("L", [256, 512, 1024, 2048, 4096])
+@pytest.mark.parametrize("n", [31, 32, 33, 4095, 4096 + 32, 3 * 4096 + 2080, 50_017])
+def test_fixed_compress_groups(oracle, glc_ctx, L, n):
+    """Tiles whose partitions mix narrow widths, widths above 31 and incomplete 32-value groups, from values
+    aligned to 16 bytes and to their own size only."""
+    torch = pytest.importorskip("torch")
+    base = _jumps(n, seed=n + L)
+    for dtype in (np.int64, np.uint64, np.int32, np.uint32):
+        v = base if dtype == np.int64 else base.astype(dtype) if np.dtype(dtype).itemsize == 8 else (base & 0x7FFFFFFF).astype(dtype)
+        if dtype == np.int64:
+            v = np.where((np.arange(n) // 900) % 2 == 0, v, -v)
+        code = {"int32": glc.I32, "int64": glc.I64, "uint64": glc.U64, "uint32": glc.U32}[v.dtype.name]
+        want = oracle.serialize(oracle.compress(v, "fixed", L))
+        for shift in (0, 1):
+            buf = torch.from_numpy(np.concatenate([np.zeros(shift, v.dtype), v]).view(np.int64 if v.itemsize == 8 else np.int32)).cuda()
+            torch.cuda.synchronize()
+            col = glc.compress_device(glc_ctx, code, buf.data_ptr() + shift * v.itemsize, n, glc.FIXED, fixed_len=L)
+            got = glc.serialize_host(glc_ctx, col)
+            col.free()
+            assert got == want
