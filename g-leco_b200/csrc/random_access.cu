@@ -56,15 +56,18 @@ __device__ __forceinline__ uint64_t read_field_global(const uint32_t* __restrict
   return low_bits(f, bits);
 }
 
+// A descriptor is one 32-byte access (the arrays are 32-byte aligned): a warp's lookups land on
+// different lines, so every access costs the L1 a tag lookup per lane, and two 16-byte halves cost
+// two (100M lookups into 64M int64 values: 1038 -> 942 us).  The field's words stay with 16 bytes:
+// its whole sector in one access measured slower (997 us).
 __device__ __forceinline__ PartDesc load_desc(const PartDesc* __restrict__ d) {
-  const double2 a = __ldg(reinterpret_cast<const double2*>(d));
-  const longlong2 b = __ldg(reinterpret_cast<const longlong2*>(d) + 1);
+  const Bytes32 x = load32_nc(d);
   PartDesc r;
-  r.theta0 = a.x;
-  r.theta1 = a.y;
-  r.bit_off = b.x;
-  r.start = (int32_t)(b.y & 0xffffffffll);
-  r.bits_type = (int32_t)(b.y >> 32);
+  r.theta0 = __longlong_as_double((long long)x.q[0]);
+  r.theta1 = __longlong_as_double((long long)x.q[1]);
+  r.bit_off = (int64_t)x.q[2];
+  r.start = (int32_t)(uint32_t)x.q[3];
+  r.bits_type = (int32_t)(x.q[3] >> 32);
   return r;
 }
 
@@ -196,8 +199,8 @@ static cudaError_t ra_shape(glc_ctx* ctx, const RAArgs& a, int mode, cudaStream_
 }
 
 // Launch shapes (lookups per thread, CTAs per SM): 0 = (4, 1), 1 = (4, 5), 2 = (2, 8), 3 = (8, 2),
-// 4 = (2, 6).  The untuned defaults were measured on 100M lookups into a 64M int64 column: packed
-// fields -> shape 4 (40 registers, more warps resident); pre-unpacked residuals (every lookup a
+// 4 = (2, 6), 5 = (1, 6; small calls).  The untuned defaults were measured on 100M lookups into a
+// 64M int64 column: packed fields -> shape 4 (40 registers, more warps resident); pre-unpacked residuals (every lookup a
 // DRAM sector) -> shape 3.  The context's tuning table picks per element type and field width;
 // GLC_RA_SHAPE overrides it for sweeps.
 template <typename T, bool PLAIN>
@@ -207,6 +210,7 @@ static cudaError_t ra_typed(glc_ctx* ctx, const RAArgs& a, int mode, int shape, 
     case 2: return ra_shape<T, PLAIN, 2, 8>(ctx, a, mode, s);
     case 3: return ra_shape<T, PLAIN, 8, 2>(ctx, a, mode, s);
     case 4: return ra_shape<T, PLAIN, 2, 6>(ctx, a, mode, s);
+    case 5: return ra_shape<T, PLAIN, 1, 6>(ctx, a, mode, s);
     default: return ra_shape<T, PLAIN, 4, 1>(ctx, a, mode, s);
   }
 }
@@ -214,7 +218,11 @@ static cudaError_t ra_typed(glc_ctx* ctx, const RAArgs& a, int mode, int shape, 
 cudaError_t launch_random_access(glc_ctx* ctx, const glc_column* c, int plain_src, const int32_t* pos, int64_t q,
                                  void* out, int32_t fixed_len, cudaStream_t s) {
   const char* v = getenv("GLC_RA_SHAPE");
-  const int shape = (v && *v) ? atoi(v) : tune_entry(ctx, c->dtype, c->max_bits, plain_src).ra_shape;
+  // A call that one lookup per thread spreads over no more than two CTAs per SM gains nothing from
+  // several lookups in a thread: their searches run one after another (10,007 lookups into a
+  // variable column: 6.8 us in shape 0, 3.3 in shape 5).
+  const bool small = q <= 2ll * kRAThreads * ctx->num_sms;
+  const int shape = (v && *v) ? atoi(v) : small ? 5 : tune_entry(ctx, c->dtype, c->max_bits, plain_src).ra_shape;
   return launch_random_access_shape(ctx, c, plain_src, pos, q, out, fixed_len, shape, s);
 }
 

@@ -551,3 +551,33 @@ def test_fixed_compress_groups(oracle, glc_ctx, L, n):
             got = glc.serialize_host(glc_ctx, col)
             col.free()
             assert got == want
+
+
+@pytest.mark.parametrize("q", [1, 255, 256, 257, 148 * 512 - 1, 148 * 512, 148 * 512 + 1, 300_001])
+@pytest.mark.parametrize("mode", ["fixed", "odd", "variable"])
+def test_lookup_counts_around_the_small_shape(glc_ctx, q, mode):
+    n = 150_007
+    v = _jumps(n, seed=q)
+    col = glc.compress_device(glc_ctx, glc.I64, v.ctypes.data, n, glc.VARIABLE if mode == "variable" else glc.FIXED,
+                              fixed_len=1000 if mode == "odd" else 1024, host=True)
+    pos = np.random.default_rng(q).integers(-5, n + 5, q).astype(np.int32)
+    want = np.where((pos >= 0) & (pos < n), v[np.clip(pos, 0, n - 1)], 0)
+    out = np.full(q, 7, np.int64)
+    glc.random_access_into(glc_ctx, col, pos.ctypes.data, q, out.ctypes.data, host_in=True, host_out=True)
+    assert np.array_equal(out, want)
+    glc.preunpack(glc_ctx, col)
+    glc.random_access_into(glc_ctx, col, pos.ctypes.data, q, out.ctypes.data, source=glc.SRC_PREUNPACKED, host_in=True, host_out=True)
+    assert np.array_equal(out, want)
+    col.free()
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 147, 148, 149, 148 * 4, 148 * 5 + 1, 148 * 8, 148 * 8 + 1, 148 * 12])
+def test_decode_tiles_around_the_resident_ctas(glc_ctx, tiles):
+    """One tile per CTA without the work counter, and more tiles than resident CTAs with it."""
+    for n in (tiles * 4096 - 1, tiles * 4096):
+        v = (np.arange(n, dtype=np.int64) * 37 + np.random.default_rng(n).integers(0, 1000, n)).astype(np.int32)
+        col = glc.compress_device(glc_ctx, glc.I32, v.ctypes.data, n, glc.FIXED, fixed_len=1024, host=True)
+        out = np.zeros(n, np.int32)
+        glc.decompress_into(glc_ctx, col, out.ctypes.data, glc.SRC_PACKED, host_out=True)
+        assert np.array_equal(out, v)
+        col.free()
