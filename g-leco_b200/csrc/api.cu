@@ -3,6 +3,7 @@
 // files.  Nothing here exits the process or falls back to host computation: every failure is a
 // glc_status with a message (the reference calls exit() on any CUDA error,
 // core/CudaUtils.cuh:5-13).
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -98,10 +99,10 @@ void free_column_arrays(glc_column* c) {
     void* ptrs[] = {c->d_plain, c->d_desc, c->d_tiles, c->owned};
     for (void* p : ptrs) col_release(c, p);
     c->owned = nullptr;
-  } else {
-    void* ptrs[] = {c->d_start, c->d_end, c->d_types, c->d_params, c->d_bits, c->d_offs, c->d_err,
-                    c->d_words, c->d_plain, c->d_desc, c->d_tiles};
+  } else {  // the metadata arrays and tables lie in one block
+    void* ptrs[] = {c->meta, c->d_words, c->d_plain};
     for (void* p : ptrs) col_release(c, p);
+    c->meta = nullptr;
   }
   c->d_start = c->d_end = c->d_types = c->d_bits = nullptr;
   c->d_params = nullptr;
@@ -111,20 +112,29 @@ void free_column_arrays(glc_column* c) {
   c->d_tiles = nullptr;
 }
 
-// Metadata arrays for P partitions and the decode tile table.
+// Metadata arrays for P partitions, the descriptors and the decode tile table, in one allocation (nine
+// took 5 us from the pool and 0.5 ms from cudaMalloc), each from a 256-byte boundary as its own
+// allocation would be: kernels store some of them in vectors.
 cudaError_t alloc_meta(glc_column* c, cudaStream_t s) {
-  const int64_t P = c->P > 0 ? c->P : 1;
-  cudaError_t e;
-  if ((e = col_alloc(c, &c->d_start, 4 * P, s)) != cudaSuccess) return e;
-  if ((e = col_alloc(c, &c->d_end, 4 * P, s)) != cudaSuccess) return e;
-  if ((e = col_alloc(c, &c->d_types, 4 * P, s)) != cudaSuccess) return e;
-  if ((e = col_alloc(c, &c->d_params, 32 * P, s)) != cudaSuccess) return e;
-  if ((e = col_alloc(c, &c->d_bits, 4 * P, s)) != cudaSuccess) return e;
-  if ((e = col_alloc(c, &c->d_offs, 8 * P, s)) != cudaSuccess) return e;
-  if ((e = col_alloc(c, &c->d_err, 8 * P, s)) != cudaSuccess) return e;
-  if ((e = col_alloc(c, &c->d_desc, sizeof(PartDesc) * P, s)) != cudaSuccess) return e;
+  const uint64_t P = c->P > 0 ? (uint64_t)c->P : 1;
   c->ntiles = (c->n + kDecodeTile - 1) / kDecodeTile;
-  if ((e = col_alloc(c, &c->d_tiles, sizeof(TileInfo) * (c->ntiles + 1), s)) != cudaSuccess) return e;
+  const uint64_t bytes[9] = {4 * P, 4 * P, 4 * P, 32 * P, 4 * P, 8 * P, 8 * P, sizeof(PartDesc) * P,
+                             sizeof(TileInfo) * ((uint64_t)c->ntiles + 1)};
+  uint64_t off[10] = {0};
+  for (int k = 0; k < 9; k++) off[k + 1] = (off[k] + bytes[k] + 255) & ~255ull;
+  uint8_t* m = nullptr;
+  cudaError_t e = col_alloc(c, &m, off[9], s);
+  if (e != cudaSuccess) return e;
+  c->meta = m;
+  c->d_start = (int32_t*)(m + off[0]);
+  c->d_end = (int32_t*)(m + off[1]);
+  c->d_types = (int32_t*)(m + off[2]);
+  c->d_params = (double*)(m + off[3]);
+  c->d_bits = (int32_t*)(m + off[4]);
+  c->d_offs = (int64_t*)(m + off[5]);
+  c->d_err = (int64_t*)(m + off[6]);
+  c->d_desc = (PartDesc*)(m + off[7]);
+  c->d_tiles = (TileInfo*)(m + off[8]);
   return cudaSuccess;
 }
 
@@ -352,7 +362,9 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
   CK(col_alloc(c, &c->d_words, 4 * c->nwords_alloc, s), "compress: word allocation");
   const int64_t parts_per_tile = ctx->h_stats[3];
   CK(launch_desc_and_tiles(c, s), "compress: tables");
-  CK(launch_pack(dtype, dev_values, c, parts_per_tile, ctx->d_flags + kFlagError, s), "compress: pack");
+  // the partitioners' starts are multiples of 128 and of kV6Base / 2
+  const bool starts32 = mode != GLC_PART_FIXED || fixed_len % 32 == 0;
+  CK(launch_pack(dtype, dev_values, c, parts_per_tile, starts32, ctx->d_flags + kFlagError, s), "compress: pack");
   c->reported_size = reported_size(c->P, c->total_bits);
   return GLC_OK;
 }
@@ -683,7 +695,12 @@ glc_status glc_serialize(glc_ctx* ctx, const glc_column* c, void* blob, uint64_t
 
 glc_status glc_deserialize(glc_ctx* ctx, glc_dtype dtype, const void* blob, uint64_t size, int flags, int crc32c,
                            int pre_unpack, glc_column** out, glc_stream stream) {
-  return glc::deserialize_column(ctx, dtype, blob, size, flags, crc32c, pre_unpack, out, stream, nullptr, false);
+  // Columns of up to 256 MB come from the context's pool (a cudaMalloc and cudaFree per array cost 1.4 ms a
+  // column of 2M values); larger ones keep giving their memory back to the device when freed.
+  cudaMemPool_t pool = ctx && size <= (256ull << 20) && !pre_unpack ? ctx->pool : nullptr;
+  const glc_status st = glc::deserialize_column(ctx, dtype, blob, size, flags, crc32c, pre_unpack, out, stream, pool, false);
+  if (st == GLC_OK && pool) (*out)->sync_free = true;  // freed as cudaFree frees
+  return st;
 }
 
 }  // extern "C"
@@ -761,10 +778,36 @@ glc_status glc::deserialize_column(glc_ctx* ctx, glc_dtype dtype, const void* bl
   auto copy_in = [&](void* d, const void* src, size_t len) {
     return host ? host_upload(ctx, d, src, len, s) : cudaMemcpyAsync(d, src, len, k, s);
   };
-  for (int j = 0; j < 7; j++)
-    if (lens[j] && (e = copy_in(dst[j], b + offs[j], lens[j])) != cudaSuccess)
-      return bail(cuda_fail(ctx, e, "deserialize: arrays"));
-  if ((e = cudaMemsetAsync(c->d_words, 0, 4 * c->nwords_alloc, s)) != cudaSuccess ||
+  // a host blob's metadata goes up as one copy where it lies in one piece (as serialize writes it: a
+  // copy from pageable memory takes 4 us however small), and a kernel deals it out to the arrays
+  uint64_t lo = offs[0], hi = 0, sum = 0;
+  bool words4 = true;
+  for (int j = 0; j < 7; j++) {
+    lo = std::min(lo, offs[j]);
+    hi = std::max(hi, offs[j] + lens[j]);
+    sum += lens[j];
+    words4 = words4 && (offs[j] & 3) == 0;
+  }
+  uint8_t* image = nullptr;
+  if (host && words4 && hi - lo <= sum + 64) {
+    ScatterArgs sa;
+    if ((e = pool_alloc(ctx, &image, hi - lo, s)) == cudaSuccess) e = host_upload(ctx, image, b + lo, hi - lo, s);
+    for (int j = 0; j < 7; j++) {
+      sa.src[j] = (const uint32_t*)(image + (offs[j] - lo));
+      sa.dst[j] = (uint32_t*)dst[j];
+      sa.words[j] = lens[j] / 4;
+    }
+    if (e == cudaSuccess) e = launch_scatter(sa, ctx->num_sms, s);
+    if (image) cudaFreeAsync(image, s);
+    if (e != cudaSuccess) return bail(cuda_fail(ctx, e, "deserialize: arrays"));
+  } else {
+    for (int j = 0; j < 7; j++)
+      if (lens[j] && (e = copy_in(dst[j], b + offs[j], lens[j])) != cudaSuccess)
+        return bail(cuda_fail(ctx, e, "deserialize: arrays"));
+  }
+  // zeros after the bitstream (all of it where the caller uploads it later)
+  const uint64_t given = defer_words ? 0 : (uint64_t)h.delta_size;
+  if ((e = cudaMemsetAsync((uint8_t*)c->d_words + given, 0, 4 * c->nwords_alloc - given, s)) != cudaSuccess ||
       (h.delta_size && !defer_words && (e = copy_in(c->d_words, b + h.delta_off, h.delta_size)) != cudaSuccess))
     return bail(cuda_fail(ctx, e, "deserialize: bitstream"));
   // structure check, fixed-length detection and max width

@@ -36,6 +36,8 @@ struct glc_batch {
   // decode work list for the last set of outputs
   std::vector<void*> outs;
   BatchWork* d_work = nullptr;
+  BatchWork* d_pieces = nullptr;              // what the work list is expanded from: a piece per column
+  int64_t* d_tile_base = nullptr;
   int64_t nwork = 0;
   unsigned long long* d_counter = nullptr;
   int64_t group_begin[5] = {0, 0, 0, 0, 0};  // work items grouped by element type
@@ -301,9 +303,6 @@ void free_batch(glc_batch* b) {
     for (glc_column* c : b->cols) delete c;
   for (void* q : b->storage) cudaFreeAsync(q, b->ctx->own_stream);
   if (!b->storage.empty()) cudaStreamSynchronize(b->ctx->own_stream);
-  if (b->d_cols) cudaFree(b->d_cols);
-  if (b->d_work) cudaFree(b->d_work);
-  if (b->d_counter) cudaFree(b->d_counter);
   delete b;
 }
 
@@ -315,10 +314,10 @@ glc_status finish_batch(glc_ctx* ctx, glc_batch* b, cudaStream_t s) {
     h[i] = BatchColumn{c->d_desc, c->d_start, c->d_tiles, c->d_words, c->n, (int32_t)c->dtype, c->max_bits};
     b->max_bits = std::max(b->max_bits, c->max_bits);
   }
-  BCK(cudaMalloc(&b->d_cols, sizeof(BatchColumn) * std::max<size_t>(1, h.size())), "batch: column table");
+  BCK(dalloc(b, &b->d_cols, std::max<size_t>(1, h.size())), "batch: column table");
   BCK(cudaMemcpyAsync(b->d_cols, h.data(), sizeof(BatchColumn) * h.size(), cudaMemcpyHostToDevice, s), "batch: column table");
-  void* q = nullptr;
-  BCK(cudaMalloc(&q, 64), "batch: counters");
+  uint8_t* q = nullptr;
+  BCK(dalloc(b, &q, 64), "batch: counters");
   BCK(cudaMemsetAsync(q, 0, 64, s), "batch: counters");
   b->d_counter = (unsigned long long*)q;  // 4 counters, one per element type
   b->d_err = (int*)((char*)q + 32);
@@ -331,31 +330,54 @@ glc_status build_work(glc_ctx* ctx, glc_batch* b, void* const* outs, cudaStream_
   bool same = b->d_work && b->outs.size() == nc;
   for (size_t i = 0; same && i < nc; i++) same = b->outs[i] == outs[i];
   if (same) return GLC_OK;
-  std::vector<BatchWork> w;
+  // one piece per column, grouped by element type, which the device expands to one item per tile (a
+  // host list of 42,000 items took 0.6 ms to build and 1.3 MB to upload)
+  std::vector<BatchWork> pieces;
+  std::vector<int64_t> tile_base(1, 0);
+  pieces.reserve(nc);
+  tile_base.reserve(nc + 1);
   for (size_t i = 0; i < nc; i++) {
     const glc_column* c = b->cols[i];
     if (c->n == 0) continue;
     if (!outs[i]) return bfail(ctx, GLC_ERR_INVALID_ARG, "null output for a column of the batch");
     if (((uintptr_t)outs[i] & 15) != 0) return bfail(ctx, GLC_ERR_INVALID_ARG, "batch outputs must be 16-byte aligned");
     if (!c->d_words) return bfail(ctx, GLC_ERR_UNSUPPORTED, "a column of the batch has no packed bitstream");
-    for (int64_t t = 0; t < c->ntiles; t++) w.push_back(BatchWork{(int32_t)i, (int32_t)t, 0, c->n, outs[i]});
   }
-  std::vector<int32_t> col_dtype(nc);
-  for (size_t i = 0; i < nc; i++) col_dtype[i] = (int32_t)b->cols[i]->dtype;
-  group_work_by_type(w, col_dtype, b->group_begin);
+  for (int d = 0; d < 4; d++) {
+    b->group_begin[d] = tile_base.back();
+    for (size_t i = 0; i < nc; i++) {
+      const glc_column* c = b->cols[i];
+      if (c->n == 0 || (int)c->dtype != d) continue;
+      pieces.push_back(BatchWork{(int32_t)i, 0, 0, c->n, outs[i]});
+      tile_base.push_back(tile_base.back() + c->ntiles);
+    }
+  }
+  b->group_begin[4] = tile_base.back();
   if (b->graph) {
     cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
   }
-  if (b->d_work) {
-    cudaStreamSynchronize(s);
-    cudaFree(b->d_work);
-    b->d_work = nullptr;
-  }
-  b->nwork = (int64_t)w.size();
-  if (!w.empty()) {
-    BCK(cudaMalloc(&b->d_work, sizeof(BatchWork) * w.size()), "batch: work list");
-    BCK(cudaMemcpyAsync(b->d_work, w.data(), sizeof(BatchWork) * w.size(), cudaMemcpyHostToDevice, s), "batch: work list");
+  // the columns, and so the number of items, never change: the list is allocated once and rewritten
+  // when no decode on any stream can be reading it
+  if (b->d_work) cudaDeviceSynchronize();
+  b->outs.clear();  // (the list is valid again at the end)
+  b->nwork = tile_base.back();
+  if (b->nwork > 0) {
+    if (!b->d_work) {  // from the pool, in this call's order; the call ends synchronised
+      const size_t wb = sizeof(BatchWork) * (size_t)b->nwork, pcb = sizeof(BatchWork) * pieces.size();
+      uint8_t* q = nullptr;
+      BCK(cudaMallocFromPoolAsync((void**)&q, wb + pcb + sizeof(int64_t) * tile_base.size(), ctx->pool, s), "batch: work list");
+      b->storage.push_back(q);
+      b->d_work = (BatchWork*)q;
+      b->d_pieces = (BatchWork*)(q + wb);
+      b->d_tile_base = (int64_t*)(q + wb + pcb);
+    }
+    BCK(cudaMemcpyAsync(b->d_pieces, pieces.data(), sizeof(BatchWork) * pieces.size(), cudaMemcpyHostToDevice, s),
+        "batch: work list");
+    BCK(cudaMemcpyAsync(b->d_tile_base, tile_base.data(), sizeof(int64_t) * tile_base.size(), cudaMemcpyHostToDevice, s),
+        "batch: work list");
+    BCK(launch_expand_pieces(b->d_pieces, b->d_tile_base, (int)pieces.size(), b->nwork, b->d_work, ctx->num_sms, s),
+        "batch: work list");
     BCK(cudaStreamSynchronize(s), "batch: work list");
   }
   b->outs.assign(outs, outs + nc);
@@ -698,6 +720,7 @@ glc_status glc_batch_create(glc_ctx* ctx, glc_column* const* cols, int32_t ncols
     if (!cols[i]) { delete b; return bfail(ctx, GLC_ERR_INVALID_ARG, "null column in batch"); }
     b->cols.push_back(cols[i]);
   }
+  b->alloc_stream = ctx->own_stream;
   glc::DeviceScope device_scope(ctx->device);
   glc_status st = finish_batch(ctx, b, ctx->own_stream);
   if (st != GLC_OK) { free_batch(b); return st; }

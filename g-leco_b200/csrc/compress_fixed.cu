@@ -19,6 +19,7 @@
 // The partition-length choice of a batch (choose_lengths_kernel) measures three lengths at once in
 // persistent CTAs of producer, solver and compute warps and packs the usual choice, 4096, on the way.
 #include <type_traits>
+#include "glc_group.cuh"
 #include "glc_internal.h"
 #include "glc_scan.cuh"
 #include "glc_tma.cuh"
@@ -99,25 +100,8 @@ __device__ __forceinline__ void cf_produce(const FixedCompressArgs& a, uint8_t* 
 
 // ---- pieces of the compute warps -----------------------------------------------------------
 
-constexpr double kMagic = 6755399441055744.0;        // K = 1.5 * 2^52: the bits of K + v are 0x4338... + v, |v| <= 2^51
-constexpr double kHalfBias = 0x1.fffffffffffffp-2;    // 0.5 - 2^-54
 constexpr int kFtStride = 129;                        // transposed fields: field f of 32-value group G at f * 129 + G
 constexpr int kFtWords = 32 * kFtStride;
-
-// How a partition's residuals are computed (uniform per partition, so per thread):
-//   CF_DIRECT   direct copy (a uint64 value above 2^53): the field is the value;
-//   CF_NONNEG   |y| < 2^51 and predictions in [-0.25, 2^51] (4-byte types: inside the type): in
-//               FP64 with K: K + y from the bits, K + pred = (x + (0.5 - 2^-54)) + K rounded toward
-//               zero, their difference is y - pred exactly;
-//   CF_NONPOS   the mirror for signed types, predictions in [-2^51, 0.25]: K - pred =
-//               ((0.5 - 2^-54) - x) + K rounded toward zero;
-//   CF_OFFSET   8-byte types with predictions in [2^50, 2^62] within 2^50 of c = trunc(theta0):
-//               x - c and x - c + 0.5 are exact, pred = c + floor(x - c + 0.5), y - c by integer
-//               arithmetic (a thread whose |y - c| reaches 2^51 recomputes its values in general);
-//   CF_GENERAL  predict_from / calc_delta / abs_ref per value.
-// Each gives calc_delta<T>(y, predict_from<T>(fma(theta1, i, theta0))) exactly; the field is its
-// low 32 bits (the low bits of (y - pred) + K), which is all the packing of a width <= 31 reads.
-enum : int { CF_DIRECT = 0, CF_NONNEG = 1, CF_NONPOS = 2, CF_GENERAL = 3, CF_OFFSET = 4 };
 
 // Exact sum over a reduction segment of W lanes (32, or 16 at L = 256) of values |v| < 2^48: for a
 // whole warp two redux sums of the 24-bit limbs (each limb's sum stays below 2^29).
@@ -450,62 +434,6 @@ template <typename T> __host__ __device__ constexpr int cf_fix_smem_bytes(int st
 // which the other CTAs of the SM cover in part; memory is at 39 %.  200M uint64 values at L = 4096:
 // 903 -> 498 us (3.9 TB/s), against persistent CTAs of 256 compute threads, three per SM,
 // that passed every field through shared memory and packed with half of their threads.
-constexpr int kCgThreads = 128;
-template <typename T> __host__ __device__ constexpr int cg_row_bytes() { return 32 * (int)sizeof(T) + 16; }
-template <typename T> __host__ __device__ constexpr int cg_stage_bytes() { return kCgThreads * cg_row_bytes<T>(); }
-static_assert(cg_row_bytes<int32_t>() >= 4 * 32, "the staged words of a segment fit its rows");
-
-// Byte offset in the stage of value j of the tile.
-template <typename T> __device__ __forceinline__ int cg_at(int j) { return j * (int)sizeof(T) + (j >> 5) * 16; }
-
-template <int BYTES> __device__ __forceinline__ void cp_async(uint32_t dst, const void* src, int valid) {
-  // copies `valid` bytes and zeroes the rest of the BYTES
-  if (BYTES == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(BYTES), "r"(valid) : "memory");
-}
-
-// The tile's values (cnt of them at src, the rest zero) into the rows of the stage.
-template <typename T> __device__ __forceinline__ void cg_load(uint8_t* stage, const T* src, int cnt, int tid) {
-  const uint32_t base = (uint32_t)__cvta_generic_to_shared(stage);
-  constexpr int kPer = 16 / (int)sizeof(T);  // values per 16-byte copy
-  constexpr int kIters = kDecodeTile / kPer / kCgThreads;
-  const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-  if (vec && cnt == kDecodeTile) {  // copies a whole number of rows apart: one address each side, constant steps
-    constexpr int kStep = kCgThreads * kPer;
-    static_assert(kStep % 32 == 0, "a step is a whole number of rows");
-    const T* p = src + tid * kPer;
-    const uint32_t d = base + cg_at<T>(tid * kPer);
-#pragma unroll
-    for (int i = 0; i < kIters; i++) cp_async<16>(d + i * (kStep / 32) * cg_row_bytes<T>(), p + i * kStep, 16);
-  } else if (vec) {
-#pragma unroll 4
-    for (int i = 0; i < kIters; i++) {
-      const int j = (i * kCgThreads + tid) * kPer;
-      const int left = (cnt - j) * (int)sizeof(T);
-      cp_async<16>(base + cg_at<T>(j), left > 0 ? src + j : src, left >= 16 ? 16 : (left > 0 ? left : 0));
-    }
-  } else {  // values aligned to their own size only
-#pragma unroll 8
-    for (int i = 0; i < kDecodeTile / kCgThreads; i++) {
-      const int j = i * kCgThreads + tid;
-      cp_async<(int)sizeof(T)>(base + cg_at<T>(j), j < cnt ? src + j : src, j < cnt ? (int)sizeof(T) : 0);
-    }
-  }
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-}
-
-// The values of 16 bytes of a row.
-template <typename T> struct CgVec {
-  static constexpr int N = 16 / (int)sizeof(T);
-  T v[N];
-  __device__ __forceinline__ explicit CgVec(const uint8_t* p) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
-    memcpy(v, &u, 16);
-  }
-};
-
 // Exact sums of a group (values past the column's end are zero): s = sum y_f, x = sum (i0 + f) y_f, by
 // halves.  Every partial is below 32 * 2^12 * 2^32 = 2^49 in magnitude.
 template <typename T>
@@ -586,84 +514,6 @@ __device__ __forceinline__ bool cg_resid(const uint8_t* __restrict__ row, int i0
   return wide == 0u;
 }
 
-// One value's residual, or the value itself for direct copy, in 64 bits (the slow path).  The fast
-// modes' formulas are those of cg_resid, exact modulo 2^64 as calc_delta is for signed types; a
-// uint64 partition outside direct copy holds values up to 2^53, where calc_delta does not saturate.
-template <typename T>
-__device__ __forceinline__ long long cg_field(T y, double xi, int mode, double t0, double t1, double c, long long ci) {
-  constexpr long long kBits = 0x4338000000000000ll;
-  const uint64_t v = TypeTraits<T>::is_signed ? (uint64_t)(long long)y : (uint64_t)y;
-  const double x = __fma_rn(t1, xi, t0);
-  if (mode == CF_NONNEG) return (long long)(v - (uint64_t)(__double_as_longlong(__dadd_rz(__dadd_rn(x, kHalfBias), kMagic)) - kBits));
-  if (sizeof(T) == 8 && mode == CF_OFFSET)
-    return (long long)(v - (uint64_t)ci -
-                       (uint64_t)(__double_as_longlong(__dadd_rz(__dadd_rn(__dsub_rn(x, c), 0.5), kMagic)) - kBits));
-  if (TypeTraits<T>::is_signed && mode == CF_NONPOS)
-    return (long long)(v + (uint64_t)(__double_as_longlong(__dadd_rz(__dsub_rn(kHalfBias, x), kMagic)) - kBits));
-  if (mode == CF_DIRECT) return (long long)v;  // the field is the value itself
-  return calc_delta<T>(y, predict_from<T>(x));
-}
-
-// The slow path's packing: the group's values become its words (width b, 1 to 64) in place.  After
-// value f, at most (f + 1) b / 32 words are complete, which end no later than value f does (4-byte
-// types, fields of up to 33 bits: the 33rd word lies in the row's padding).
-template <typename T>
-__device__ __forceinline__ void cg_pack_slow(uint8_t* row, int glen, int i0, int b, int mode, double t0, double t1,
-                                             double c, long long ci) {
-  uint32_t* words = reinterpret_cast<uint32_t*>(row);
-  const uint64_t mask = b >= 64 ? ~0ull : ((1ull << b) - 1ull);
-  uint32_t acc = 0u;  // bits not yet stored: `have` (0 to 31) of them
-  int have = 0, k = 0;
-  double xi = (double)i0;
-#pragma unroll 1
-  for (int f = 0; f < glen; f++) {
-    const T y = *reinterpret_cast<const T*>(row + f * (int)sizeof(T));
-    const uint64_t v = (uint64_t)cg_field<T>(y, xi, mode, t0, t1, c, ci) & mask;
-    xi = __dadd_rn(xi, 1.0);
-    const uint64_t lo = (v << have) | acc;
-    const uint32_t over = have ? (uint32_t)(v >> 32 >> (32 - have)) : 0u;  // the bits past 64
-    int n = have + b;  // 1 to 95 bits in (over, lo)
-    uint32_t w0 = (uint32_t)lo, w1 = (uint32_t)(lo >> 32), w2 = over;
-    if (n >= 32) { words[k++] = w0; w0 = w1; w1 = w2; n -= 32; }
-    if (n >= 32) { words[k++] = w0; w0 = w1; n -= 32; }
-    acc = w0;
-    have = n;
-  }
-  if (have) words[k] = acc;
-}
-
-// Packs a group's 32 fields (width B) into its B words at stg.  acc holds the bits so far at its top
-// and older bits below them: one funnel shift appends a field (whatever lies above its B bits is
-// shifted out), and a word is complete when 32 bits have come in.
-template <int B>
-__device__ __forceinline__ void cg_pack(const uint32_t (&fl)[32], uint32_t* __restrict__ stg) {
-  uint32_t acc = 0u;
-#pragma unroll
-  for (int f = 0; f < 32; f++) {
-    const int sh = (f * B) & 31;  // bits of the open word
-    if (sh + B < 32) {
-      acc = __funnelshift_r(acc, fl[f], B);
-    } else {
-      stg[(f * B) >> 5] = __funnelshift_r(acc, fl[f], 32 - sh);
-      acc = fl[f] << (32 - B);
-    }
-  }
-}
-
-__device__ __forceinline__ void cg_pack_dispatch(int b, const uint32_t (&fl)[32], uint32_t* __restrict__ stg) {
-  switch (b) {
-#define GLC_CG_PACK(B) \
-  case B: cg_pack<B>(fl, stg); break;
-    GLC_CG_PACK(1) GLC_CG_PACK(2) GLC_CG_PACK(3) GLC_CG_PACK(4) GLC_CG_PACK(5) GLC_CG_PACK(6) GLC_CG_PACK(7)
-    GLC_CG_PACK(8) GLC_CG_PACK(9) GLC_CG_PACK(10) GLC_CG_PACK(11) GLC_CG_PACK(12) GLC_CG_PACK(13) GLC_CG_PACK(14)
-    GLC_CG_PACK(15) GLC_CG_PACK(16) GLC_CG_PACK(17) GLC_CG_PACK(18) GLC_CG_PACK(19) GLC_CG_PACK(20)
-    GLC_CG_PACK(21) GLC_CG_PACK(22) GLC_CG_PACK(23) GLC_CG_PACK(24) GLC_CG_PACK(25) GLC_CG_PACK(26)
-    GLC_CG_PACK(27) GLC_CG_PACK(28) GLC_CG_PACK(29) GLC_CG_PACK(30) GLC_CG_PACK(31)
-#undef GLC_CG_PACK
-    default: break;  // width 0: no words
-  }
-}
-
 template <typename T> __global__ void __launch_bounds__(kCgThreads, 6)
 fixed_compress_kernel(const __grid_constant__ FixedCompressArgs a) {
   extern __shared__ __align__(128) uint8_t stage[];
@@ -689,6 +539,7 @@ fixed_compress_kernel(const __grid_constant__ FixedCompressArgs a) {
   uint8_t* row = stage + tid * cg_row_bytes<T>();
 
   cg_load<T>(stage, reinterpret_cast<const T*>(col.values) + e0, cnt, tid);
+  cg_load_wait();
   __syncthreads();
 
   {  // ---- A: exact sums and range flags per segment ----
@@ -826,8 +677,7 @@ const double c = s_c[p];
   const int bp = __shfl_sync(FULL_MASK, b, p & 31), blp = __shfl_sync(FULL_MASK, bl, p & 31);
   if (!slow) {
     // ---- C: the group's words, staged over its warp's rows (read by no other warp), then to the
-    // slot, a reduction segment at a time: its groups are consecutive words of one partition.  Groups
-    // lie b words apart, or b + 1 for an even b, so that the lanes' stores fall on different banks ----
+    // slot, a reduction segment at a time: its groups are consecutive words of one partition ----
     uint32_t* stg = reinterpret_cast<uint32_t*>(stage + (tid & ~31) * cg_row_bytes<T>());
     __syncwarp();
     if (glen > 0) cg_pack_dispatch(bp, fl, stg + (lane & ~(W - 1)) * 32 + (lane & (W - 1)) * (bp | 1));
@@ -836,18 +686,8 @@ const double c = s_c[p];
     for (int l = 0; l < 32; l += W) {
       const int bs = __shfl_sync(FULL_MASK, bp, l), os = __shfl_sync(FULL_MASK, o0, l);
       const int groups = __popc(__ballot_sync(FULL_MASK, glen > 0) >> l & (uint32_t)((1ull << W) - 1ull));
-      const int nw = groups * bs, pad = (bs & 1) ^ 1;
-      const uint32_t mb = bs > 1 ? 0xffffffffu / (uint32_t)bs + 1u : 0u;  // w / b by a multiply-high (w < 2^10)
-      const uint32_t* q = stg + l * 32;
-      uint32_t* ow = out + os;  // 16-byte aligned: a segment holds at least 8 groups
-      for (int w = 4 * lane; w + 3 < nw; w += 128) {
-        uint32_t v[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) v[u] = q[w + u + (pad ? (int)__umulhi((uint32_t)(w + u), mb) : 0)];
-        *reinterpret_cast<uint4*>(ow + w) = make_uint4(v[0], v[1], v[2], v[3]);
-      }
-      const int w = (nw & ~3) + lane;
-      if (w < nw) ow[w] = q[w + (pad ? (int)__umulhi((uint32_t)w, mb) : 0)];
+      // (16-byte aligned: a segment holds at least 8 groups)
+      cg_copy_words<true>(stg + l * 32, out + os, groups * bs, bs, lane);
     }
     return;
   }

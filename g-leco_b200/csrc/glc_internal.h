@@ -97,6 +97,7 @@ struct glc_column {
   int32_t fixed_len = 0;
   int64_t reported_size = 0;
   // reference SoA (CompressedData<T>)
+  void* meta = nullptr;      // one allocation that holds d_start .. d_err, d_desc and d_tiles (null: views)
   int32_t* d_start = nullptr;
   int32_t* d_end = nullptr;
   int32_t* d_types = nullptr;
@@ -248,6 +249,13 @@ struct SerializeArgs {
   uint64_t off[kSerPieces], bytes[kSerPieces];
   uint32_t header[kSerHeaderWords];
 };
+// The metadata of an uploaded blob into a column's arrays (4-byte aligned words).
+struct ScatterArgs {
+  const uint32_t* src[kSerPieces - 1];
+  uint32_t* dst[kSerPieces - 1];
+  uint64_t words[kSerPieces - 1];
+};
+cudaError_t launch_scatter(const ScatterArgs& a, int num_sms, cudaStream_t s);
 cudaError_t launch_serialize(const SerializeArgs& a, int num_sms, cudaStream_t s);
 cudaError_t launch_validate(const glc_column* c, int* d_bad, cudaStream_t s);
 cudaError_t launch_max_bits(const glc_column* c, int64_t* d_out, cudaStream_t s);
@@ -277,9 +285,10 @@ cudaError_t launch_batch_pack_tiles(glc_dtype dt, const PackTileCol* cols, const
 cudaError_t launch_pack_item_owner(const int64_t* item_base, int ncols, int32_t* owner, cudaStream_t s);
 // pack.cu: packs c's values; the column's descriptor and tile tables must be built.
 // parts_per_tile bounds the partitions a 4096-value tile spans (the fit's stats[3]); a device
-// wait that gives up is reported in *status (the context's error word, read by glc_sync).
-cudaError_t launch_pack(glc_dtype dt, const void* values, glc_column* c, int64_t parts_per_tile, int* status,
-                        cudaStream_t s);
+// wait that gives up is reported in *status (the context's error word, read by glc_sync).  starts32:
+// every partition starts at a multiple of 32 values.
+cudaError_t launch_pack(glc_dtype dt, const void* values, glc_column* c, int64_t parts_per_tile, bool starts32,
+                        int* status, cudaStream_t s);
 // decode.cu: values (or residuals when residual_out) of positions [lo, hi) to out_base[lo..hi)
 cudaError_t launch_decode(glc_ctx* ctx, const glc_column* c, int plain_src, int residual_out, int64_t lo,
                           int64_t hi, void* out_base, cudaStream_t s);

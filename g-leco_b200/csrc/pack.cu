@@ -20,6 +20,7 @@
 //   * the finished tile is written with coalesced 128-bit stores, padding words included, so
 //     every word of the array is written exactly once and no memset pass is needed.
 // Values whose fields straddle two tiles are computed by both CTAs; each keeps its own bits.
+#include "glc_group.cuh"
 #include "glc_internal.h"
 #include "glc_tma.cuh"
 
@@ -477,9 +478,184 @@ cudaError_t launch_pack_item_owner(const int64_t* item_base, int ncols, int32_t*
   return cudaGetLastError();
 }
 
-cudaError_t launch_pack(glc_dtype dt, const void* values, glc_column* c, int64_t parts_per_tile, int* status,
-                        cudaStream_t s) {
+// ---------------------------------------------------------------------------------------
+// Pack of a column whose partitions all start at multiples of 32 values (the partitioners' always do,
+// fixed ones where 32 divides the length): a thread per 32-value group (glc_group.cuh), a CTA of 128
+// threads per 4096-value tile.  Every partition's bits, and so every group's, start at a whole word:
+// no word is shared, and none needs clearing first.
+//   load      the tile's values by asynchronous copies, its descriptors beside them;
+//   fields    the group's partition by a search of the staged descriptors, then the low 32 bits of
+//             value - prediction (the prediction rounded in FP64 without conversion instructions
+//             where the group's two ends allow it): a field of at most 31 bits is all in them;
+//   words     appended in registers, staged over the warp's values, and copied to the column; a warp
+//             whose groups have different widths copies group by group.
+// Wider fields, direct copies and the column's incomplete last group are packed value by value in
+// their row.  Bound by memory: one barrier per tile, about 10 instructions per value and lane.  200M
+// uint64 in variable partitions: PACKFIG.
+// ---------------------------------------------------------------------------------------
+struct PackGroupArgs {
+  PackTileCol col;
+  int64_t nwords, nwords_alloc;  // the last tile's CTA zeroes the words after the bitstream
+  int* status;                   // DEVERR_* (the context's device error word)
+};
+
+// The residual mode of a group from its line's predictions at its two ends (fma is monotone in the
+// index).  Only low bits are taken, so the values' own range does not matter here.
+// c: the whole number near which the group's predictions lie (CF_OFFSET).
+template <typename T> __device__ __forceinline__ int pg_mode(double xa, double xb, double& c) {
+  const double lo = fmin(xa, xb), hi = fmax(xa, xb);
+  constexpr double kS = 2251799813685248.0;  // 2^51
+  const double hi_ok = sizeof(T) == 4 ? (TypeTraits<T>::is_signed ? 2147483646.0 : 4294967294.0) : kS;
+  const double lo_ok = sizeof(T) == 4 ? -2147483647.0 : -kS;
+  if (lo >= -0.25 && hi <= hi_ok) return CF_NONNEG;
+  if (TypeTraits<T>::is_signed && hi <= 0.25 && lo >= lo_ok) return CF_NONPOS;
+  if (sizeof(T) == 8 && lo >= 1125899906842624.0 && hi <= 4611686018427387904.0) {  // [2^50, 2^62]
+    c = trunc(xa);
+    if (fabs(__dsub_rn(xb, c)) < 562949953421312.0) return CF_OFFSET;  // 2^49
+  }
+  return CF_GENERAL;
+}
+
+// The low 32 bits of a full group's residuals, by the fast modes.
+template <typename T, int MODE>
+__device__ __forceinline__ void pg_fields(const uint8_t* __restrict__ row, double xd, double t0, double t1, double c,
+                                          uint32_t (&fl)[32]) {
+  const uint32_t ci = MODE == CF_OFFSET ? (uint32_t)__double2ll_rz(c) : 0u;
+#pragma unroll
+  for (int k = 0; k < 32 / CgVec<T>::N; k++) {
+    const CgVec<T> vec(row + 16 * k);
+#pragma unroll
+    for (int u = 0; u < CgVec<T>::N; u++) {
+      const double x = __fma_rn(t1, xd, t0);
+      xd = __dadd_rn(xd, 1.0);
+      const uint32_t y = (uint32_t)vec.v[u];  // (the low 32 bits of K are zero)
+      if (MODE == CF_NONNEG) fl[k * CgVec<T>::N + u] = y - (uint32_t)__double2loint(__dadd_rz(__dadd_rn(x, kHalfBias), kMagic));
+      else if (MODE == CF_NONPOS) fl[k * CgVec<T>::N + u] = y + (uint32_t)__double2loint(__dadd_rz(__dsub_rn(kHalfBias, x), kMagic));
+      else fl[k * CgVec<T>::N + u] = y - ci - (uint32_t)__double2loint(__dadd_rz(__dadd_rn(__dsub_rn(x, c), 0.5), kMagic));
+    }
+  }
+}
+
+template <typename T> __global__ void __launch_bounds__(kCgThreads, 6) pack_group_kernel(const __grid_constant__ PackGroupArgs a) {
+  extern __shared__ __align__(128) uint8_t stage[];
+  __shared__ PartDesc s_desc[kPackTileParts];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int64_t t = blockIdx.x, e0 = t * kDecodeTile, left = a.col.n - e0;
+  const int cnt = (int)(left < kDecodeTile ? left : kDecodeTile);
+  cg_load<T>(stage, reinterpret_cast<const T*>(a.col.v) + e0, cnt, tid);
+  const TileInfo ti = a.col.tiles[t];
+  const int np = ti.p_last - ti.p_first + 1;
+  if (np > kPackTileParts) {  // excluded by the host (partitions of >= 108 values); never packed wrong
+    if (tid == 0) atomicExch(a.status, DEVERR_BOUNDS);
+    cg_load_wait();
+    return;
+  }
+  if (tid < np) s_desc[tid] = a.col.desc[ti.p_first + tid];
+  if (t == a.col.ntiles - 1)
+    for (int64_t w = a.nwords + tid; w < a.nwords_alloc; w += kCgThreads) a.col.words[w] = 0u;
+  cg_load_wait();
+  __syncthreads();
+
+  const int glen = cnt - 32 * tid < 32 ? cnt - 32 * tid : 32;  // values of the group (<= 0: none)
+  const int eg = (int)e0 + 32 * tid;                           // its first value
+  uint8_t* row = stage + tid * cg_row_bytes<T>();
+  int b = 0;
+  int64_t w0 = 0;  // the group's first word
+  PartDesc d{};
+  bool slow = false;
+  if (glen > 0) {
+    int q = 0;
+    for (int step = 32; step > 0; step >>= 1)  // the last partition that starts at or before the group
+      if (q + step < np && s_desc[q + step].start <= eg) q += step;
+    d = s_desc[q];
+    b = d.bits_type & 0xff;
+    const int64_t bit = d.bit_off + (int64_t)(eg - d.start) * b;
+    w0 = bit >> 5;
+    if ((bit & 31) != 0 || (q + 1 < np && s_desc[q + 1].start < eg + glen)) {  // not a column for this kernel
+      atomicExch(a.status, DEVERR_BOUNDS);
+      b = 0;
+    }
+    slow = b > 31 || glen < 32 || (d.bits_type >> 8) == MODEL_DIRECT_COPY;
+  }
+  const bool any_slow = __any_sync(FULL_MASK, slow && b > 0);
+  const bool uniform = !any_slow && __all_sync(FULL_MASK, b == __shfl_sync(FULL_MASK, b, 0));
+  if (b > 0) {
+    const double x0 = (double)(eg - d.start);
+    if (!slow) {
+      uint32_t fl[32];
+      double c = 0.0;
+      const int mode = pg_mode<T>(__fma_rn(d.theta1, x0, d.theta0), __fma_rn(d.theta1, __dadd_rn(x0, 31.0), d.theta0), c);
+      if (mode == CF_NONNEG) {
+        pg_fields<T, CF_NONNEG>(row, x0, d.theta0, d.theta1, 0.0, fl);
+      } else if (TypeTraits<T>::is_signed && mode == CF_NONPOS) {
+        pg_fields<T, CF_NONPOS>(row, x0, d.theta0, d.theta1, 0.0, fl);
+      } else if (sizeof(T) == 8 && mode == CF_OFFSET) {
+        pg_fields<T, CF_OFFSET>(row, x0, d.theta0, d.theta1, c, fl);
+      } else {
+        double xd = x0;
+#pragma unroll 2
+        for (int f = 0; f < 32; f++) {  // the residuals' low bits over the values, then to registers
+          T* v = reinterpret_cast<T*>(row) + f;
+          *v = (T)((uint64_t)*v - (uint64_t)predict_from<T>(__fma_rn(d.theta1, xd, d.theta0)));
+          xd = __dadd_rn(xd, 1.0);
+        }
+#pragma unroll
+        for (int f = 0; f < 32; f++) fl[f] = (uint32_t)reinterpret_cast<const T*>(row)[f];
+      }
+      // groups of one width: packed close, over the warp's rows (once all of them are read); else in
+      // the group's own row
+      if (uniform) __syncwarp();  // (every lane is here then)
+      cg_pack_dispatch(b, fl, uniform ? reinterpret_cast<uint32_t*>(stage + (tid & ~31) * cg_row_bytes<T>()) + lane * (b | 1)
+                                      : reinterpret_cast<uint32_t*>(row));
+    } else {
+      cg_pack_slow<T>(row, glen, eg - d.start, b, (d.bits_type >> 8) == MODEL_DIRECT_COPY ? CF_DIRECT : CF_GENERAL,
+                      d.theta0, d.theta1, 0.0, 0);
+    }
+  }
+  __syncwarp();
+  if (uniform) {
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(stage + (tid & ~31) * cg_row_bytes<T>());
+    const int nw = b * 32;
+    uint32_t* dst = a.col.words + __shfl_sync(FULL_MASK, w0, 0);
+    if (b > 0) {
+      if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) cg_copy_words<true>(q, dst, nw, b, lane);
+      else cg_copy_words<false>(q, dst, nw, b, lane);
+    }
+  } else {
+    for (int l = 0; l < 32; l++) {
+      const int bl = __shfl_sync(FULL_MASK, b, l), gl = __shfl_sync(FULL_MASK, glen, l);
+      const int64_t wl = __shfl_sync(FULL_MASK, w0, l);
+      if (gl <= 0) break;
+      const uint32_t* q = reinterpret_cast<const uint32_t*>(stage + ((tid & ~31) + l) * cg_row_bytes<T>());
+      const int nw = (gl * bl + 31) >> 5;
+      for (int w = lane; w < nw; w += 32) a.col.words[wl + w] = q[w];
+    }
+  }
+}
+
+template <typename T>
+static cudaError_t launch_pack_groups(const T* v, glc_column* c, int* status, cudaStream_t s) {
+  PackGroupArgs a{};
+  a.col = PackTileCol{v, c->d_desc, c->d_tiles, c->n, c->ntiles, c->d_words};
+  a.nwords = c->nwords;
+  a.nwords_alloc = c->nwords_alloc;
+  a.status = status;
+  pack_group_kernel<T><<<(unsigned)c->ntiles, kCgThreads, cg_stage_bytes<T>(), s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pack(glc_dtype dt, const void* values, glc_column* c, int64_t parts_per_tile, bool starts32,
+                        int* status, cudaStream_t s) {
   if (c->nwords_alloc <= 0) return cudaSuccess;
+  if (starts32 && parts_per_tile + 2 <= kPackTileParts && c->d_tiles && c->d_desc && c->ntiles > 0) {
+    switch (dt) {
+      case GLC_I32: return launch_pack_groups<int32_t>((const int32_t*)values, c, status, s);
+      case GLC_I64: return launch_pack_groups<int64_t>((const int64_t*)values, c, status, s);
+      case GLC_U64: return launch_pack_groups<uint64_t>((const uint64_t*)values, c, status, s);
+      case GLC_U32: return launch_pack_groups<uint32_t>((const uint32_t*)values, c, status, s);
+    }
+    return cudaErrorInvalidValue;
+  }
   if (parts_per_tile + 2 <= kPackTileParts && c->d_tiles && c->d_desc && c->ntiles > 0) {
     switch (dt) {
       case GLC_I32: return launch_pack_tiles<int32_t>((const int32_t*)values, c, status, s);

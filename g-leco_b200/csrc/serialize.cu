@@ -1,4 +1,5 @@
-// serialize.cu -- a column's version-5 blob written to device memory by one kernel.
+// serialize.cu -- a column's version-5 blob written to device memory by one kernel, and an uploaded
+// blob's metadata dealt out to a column's arrays.
 //
 // The blob is a 120-byte header, seven metadata arrays and the bitstream, each from an 8-byte
 // boundary with zeros between them (api/G-LeCo.cuh:1878-2047 copies them one by one).  As eight
@@ -86,6 +87,21 @@ __global__ void __launch_bounds__(kSerThreads) serialize_kernel(const __grid_con
     else if (w == nfull && (bytes & 3)) v = __ldg(src + w) & ((1u << (8 * (bytes & 3))) - 1u);
     dst[w] = v;
   }
+}
+
+__global__ void __launch_bounds__(kSerThreads) scatter_kernel(const __grid_constant__ ScatterArgs a) {
+  const int64_t tid = (int64_t)blockIdx.x * kSerThreads + threadIdx.x, nthreads = (int64_t)gridDim.x * kSerThreads;
+#pragma unroll
+  for (int j = 0; j < kSerPieces - 1; j++)
+    for (int64_t w = tid; w < (int64_t)a.words[j]; w += nthreads) a.dst[j][w] = __ldg(a.src[j] + w);
+}
+
+cudaError_t launch_scatter(const ScatterArgs& a, int num_sms, cudaStream_t s) {
+  uint64_t most = 0;
+  for (uint64_t w : a.words) most = std::max(most, w);
+  const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(((int64_t)most + kSerThreads - 1) / kSerThreads, (int64_t)num_sms * 8));
+  scatter_kernel<<<(unsigned)grid, kSerThreads, 0, s>>>(a);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_serialize(const SerializeArgs& a, int num_sms, cudaStream_t s) {
