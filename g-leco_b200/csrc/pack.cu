@@ -491,7 +491,8 @@ cudaError_t launch_pack_item_owner(const int64_t* item_base, int ncols, int32_t*
 //             whose groups have different widths copies group by group.
 // Wider fields, direct copies and the column's incomplete last group are packed value by value in
 // their row.  Bound by memory: one barrier per tile, about 10 instructions per value and lane.  200M
-// uint64 in variable partitions: PACKFIG.
+// uint64 in variable partitions: 494 -> 347 us (5.5 TB/s), 30M uint32: 87 -> 39 us, against 256
+// threads that passed every field through shared memory with three barriers per tile.
 // ---------------------------------------------------------------------------------------
 struct PackGroupArgs {
   PackTileCol col;

@@ -581,3 +581,30 @@ def test_decode_tiles_around_the_resident_ctas(glc_ctx, tiles):
         glc.decompress_into(glc_ctx, col, out.ctypes.data, glc.SRC_PACKED, host_out=True)
         assert np.array_equal(out, v)
         col.free()
+
+
+@pytest.mark.parametrize("n", [128, 4096, 4097, 4128, 131_072 + 31, 200_011])
+@pytest.mark.parametrize("mode", ["variable", "v6", "fixed 8192", "fixed 160", "fixed 4128", "fixed 1000"])
+def test_pack_by_groups(oracle, glc_ctx, n, mode):
+    """Partitions that start at multiples of 32 values, with warps of one width and of several, widths above
+    31, and an incomplete last group; and lengths that 32 does not divide."""
+    torch = pytest.importorskip("torch")
+    base = _jumps(n, seed=n)
+    for v in (base, -base, base.astype(np.uint64), (1 << 60) + base // 1024, (base & 0x7FFFFFFF).astype(np.int32),
+              (base & 0xFFFFFFFF).astype(np.uint32), _data("u64_big", n)):
+        code = {"int32": glc.I32, "int64": glc.I64, "uint64": glc.U64, "uint32": glc.U32}[v.dtype.name]
+        if mode.startswith("fixed"):
+            L = int(mode.split()[1])
+            want, how = oracle.serialize(oracle.compress(v, "fixed", L)), glc.FIXED
+        elif mode == "v6":
+            s, e = oracle.partition_v6(v, 2048)
+            want, L, how = oracle.serialize(oracle.compress(v, starts=s, ends=e)), 4096, glc.VARIABLE_V6
+        else:
+            want, L, how = oracle.serialize(oracle.compress(v, "variable")), 4096, glc.VARIABLE
+        for shift in (0, 1):
+            buf = torch.from_numpy(np.concatenate([np.zeros(shift, v.dtype), v]).view(np.int64 if v.itemsize == 8 else np.int32)).cuda()
+            torch.cuda.synchronize()
+            col = glc.compress_device(glc_ctx, code, buf.data_ptr() + shift * v.itemsize, n, how, fixed_len=L)
+            got = glc.serialize_host(glc_ctx, col)
+            col.free()
+            assert got == want
