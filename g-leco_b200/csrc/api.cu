@@ -143,17 +143,20 @@ void set_word_counts(glc_column* c) {
   c->nwords_alloc = ((c->nwords + 3) & ~3ll) + 8;  // decoders read up to 3 words past a field
 }
 
-// A private pool that keeps freed memory (release threshold = max), so per-call temporaries
-// (host-output staging, scratch) cost no fresh device allocation after the first call.
-cudaError_t create_pool(glc_ctx* ctx) {
+// Private pools that keep freed memory, so that columns and per-call temporaries (host-output
+// staging, scratch) cost no fresh device allocation after the first call: the columns' with release
+// threshold = max, the temporaries' up to 8 GB.
+cudaError_t create_pools(glc_ctx* ctx) {
   cudaMemPoolProps props = {};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
   props.location.id = ctx->device;
   cudaError_t e = cudaMemPoolCreate(&ctx->pool, &props);
   if (e != cudaSuccess) return e;
-  uint64_t keep = ~0ull;
-  return cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  uint64_t keep = ~0ull, keep_temp = 8ull << 30;
+  if ((e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) return e;
+  if ((e = cudaMemPoolCreate(&ctx->temp_pool, &props)) != cudaSuccess) return e;
+  return cudaMemPoolSetAttribute(ctx->temp_pool, cudaMemPoolAttrReleaseThreshold, &keep_temp);
 }
 
 int64_t reported_size(int64_t P, int64_t total_bits) {  // api/G-LeCo.cuh:589-603
@@ -194,7 +197,7 @@ glc_status glc_create(glc_ctx** out, int device) {
   ctx->device = device;
   if ((e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking)) != cudaSuccess ||
-      (e = create_pool(ctx)) != cudaSuccess ||
+      (e = create_pools(ctx)) != cudaSuccess ||
       (e = cudaMalloc(&ctx->d_flags, sizeof(int) * kFlagWords)) != cudaSuccess ||
       (e = cudaMemset(ctx->d_flags, 0, sizeof(int) * kFlagWords)) != cudaSuccess ||
       (e = cudaMalloc(&ctx->d_stats, sizeof(int64_t) * 16)) != cudaSuccess ||
@@ -222,10 +225,9 @@ glc_status glc_destroy(glc_ctx* ctx) {
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   for (cudaStream_t a : ctx->aux_stream)
     if (a) cudaStreamDestroy(a);
-  if (ctx->pool) {
-    cudaDeviceSynchronize();
-    cudaMemPoolDestroy(ctx->pool);
-  }
+  if (ctx->pool || ctx->temp_pool) cudaDeviceSynchronize();
+  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+  if (ctx->temp_pool) cudaMemPoolDestroy(ctx->temp_pool);
   delete ctx;
   return GLC_OK;
 }
@@ -328,7 +330,7 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
       c->total_bits = ctx->h_stats[0];
       c->max_bits = (int32_t)ctx->h_stats[1];
       set_word_counts(c);
-      e = col_alloc(c, &c->d_words, 4 * c->nwords_alloc, s);
+      e = col_alloc(c, &c->d_words, words_alloc_bytes(4 * c->nwords_alloc), s);
     }
     if (e == cudaSuccess) e = launch_fixed_place(dtype, c, fixed_len, scratch, st, s);
     cudaFreeAsync(scratch, s);
@@ -359,7 +361,7 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
   c->total_bits = ctx->h_stats[0];
   c->max_bits = (int32_t)ctx->h_stats[1];
   set_word_counts(c);
-  CK(col_alloc(c, &c->d_words, 4 * c->nwords_alloc, s), "compress: word allocation");
+  CK(col_alloc(c, &c->d_words, words_alloc_bytes(4 * c->nwords_alloc), s), "compress: word allocation");
   const int64_t parts_per_tile = ctx->h_stats[3];
   CK(launch_desc_and_tiles(c, s), "compress: tables");
   // the partitioners' starts are multiples of 128 and of kV6Base / 2

@@ -398,7 +398,7 @@ struct PrePacked {
   std::vector<int> cols;          // the batch's column index of each entry of the table
   std::vector<int64_t> item_base; // per entry
   int32_t* d_owner = nullptr;
-  void* scratch = nullptr;        // from the context's pool, returned after the place
+  void* scratch = nullptr;        // from pool_alloc, returned after the place
   PartDesc* tdesc = nullptr;
   long long* terr = nullptr;
 };
@@ -494,7 +494,8 @@ glc_status compress_one_pass(glc_ctx* ctx, glc_batch* b, const glc_dtype* dtypes
   }
   uint32_t* words;
   cudaError_t e;
-  if ((e = dalloc(b, &words, wb[nc])) != cudaSuccess) return bcuda(ctx, e, "batch compress: allocation");
+  if ((e = dalloc(b, &words, words_alloc_bytes(4 * (size_t)wb[nc]) / 4)) != cudaSuccess)
+    return bcuda(ctx, e, "batch compress: allocation");
   unsigned long long* stats = prep.stats;
   std::vector<CfColumn>& hc = prep.hc;
   std::vector<glc_column*> cols(b->cols.begin(), b->cols.end());
@@ -569,9 +570,8 @@ glc_status compress_one_pass(glc_ctx* ctx, glc_batch* b, const glc_dtype* dtypes
     uint8_t* scratch;
     if ((e = dalloc(b, &d_g, g.size())) || (e = dalloc(b, &d_ib, ib.size())) || (e = dalloc(b, &d_owner, nitems)))
       return bcuda(ctx, e, "batch compress: allocation");
-    // the tiles' slots are scratch: from the context's pool, returned after the launch
-    BCK(cudaMallocFromPoolAsync((void**)&scratch, fixed_compress_scratch_bytes(dt, nitems), ctx->pool, s),
-        "batch compress: scratch");
+    // the tiles' slots are scratch, returned after the launch
+    BCK(pool_alloc(ctx, &scratch, fixed_compress_scratch_bytes(dt, nitems), s), "batch compress: scratch");
     BCK(cudaMemcpyAsync(d_g, g.data(), sizeof(CfColumn) * g.size(), cudaMemcpyHostToDevice, s), "batch compress: columns");
     BCK(cudaMemcpyAsync(d_ib, ib.data(), sizeof(int64_t) * ib.size(), cudaMemcpyHostToDevice, s), "batch compress: columns");
     BCK(launch_pack_item_owner(d_ib, (int)g.size(), d_owner, s), "batch compress: work list");
@@ -828,7 +828,7 @@ glc_status glc_batch_compress(glc_ctx* ctx, const glc_dtype* dtypes, const void*
       pp.d_owner = d_owner;
       if (pack) {
         if ((e = dalloc(b, &pp.tdesc, pp.nitems)) || (e = dalloc(b, &pp.terr, pp.nitems)) ||
-            (e = cudaMallocFromPoolAsync(&pp.scratch, fixed_compress_scratch_bytes(dt, pp.nitems), ctx->pool, s)))
+            (e = pool_alloc(ctx, &pp.scratch, fixed_compress_scratch_bytes(dt, pp.nitems), s)))
           return release_pre(), bail(bcuda(ctx, e, "batch compress: allocation"));
       }
       void* scratch = pp.scratch;
