@@ -291,17 +291,16 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
   // the column synchronises the device first, so a free behaves as cudaFree does.
   c->pool = ctx->pool;
   c->sync_free = true;
-  int32_t* tmp_s = nullptr;
-  int32_t* tmp_e = nullptr;
   if (mode == GLC_PART_FIXED) {
     c->P = (n + fixed_len - 1) / fixed_len;
     c->fixed_len = fixed_len;
   } else if (mode == GLC_PART_VARIABLE_V6) {
-    int64_t P = 0;
-    cudaError_t e = launch_partition_v6(ctx, dtype, dev_values, n, kV6Base, &tmp_s, &tmp_e, &P, s);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "GPU partitioner (V6)");
-    c->P = P;
     c->fixed_len = 0;
+    PartOut po;
+    po.column = c;
+    po.alloc = alloc_meta;
+    cudaError_t e = launch_partition_v6(ctx, dtype, dev_values, n, kV6Base, po, s);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "GPU partitioner (V6)");
   } else {
     c->fixed_len = 0;
     std::string perr;
@@ -312,7 +311,7 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
     cudaError_t e = launch_partition_variable(ctx, dtype, dev_values, n, po, s, &perr);
     if (e != cudaSuccess) return perr.empty() ? cuda_fail(ctx, e, "variable partitioner") : fail(ctx, GLC_ERR_CUDA, perr);
   }
-  if (mode != GLC_PART_VARIABLE) CK(alloc_meta(c, s), "compress: metadata allocation");
+  if (mode == GLC_PART_FIXED) CK(alloc_meta(c, s), "compress: metadata allocation");
   if (mode == GLC_PART_FIXED && fixed_compress_supported(n, fixed_len)) {
     // one read of the values: fit, widths and words of every tile (into scratch slots), a scan of
     // the tiles' bits; then, with the total known, the words placed into an exact-size array
@@ -340,18 +339,17 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
   }
   if (mode == GLC_PART_FIXED) {
     CK(launch_fixed_partitions(c->d_start, c->d_end, n, fixed_len, c->P, s), "compress: fixed partitions");
-  } else if (mode == GLC_PART_VARIABLE_V6) {
-    CK(cudaMemcpyAsync(c->d_start, tmp_s, 4 * c->P, cudaMemcpyDeviceToDevice, s), "compress: partition copy");
-    CK(cudaMemcpyAsync(c->d_end, tmp_e, 4 * c->P, cudaMemcpyDeviceToDevice, s), "compress: partition copy");
-    cudaFreeAsync(tmp_s, s);
-    cudaFreeAsync(tmp_e, s);
   }
   cudaError_t e = cudaSuccess;
   if (mode != GLC_PART_VARIABLE) {
-    const size_t sb = fit_scratch_bytes(nullptr, n, c->P);
+    // V6 partitions hold at most 4 * kV6Base values: one CTA fits each
+    static_assert(4 * kV6Base <= kFitShort, "V6 partitions are short");
+    const bool brief = mode == GLC_PART_VARIABLE_V6;
+    const size_t sb = brief ? fit_short_scratch_bytes(c->P) : fit_scratch_bytes(nullptr, n, c->P);
     void* scratch = nullptr;
     CK(pool_alloc(ctx, &scratch, sb, s), "compress: scratch allocation");
-    e = launch_fit(dtype, dev_values, c, scratch, sb, ctx->d_stats, s);
+    e = brief ? launch_fit_short(dtype, dev_values, c, scratch, ctx->d_stats, s)
+              : launch_fit(dtype, dev_values, c, scratch, sb, ctx->d_stats, s);
     cudaFreeAsync(scratch, s);
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
@@ -459,7 +457,7 @@ static glc_status partition_only(glc_ctx* ctx, glc_dtype dtype, const void* valu
   po.starts = &ds;
   po.ends = &de;
   po.P = &P;
-  cudaError_t e = v6_base > 0 ? launch_partition_v6(ctx, dtype, dev_values, n, v6_base, &ds, &de, &P, s)
+  cudaError_t e = v6_base > 0 ? launch_partition_v6(ctx, dtype, dev_values, n, v6_base, po, s)
                               : launch_partition_variable(ctx, dtype, dev_values, n, po, s, &perr);
   if (staged) cudaFreeAsync(staged, s);
   if (e != cudaSuccess) return perr.empty() ? cuda_fail(ctx, e, "partition") : fail(ctx, GLC_ERR_CUDA, perr);

@@ -103,36 +103,6 @@ __device__ __forceinline__ void cf_produce(const FixedCompressArgs& a, uint8_t* 
 constexpr int kFtStride = 129;                        // transposed fields: field f of 32-value group G at f * 129 + G
 constexpr int kFtWords = 32 * kFtStride;
 
-// Exact sum over a reduction segment of W lanes (32, or 16 at L = 256) of values |v| < 2^48: for a
-// whole warp two redux sums of the 24-bit limbs (each limb's sum stays below 2^29).
-__device__ __forceinline__ long long seg_sum48(long long v, int W) {
-  if (W == 32) {
-    const unsigned lo = __reduce_add_sync(FULL_MASK, (unsigned)v & 0xFFFFFFu);
-    const int hi = __reduce_add_sync(FULL_MASK, (int)(v >> 24));
-    return (long long)hi * 16777216ll + (long long)lo;
-  }
-  for (int msk = W >> 1; msk > 0; msk >>= 1) v += __shfl_xor_sync(FULL_MASK, v, msk);
-  return v;
-}
-__device__ __forceinline__ unsigned seg_max_u32(unsigned v, int W) {
-  if (W == 32) return __reduce_max_sync(FULL_MASK, v);
-  for (int msk = W >> 1; msk > 0; msk >>= 1) {
-    const unsigned o = __shfl_xor_sync(FULL_MASK, v, msk);
-    v = o > v ? o : v;
-  }
-  return v;
-}
-__device__ __forceinline__ unsigned seg_or_u32(unsigned v, int W) {
-  if (W == 32) return __reduce_or_sync(FULL_MASK, v);
-  for (int msk = W >> 1; msk > 0; msk >>= 1) v |= __shfl_xor_sync(FULL_MASK, v, msk);
-  return v;
-}
-__device__ __forceinline__ unsigned long long seg_max_u64(unsigned long long v, int W) {
-  const unsigned hi = seg_max_u32((unsigned)(v >> 32), W);
-  const unsigned lo = seg_max_u32((unsigned)(v >> 32) == hi ? (unsigned)v : 0u, W);
-  return ((unsigned long long)hi << 32) | lo;
-}
-
 // Per value, for the range tests of the partition: uint64 keeps the max of the high words, above
 // 2^21 when some value exceeds 2^53 (direct copy; exactly 2^21 is decided by a rescan of the
 // partition, cf_any_above_2_53) and below 2^19 iff every value is below 2^51; int64 keeps the OR of
@@ -290,26 +260,6 @@ __device__ __forceinline__ unsigned long long cf_resid_general(const T* __restri
     }
   }
   return mx;
-}
-
-// The residual mode of a partition from its line and the range test of its values.
-template <typename T>
-__device__ __forceinline__ int cf_mode(double t0, double t1, int len, bool vsafe, double& c, long long& ci) {
-  const double xa = t0, xb = __fma_rn(t1, (double)(len - 1), t0);  // the ends (fma is monotone in i)
-  const double lo = fmin(xa, xb), hi = fmax(xa, xb);
-  constexpr double kS = 2251799813685248.0;  // 2^51
-  const double hi_ok = sizeof(T) == 4 ? (TypeTraits<T>::is_signed ? 2147483646.0 : 4294967294.0) : kS;
-  const double lo_ok = sizeof(T) == 4 ? -2147483647.0 : -kS;
-  if (vsafe && lo >= -0.25 && hi <= hi_ok) return CF_NONNEG;
-  if (TypeTraits<T>::is_signed && vsafe && hi <= 0.25 && lo >= lo_ok) return CF_NONPOS;
-  if (sizeof(T) == 8 && lo >= 1125899906842624.0 && hi <= 4611686018427387904.0) {  // [2^50, 2^62]
-    c = trunc(t0);
-    if (fabs(__dsub_rn(xb, c)) < 562949953421312.0) {  // 2^49
-      ci = __double2ll_rz(c);
-      return CF_OFFSET;
-    }
-  }
-  return CF_GENERAL;
 }
 
 // Packs the 32 fields of one group (width B, 1..31, at fg[f * kFtStride]) into B words at staged

@@ -11,6 +11,7 @@
 // bit offsets are an exclusive scan of len * bits.  All passes read the values once or twice
 // with coalesced loads; nothing here is a contraction, so the bound is HBM bandwidth.
 #include <type_traits>
+#include "glc_group.cuh"
 #include "glc_internal.h"
 #include "glc_scan.cuh"
 #include "glc_tma.cuh"
@@ -521,6 +522,159 @@ cudaError_t launch_fit(glc_dtype dt, const void* values, glc_column* c, void* sc
   }
   return cudaErrorInvalidValue;
 }
+
+// ---------------------------------------------------------------------------------------
+// Partitions of at most kFitShort values: a CTA fits one, from its exact sums to its width, in one
+// launch.  The values are read twice, the second time from L1 or L2 (a partition is at most 64 KB);
+// no chunk tables, and so no scans before the fit.  The residuals are 64-bit integers against a
+// prediction rounded in FP64 (glc_group.cuh).  30M uint32 in V6 partitions: 11 launches and their
+// gaps, 170 us, become one launch of 77 us.  Bound by the latency of a CTA (two barriers and the solve
+// between its two short passes), with eight CTAs per SM.
+// ---------------------------------------------------------------------------------------
+constexpr int kFsThreads = 256;
+constexpr int kFsWarps = kFsThreads / 32;
+
+// f(value, index) for this thread's values of a partition, 16 bytes at a time where they are aligned.
+template <typename T, typename F> __device__ __forceinline__ void fs_each(const T* __restrict__ v, int len, F f) {
+  constexpr int N = CgVec<T>::N;
+  int done = 0;
+  if ((reinterpret_cast<uintptr_t>(v) & 15) == 0) {
+    done = len / N * N;
+#pragma unroll 4
+    for (int j = threadIdx.x * N; j < done; j += kFsThreads * N) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(v + j));
+      T y[N];
+      memcpy(y, &u, 16);
+#pragma unroll
+      for (int k = 0; k < N; k++) f(y[k], j + k);
+    }
+  }
+#pragma unroll 4
+  for (int j = done + threadIdx.x; j < len; j += kFsThreads) f(__ldg(v + j), j);
+}
+
+// The largest |residual| of this thread's values: in 32 bits, or again in 64 where one does not fit.
+template <typename T>
+__device__ __forceinline__ unsigned long long fs_max(const T* __restrict__ v, int len, int mode, double t0, double t1,
+                                                     double c, long long ci) {
+  int mn = 0, mx = 0;
+  uint32_t wide = 0u;
+  auto one = [&](T y, int j, int m) {
+    const long long d = cg_field<T>(y, (double)j, m, t0, t1, c, ci);
+    const int lo = (int)(uint32_t)(unsigned long long)d;
+    wide |= (uint32_t)((unsigned long long)d >> 32) ^ (uint32_t)(lo >> 31);
+    mn = min(mn, lo);
+    mx = max(mx, lo);
+  };
+  // (the mode a constant in each loop)
+  if (mode == CF_NONNEG) fs_each<T>(v, len, [&](T y, int j) { one(y, j, CF_NONNEG); });
+  else if (TypeTraits<T>::is_signed && mode == CF_NONPOS) fs_each<T>(v, len, [&](T y, int j) { one(y, j, CF_NONPOS); });
+  else if (sizeof(T) == 8 && mode == CF_OFFSET) fs_each<T>(v, len, [&](T y, int j) { one(y, j, CF_OFFSET); });
+  else wide = 1u;
+  unsigned long long m = max((uint32_t)mx, 0u - (uint32_t)mn);
+  if (wide) {
+    m = 0;
+    fs_each<T>(v, len, [&](T y, int j) {
+      const unsigned long long ad = (unsigned long long)abs_ref(cg_field<T>(y, (double)j, mode, t0, t1, c, ci));
+      m = ad > m ? ad : m;
+    });
+  }
+  return m;
+}
+
+template <typename T> __global__ void __launch_bounds__(kFsThreads)
+fit_short_kernel(const T* __restrict__ values, const int32_t* __restrict__ starts, const int32_t* __restrict__ ends,
+                 int64_t P, int32_t* __restrict__ types, double* __restrict__ params, int32_t* __restrict__ bits,
+                 int64_t* __restrict__ err, int64_t* __restrict__ widths, unsigned long long* __restrict__ stats) {
+  __shared__ long long s_acc[kFsWarps][4];
+  __shared__ unsigned long long s_mx[kFsWarps];
+  __shared__ double s_line[3];
+  __shared__ long long s_ci;
+  __shared__ int s_mode;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t p = blockIdx.x;
+  const int s = starts[p], len = ends[p] - s;
+  const T* v = values + s;
+  HalfSums<T> hs;
+  bool over = false;
+  fs_each<T>(v, len, [&](T y, int j) {
+    hs.add(y, j);
+    over |= overflows_double<T>(y);
+  });
+  // (32 values a thread, j < 2^13, 32-bit halves: partials below 2^50)
+  const long long c0 = seg_sum48((long long)hs.s_lo, 32), c1 = sizeof(T) == 8 ? seg_sum48((long long)hs.s_hi, 32) : 0;
+  const long long c2 = seg_sum48((long long)hs.x_lo, 32), c3 = sizeof(T) == 8 ? seg_sum48((long long)hs.x_hi, 32) : 0;
+  if (lane == 0) {
+    s_acc[warp][0] = c0;
+    s_acc[warp][1] = c1;
+    s_acc[warp][2] = c2;
+    s_acc[warp][3] = c3;
+  }
+  over = __syncthreads_or(over);
+  if (tid == 0) {
+    long long a[4] = {0, 0, 0, 0};
+    for (int w = 0; w < kFsWarps; w++)
+      for (int k = 0; k < 4; k++) a[k] += s_acc[w][k];
+    double t0 = 0.0, t1 = 0.0, c = 0.0;
+    long long ci = 0;
+    int mode = CF_DIRECT;
+    if (!over) {
+      solve_line(len, (i128)a[0] + (i128)a[1] * ((i128)1 << 32), (i128)a[2] + (i128)a[3] * ((i128)1 << 32), t0, t1);
+      mode = cf_mode<T>(t0, t1, len, true, c, ci);  // (cg_field's differences need no bound on the values)
+    }
+    s_line[0] = t0;
+    s_line[1] = t1;
+    s_line[2] = c;
+    s_ci = ci;
+    s_mode = mode;
+  }
+  __syncthreads();
+  unsigned long long m = over ? 0ull : seg_max_u64(fs_max<T>(v, len, s_mode, s_line[0], s_line[1], s_line[2], s_ci), 32);
+  if (lane == 0) s_mx[warp] = m;
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 0; w < kFsWarps; w++) m = s_mx[w] > m ? s_mx[w] : m;
+    const int b = over ? (int)sizeof(T) * 8 : bits_for((long long)m);
+    types[p] = over ? MODEL_DIRECT_COPY : MODEL_LINEAR;
+    params[4 * p] = s_line[0];
+    params[4 * p + 1] = s_line[1];
+    params[4 * p + 2] = 0.0;
+    params[4 * p + 3] = 0.0;
+    bits[p] = b;
+    err[p] = (long long)m;
+    widths[p] = (int64_t)len * b;
+    // [1] the widest field, [3] the bound on partitions per 4096-value tile (without the last partition)
+    const unsigned long long k = p < P - 1 ? (unsigned long long)((kDecodeTile + len - 1) / len) : 0ull;
+    if ((unsigned long long)b > *(volatile unsigned long long*)(stats + 1)) atomicMax(stats + 1, (unsigned long long)b);
+    if (k > *(volatile unsigned long long*)(stats + 3)) atomicMax(stats + 3, k);
+  }
+}
+
+size_t fit_short_scratch_bytes(int64_t P) { return sizeof(int64_t) * (size_t)(P + scan_num_tiles(P) + 4); }
+
+cudaError_t launch_fit_short(glc_dtype dt, const void* values, glc_column* c, void* scratch, int64_t* d_stats, cudaStream_t s) {
+  const int64_t P = c->P;
+  int64_t* widths = (int64_t*)scratch;
+  int64_t* tmp = widths + ((P + 3) & ~3ll);
+  cudaError_t e = cudaMemsetAsync(d_stats, 0, 4 * sizeof(int64_t), s);
+  if (e != cudaSuccess) return e;
+  const unsigned g = (unsigned)P;
+  unsigned long long* st = (unsigned long long*)d_stats;
+#define GLC_FIT_SHORT(T)                                                                                              \
+  fit_short_kernel<T><<<g, kFsThreads, 0, s>>>((const T*)values, c->d_start, c->d_end, P, c->d_types, c->d_params, \
+                                               c->d_bits, c->d_err, widths, st)
+  switch (dt) {
+    case GLC_I32: GLC_FIT_SHORT(int32_t); break;
+    case GLC_I64: GLC_FIT_SHORT(int64_t); break;
+    case GLC_U64: GLC_FIT_SHORT(uint64_t); break;
+    case GLC_U32: GLC_FIT_SHORT(uint32_t); break;
+    default: return cudaErrorInvalidValue;
+  }
+#undef GLC_FIT_SHORT
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  return exclusive_scan<int64_t>(widths, c->d_offs, P, d_stats, tmp, s);
+}
+
 
 // ---------------------------------------------------------------------------------------
 // Derived tables: 32-byte partition descriptors and the decode tile table.

@@ -89,6 +89,56 @@ constexpr double kHalfBias = 0x1.fffffffffffffp-2;    // 0.5 - 2^-54
 // low 32 bits (the low bits of (y - pred) + K), which is all the packing of a width <= 31 reads.
 enum : int { CF_DIRECT = 0, CF_NONNEG = 1, CF_NONPOS = 2, CF_GENERAL = 3, CF_OFFSET = 4 };
 
+// Exact sum over a reduction segment of W lanes (32, or 16 at L = 256) of values |v| < 2^48: for a
+// whole warp two redux sums of the 24-bit limbs (each limb's sum stays below 2^29).
+__device__ __forceinline__ long long seg_sum48(long long v, int W) {
+  if (W == 32) {
+    const unsigned lo = __reduce_add_sync(FULL_MASK, (unsigned)v & 0xFFFFFFu);
+    const int hi = __reduce_add_sync(FULL_MASK, (int)(v >> 24));
+    return (long long)hi * 16777216ll + (long long)lo;
+  }
+  for (int msk = W >> 1; msk > 0; msk >>= 1) v += __shfl_xor_sync(FULL_MASK, v, msk);
+  return v;
+}
+__device__ __forceinline__ unsigned seg_max_u32(unsigned v, int W) {
+  if (W == 32) return __reduce_max_sync(FULL_MASK, v);
+  for (int msk = W >> 1; msk > 0; msk >>= 1) {
+    const unsigned o = __shfl_xor_sync(FULL_MASK, v, msk);
+    v = o > v ? o : v;
+  }
+  return v;
+}
+__device__ __forceinline__ unsigned seg_or_u32(unsigned v, int W) {
+  if (W == 32) return __reduce_or_sync(FULL_MASK, v);
+  for (int msk = W >> 1; msk > 0; msk >>= 1) v |= __shfl_xor_sync(FULL_MASK, v, msk);
+  return v;
+}
+__device__ __forceinline__ unsigned long long seg_max_u64(unsigned long long v, int W) {
+  const unsigned hi = seg_max_u32((unsigned)(v >> 32), W);
+  const unsigned lo = seg_max_u32((unsigned)(v >> 32) == hi ? (unsigned)v : 0u, W);
+  return ((unsigned long long)hi << 32) | lo;
+}
+
+// The residual mode of a partition from its line and the range test of its values.
+template <typename T>
+__device__ __forceinline__ int cf_mode(double t0, double t1, int len, bool vsafe, double& c, long long& ci) {
+  const double xa = t0, xb = __fma_rn(t1, (double)(len - 1), t0);  // the ends (fma is monotone in i)
+  const double lo = fmin(xa, xb), hi = fmax(xa, xb);
+  constexpr double kS = 2251799813685248.0;  // 2^51
+  const double hi_ok = sizeof(T) == 4 ? (TypeTraits<T>::is_signed ? 2147483646.0 : 4294967294.0) : kS;
+  const double lo_ok = sizeof(T) == 4 ? -2147483647.0 : -kS;
+  if (vsafe && lo >= -0.25 && hi <= hi_ok) return CF_NONNEG;
+  if (TypeTraits<T>::is_signed && vsafe && hi <= 0.25 && lo >= lo_ok) return CF_NONPOS;
+  if (sizeof(T) == 8 && lo >= 1125899906842624.0 && hi <= 4611686018427387904.0) {  // [2^50, 2^62]
+    c = trunc(t0);
+    if (fabs(__dsub_rn(xb, c)) < 562949953421312.0) {  // 2^49
+      ci = __double2ll_rz(c);
+      return CF_OFFSET;
+    }
+  }
+  return CF_GENERAL;
+}
+
 // One value's residual, or the value itself for direct copy, in 64 bits (the slow path).  The fast
 // modes' formulas are those of cg_resid, exact modulo 2^64 as calc_delta is for signed types; a
 // uint64 partition outside direct copy holds values up to 2^53, where calc_delta does not saturate.

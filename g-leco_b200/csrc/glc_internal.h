@@ -202,6 +202,11 @@ size_t fit_scratch_bytes(const int32_t* unused, int64_t n, int64_t P);
 // Fits every partition of c (starts/ends set); d_stats[0] = total bits, d_stats[1] = max bits.
 cudaError_t launch_fit(glc_dtype dt, const void* values, glc_column* c, void* scratch, size_t scratch_bytes,
                        int64_t* d_stats, cudaStream_t s);
+// The same for partitions of at most kFitShort values each (scratch:
+// fit_short_scratch_bytes).
+constexpr int kFitShort = 8192;
+size_t fit_short_scratch_bytes(int64_t P);
+cudaError_t launch_fit_short(glc_dtype dt, const void* values, glc_column* c, void* scratch, int64_t* d_stats, cudaStream_t s);
 cudaError_t launch_desc_and_tiles(glc_column* c, cudaStream_t s);
 // compress_fixed.cu: one-pass compression of fixed partitions of L values, L a divisor of 4096 and >= 256
 // One column of a launch (its arrays are the column's own, or its slices of a batch's arrays).
@@ -393,9 +398,10 @@ struct PartOut {
 };
 cudaError_t launch_partition_variable(glc_ctx* ctx, glc_dtype dt, const void* values, int64_t n, const PartOut& out,
                                       cudaStream_t s, std::string* err);
-// partition_v6.cu: the reference's GPU partitioner boundaries (pool-allocated starts/ends)
+// partition_v6.cu: the reference's GPU partitioner boundaries, into starts/ends from pool_alloc or a
+// column's arrays (out.stats is not used: the partitions come unfitted)
 constexpr int32_t kV6Base = 2048;  // base size compress passes (api/G-LeCo.cuh:384-387)
 cudaError_t launch_partition_v6(glc_ctx* ctx, glc_dtype dt, const void* values, int64_t n, int32_t base,
-                                int32_t** d_starts, int32_t** d_ends, int64_t* P, cudaStream_t s);
+                                const PartOut& out, cudaStream_t s);
 
 }  // namespace glc

@@ -22,11 +22,10 @@
 // and S2/n - m*m as one fma, as the reference's compiler contracts them) so the oracle can
 // restate it bit for bit; the four warp values are added in warp order (the reference adds them
 // with float atomics in whatever order the warps finish).  The thresholds come from a radix
-// select instead of a sort, and partitions are emitted in order from a prefix sum of per-block
-// counts instead of atomics followed by a sort.  "The i-th smallest value is below threshold k"
-// is "i < the number of values below threshold k", so only those three counts are needed.
+// select instead of a sort.  "The i-th smallest value is below threshold k" is "i < the number of
+// values below threshold k", so only those three counts are needed; the sizes then are four runs of
+// blocks, and partition o is computed from o instead of atomics followed by a sort.
 #include "glc_internal.h"
-#include "glc_scan.cuh"
 
 namespace glc {
 namespace {
@@ -85,156 +84,176 @@ __device__ __forceinline__ float key_float(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-// The values of rank nb/4, nb/2, 3nb/4 (0-based, ascending): a most-significant-digit radix
-// select, 8 bits per pass, one CTA.
-__global__ void __launch_bounds__(1024) v6_threshold_kernel(const float* __restrict__ var, int64_t nb,
-                                                            float* __restrict__ thr) {
-  __shared__ unsigned int hist[256];
-  __shared__ uint32_t s_prefix;
-  __shared__ long long s_rank;
-  for (int q = 0; q < 3; q++) {
-    long long rank = q == 0 ? nb / 4 : (q == 1 ? nb / 2 : 3 * nb / 4);
-    uint32_t prefix = 0, mask = 0;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-      for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
-      __syncthreads();
-      for (int64_t i = threadIdx.x; i < nb; i += blockDim.x) {
-        const uint32_t k = float_key(var[i]);
-        if ((k & mask) == prefix) atomicAdd(&hist[(k >> shift) & 255u], 1u);
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        long long r = rank;
-        uint32_t b = 0;
-        for (; b < 255u; b++) {
-          if (r < (long long)hist[b]) break;
-          r -= hist[b];
-        }
-        s_prefix = prefix | (b << shift);
-        s_rank = r;
-      }
-      __syncthreads();
-      prefix = s_prefix;
-      rank = s_rank;
-      mask |= 0xffu << shift;
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) thr[q] = key_float(prefix);
-    __syncthreads();
-  }
+// Everything between the block values and the partitions, in one CTA (as five launches, with one
+// thread walking the bins, it took 70 us of a 30M-value column's 380; 10 us here): the values of rank
+// nb/4, nb/2, 3nb/4 (0-based, ascending) by a most-significant-digit radix select, 8 bits per pass, a
+// warp per rank; how many block values lie below each (float comparison, as the reference's); and
+// the number of partitions.
+//
+// edge[k], k < 3: blocks [edge[k - 1], edge[k]) (edge[-1] = 0) have partitions of 4, 2 and 1 times the
+// base, those from edge[2] on of half the base.
+struct V6Plan {
+  int64_t edge[3];
+  int64_t total;
+};
+
+// Partitions of the blocks before block i (all of them full).
+__device__ __forceinline__ int64_t v6_before(int64_t i, const int64_t* e) {
+  const int64_t a = i < e[0] ? i : e[0], b = i < e[1] ? i : e[1], c = i < e[2] ? i : e[2];
+  return 2 * a + 4 * (b - a) + 8 * (c - b) + 16 * (i - c);
+}
+// Partition size of block i: its rank among the sorted values against the three counts.
+__device__ __forceinline__ int64_t v6_size(int64_t i, const int64_t* e, int64_t base) {
+  return i < e[0] ? 4 * base : (i < e[1] ? 2 * base : (i < e[2] ? base : base / 2));
 }
 
-// below[k] = number of block values below threshold k (float comparison, as the reference's).
-__global__ void v6_below_kernel(const float* __restrict__ var, int64_t nb, const float* __restrict__ thr,
-                                unsigned long long* __restrict__ below) {
-  const float t0 = thr[0], t1 = thr[1], t2 = thr[2];
-  unsigned long long c0 = 0, c1 = 0, c2 = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += (int64_t)gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(1024)
+v6_select_kernel(const float* __restrict__ var, int64_t nb, int64_t n, int64_t base, V6Plan* __restrict__ plan) {
+  __shared__ unsigned int hist[3][256];
+  __shared__ uint32_t s_prefix[3];
+  __shared__ long long s_rank[3];
+  __shared__ unsigned int s_below[3];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < 3) {
+    s_rank[tid] = tid == 0 ? nb / 4 : (tid == 1 ? nb / 2 : 3 * nb / 4);
+    s_prefix[tid] = 0u;
+    s_below[tid] = 0u;
+  }
+  uint32_t mask = 0u;
+  for (int shift = 24; shift >= 0; shift -= 8) {
+    if (tid < 768) hist[tid >> 8][tid & 255] = 0u;
+    __syncthreads();
+    const uint32_t p0 = s_prefix[0], p1 = s_prefix[1], p2 = s_prefix[2];
+    for (int64_t i = tid; i < nb; i += 1024) {
+      const uint32_t k = float_key(var[i]), bin = (k >> shift) & 255u, pre = k & mask;
+      if (pre == p0) atomicAdd(&hist[0][bin], 1u);
+      if (pre == p1) atomicAdd(&hist[1][bin], 1u);
+      if (pre == p2) atomicAdd(&hist[2][bin], 1u);
+    }
+    __syncthreads();
+    if (warp < 3) {  // lane l holds bins [8 l, 8 l + 8): the first bin whose running count passes the rank
+      unsigned int c[8], sum = 0u;
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        c[j] = hist[warp][8 * lane + j];
+        sum += c[j];
+      }
+      unsigned int inc = sum;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const unsigned int y = __shfl_up_sync(FULL_MASK, inc, d);
+        if (lane >= d) inc += y;
+      }
+      const long long rank = s_rank[warp];
+      const unsigned hit = __ballot_sync(FULL_MASK, (long long)inc > rank);
+      const int l = hit ? __ffs(hit) - 1 : 31;
+      __syncwarp();
+      if (lane == l) {
+        long long r = rank - (long long)(inc - sum);
+        int j = 0;
+        for (; j < 7; j++) {
+          if (r < (long long)c[j]) break;
+          r -= c[j];
+        }
+        s_prefix[warp] |= (uint32_t)(8 * lane + j) << shift;
+        s_rank[warp] = r;
+      }
+    }
+    mask |= 0xffu << shift;
+    __syncthreads();
+  }
+  const float t0 = key_float(s_prefix[0]), t1 = key_float(s_prefix[1]), t2 = key_float(s_prefix[2]);
+  unsigned int c0 = 0, c1 = 0, c2 = 0;
+  for (int64_t i = tid; i < nb; i += 1024) {
     const float x = var[i];
     c0 += x < t0;
     c1 += x < t1;
     c2 += x < t2;
   }
-  if (c0) atomicAdd(below, c0);
-  if (c1) atomicAdd(below + 1, c1);
-  if (c2) atomicAdd(below + 2, c2);
-}
-
-// Partition size of block i: its rank among the sorted values against the three counts.
-__device__ __forceinline__ int64_t v6_size(int64_t i, const unsigned long long* below, int64_t base) {
-  return i < (int64_t)below[0] ? 4 * base : (i < (int64_t)below[1] ? 2 * base : (i < (int64_t)below[2] ? base : base / 2));
-}
-
-__global__ void v6_count_kernel(int64_t nb, const unsigned long long* __restrict__ below, int64_t n, int64_t base,
-                                int64_t* __restrict__ counts) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nb) return;
-  const int64_t start = i * 8 * base;
-  const int64_t end = start + 8 * base < n ? start + 8 * base : n;
-  const int64_t size = v6_size(i, below, base);
-  counts[i] = (end - start + size - 1) / size;
-}
-
-__global__ void v6_emit_kernel(int64_t nb, const unsigned long long* __restrict__ below, int64_t n, int64_t base,
-                               const int64_t* __restrict__ offs, int32_t* __restrict__ starts,
-                               int32_t* __restrict__ ends) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nb) return;
-  const int64_t start = i * 8 * base;
-  const int64_t end = start + 8 * base < n ? start + 8 * base : n;
-  const int64_t size = v6_size(i, below, base);
-  int64_t o = offs[i];
-  for (int64_t j = start; j < end; j += size, o++) {
-    starts[o] = (int32_t)j;
-    ends[o] = (int32_t)(j + size < end ? j + size : end);
+  c0 = __reduce_add_sync(FULL_MASK, c0);
+  c1 = __reduce_add_sync(FULL_MASK, c1);
+  c2 = __reduce_add_sync(FULL_MASK, c2);
+  if (lane == 0) {
+    atomicAdd(&s_below[0], c0);
+    atomicAdd(&s_below[1], c1);
+    atomicAdd(&s_below[2], c2);
   }
+  __syncthreads();
+  if (tid == 0) {
+    int64_t e[3];
+    e[0] = s_below[0];
+    e[1] = s_below[1] > e[0] ? s_below[1] : e[0];
+    e[2] = s_below[2] > e[1] ? s_below[2] : e[1];
+    const int64_t last = n - (nb - 1) * 8 * base, size = v6_size(nb - 1, e, base);
+    for (int k = 0; k < 3; k++) plan->edge[k] = e[k];
+    plan->total = v6_before(nb - 1, e) + (last + size - 1) / size;
+  }
+}
+
+__global__ void v6_emit_kernel(int64_t nb, const V6Plan* __restrict__ plan, int64_t n, int64_t base, int64_t P,
+                               int32_t* __restrict__ starts, int32_t* __restrict__ ends) {
+  const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (o >= P) return;
+  int64_t e[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) e[k] = plan->edge[k];
+  int64_t i = nb - 1;  // the partition's block
+  const int64_t c0 = 2 * e[0], c1 = c0 + 4 * (e[1] - e[0]), c2 = c1 + 8 * (e[2] - e[1]);
+  if (o < v6_before(nb - 1, e)) i = o < c0 ? o / 2 : o < c1 ? e[0] + (o - c0) / 4 : o < c2 ? e[1] + (o - c1) / 8 : e[2] + (o - c2) / 16;
+  const int64_t size = v6_size(i, e, base), end = 8 * base * (i + 1) < n ? 8 * base * (i + 1) : n;
+  const int64_t s = 8 * base * i + (o - v6_before(i, e)) * size;
+  starts[o] = (int32_t)s;
+  ends[o] = (int32_t)(s + size < end ? s + size : end);
 }
 
 template <typename T>
-cudaError_t v6_typed(glc_ctx* ctx, const T* values, int64_t n, int64_t base, int32_t** d_starts, int32_t** d_ends,
-                     int64_t* P, cudaStream_t s) {
+cudaError_t v6_typed(glc_ctx* ctx, const T* values, int64_t n, int64_t base, const PartOut& out, cudaStream_t s) {
   const int64_t block_len = 8 * base;
   const int64_t nb = (n + block_len - 1) / block_len;
-  float* var = nullptr;
-  float* thr = nullptr;  // 3 thresholds, then (8-byte aligned) 3 counts of values below them
-  int64_t* counts = nullptr;
-  int64_t* scratch = nullptr;
-  int64_t* total = nullptr;
-  const int64_t ntiles = scan_num_tiles(nb);
-  cudaError_t e;
-  auto cleanup = [&]() {
-    if (var) cudaFreeAsync(var, s);
-    if (thr) cudaFreeAsync(thr, s);
-    if (counts) cudaFreeAsync(counts, s);
-    if (scratch) cudaFreeAsync(scratch, s);
-    if (total) cudaFreeAsync(total, s);
-  };
-  if ((e = pool_alloc(ctx, &var, 4 * nb, s)) != cudaSuccess || (e = pool_alloc(ctx, &thr, 64, s)) != cudaSuccess ||
-      (e = pool_alloc(ctx, &counts, 8 * nb, s)) != cudaSuccess ||
-      (e = pool_alloc(ctx, &scratch, 8 * (ntiles + 1), s)) != cudaSuccess ||
-      (e = pool_alloc(ctx, &total, 8, s)) != cudaSuccess) {
-    cleanup();
-    return e;
-  }
+  V6Plan* plan = nullptr;  // then the block values
+  cudaError_t e = pool_alloc(ctx, &plan, sizeof(V6Plan) + 4 * (size_t)nb, s);
+  if (e != cudaSuccess) return e;
+  float* var = (float*)(plan + 1);
+  int32_t *starts = nullptr, *ends = nullptr;
   v6_variance_kernel<T><<<(unsigned)nb, kV6Threads, 0, s>>>(values, n, block_len, var);
-  v6_threshold_kernel<<<1, 1024, 0, s>>>(var, nb, thr);
-  unsigned long long* below = (unsigned long long*)(thr + 4);
-  if ((e = cudaMemsetAsync(below, 0, 3 * sizeof(unsigned long long), s)) != cudaSuccess) {
-    cleanup();
-    return e;
+  v6_select_kernel<<<1, 1024, 0, s>>>(var, nb, n, base, plan);
+  if ((e = cudaGetLastError()) == cudaSuccess &&
+      (e = cudaMemcpyAsync(ctx->h_stats, &plan->total, 8, cudaMemcpyDeviceToHost, s)) == cudaSuccess)
+    e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) {
+    const int64_t P = ctx->h_stats[0];
+    if (out.column) {
+      out.column->P = P;
+      if ((e = out.alloc(out.column, s)) == cudaSuccess) {
+        starts = out.column->d_start;
+        ends = out.column->d_end;
+      }
+    } else {
+      *out.P = P;
+      if ((e = pool_alloc(ctx, out.starts, 4 * P, s)) == cudaSuccess && (e = pool_alloc(ctx, out.ends, 4 * P, s)) == cudaSuccess) {
+        starts = *out.starts;
+        ends = *out.ends;
+      }
+    }
+    if (e == cudaSuccess) {
+      v6_emit_kernel<<<(unsigned)((P + 255) / 256), 256, 0, s>>>(nb, plan, n, base, P, starts, ends);
+      e = cudaGetLastError();
+    }
   }
-  const unsigned g = (unsigned)((nb + 255) / 256);
-  v6_below_kernel<<<g < 64 ? g : 64, 256, 0, s>>>(var, nb, thr, below);
-  v6_count_kernel<<<g, 256, 0, s>>>(nb, below, n, base, counts);
-  if ((e = cudaGetLastError()) != cudaSuccess || (e = exclusive_scan<int64_t>(counts, counts, nb, total, scratch, s)) != cudaSuccess ||
-      (e = cudaMemcpyAsync(ctx->h_stats, total, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-      (e = cudaStreamSynchronize(s)) != cudaSuccess) {
-    cleanup();
-    return e;
-  }
-  *P = ctx->h_stats[0];
-  if ((e = pool_alloc(ctx, d_starts, 4 * *P, s)) != cudaSuccess || (e = pool_alloc(ctx, d_ends, 4 * *P, s)) != cudaSuccess) {
-    cleanup();
-    return e;
-  }
-  v6_emit_kernel<<<g, 256, 0, s>>>(nb, below, n, base, counts, *d_starts, *d_ends);
-  e = cudaGetLastError();
-  cleanup();
+  cudaFreeAsync(plan, s);
   return e;
 }
 
 }  // namespace
 
 cudaError_t launch_partition_v6(glc_ctx* ctx, glc_dtype dt, const void* values, int64_t n, int32_t base,
-                                int32_t** d_starts, int32_t** d_ends, int64_t* P, cudaStream_t s) {
-  *d_starts = *d_ends = nullptr;
-  *P = 0;
+                                const PartOut& out, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   switch (dt) {
-    case GLC_I32: return v6_typed<int32_t>(ctx, (const int32_t*)values, n, base, d_starts, d_ends, P, s);
-    case GLC_I64: return v6_typed<int64_t>(ctx, (const int64_t*)values, n, base, d_starts, d_ends, P, s);
-    case GLC_U64: return v6_typed<uint64_t>(ctx, (const uint64_t*)values, n, base, d_starts, d_ends, P, s);
-    case GLC_U32: return v6_typed<uint32_t>(ctx, (const uint32_t*)values, n, base, d_starts, d_ends, P, s);
+    case GLC_I32: return v6_typed<int32_t>(ctx, (const int32_t*)values, n, base, out, s);
+    case GLC_I64: return v6_typed<int64_t>(ctx, (const int64_t*)values, n, base, out, s);
+    case GLC_U64: return v6_typed<uint64_t>(ctx, (const uint64_t*)values, n, base, out, s);
+    case GLC_U32: return v6_typed<uint32_t>(ctx, (const uint32_t*)values, n, base, out, s);
   }
   return cudaErrorInvalidValue;
 }
