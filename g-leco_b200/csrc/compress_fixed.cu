@@ -16,8 +16,8 @@
 // The column's word array is allocated at its exact size between the two kernels (the scan gives
 // the total); the slots cost one extra write and read of the compressed bits.
 //
-// The partition-length choice of a batch (choose_lengths_kernel) measures three lengths at once in
-// persistent CTAs of producer, solver and compute warps and packs the usual choice, 4096, on the way.
+// The partition-length choice of a batch (choose_lengths_kernel) measures three lengths at once and
+// packs the usual choice, 4096, on the way.
 #include <type_traits>
 #include "glc_group.cuh"
 #include "glc_internal.h"
@@ -26,21 +26,9 @@
 
 namespace glc {
 
-constexpr int kCfThreads = 256;                       // compute threads (8 warps)
 constexpr int kCfMinLen = 256;
 constexpr int kCfMaxParts = kDecodeTile / kCfMinLen;  // 16 partitions per tile at L = 256
-constexpr int kCfPerThread = kDecodeTile / kCfThreads;  // 16 values per thread
-constexpr int kCfMaxSegs = 16;                        // reduction segments (half-warps at L = 256)
-
-// The work area of the packing: the transposed fields (32 x 129 words) and the staged words (4096
-// plus a pad word per 32), or the 64-bit residuals of the wide-field path (4096 x 8 bytes).
-constexpr int kCfWorkBytes = (32 * 129 + kDecodeTile + kDecodeTile / 32) * 4;
-static_assert(kCfWorkBytes >= kDecodeTile * 8, "the work area holds a tile's 64-bit residuals");
-// A stage holds a tile's values from the 16-byte block of the first one; for 8-byte types it is
-// also the work area of its tile.
-template <typename T> __host__ __device__ constexpr int cf_stage_bytes() {
-  return sizeof(T) == 8 ? kCfWorkBytes : kDecodeTile * (int)sizeof(T) + 16;
-}
+constexpr int kCfMaxSegs = 16;                        // reduction segments (8 lanes each at L = 256)
 
 // A launch: work item i = one 4096-value tile of column owner[i] (every column of one element
 // type, tiles in order), or of `single` when cols is null.
@@ -58,50 +46,7 @@ struct FixedCompressArgs {
   long long* terr;            // partition's descriptor (tile-relative offset) and max error
 };
 
-__device__ __forceinline__ void cf_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kCfThreads) : "memory"); }
-
-// The producer lane of a launch: stages item blockIdx.x + k * gridDim.x of the work list into stage
-// k % S (its values, from the 16-byte block that holds the first one), with the item, its
-// column and the offset of its first value in the stage; an item of -1 marks the end.
-template <typename T, int S>
-__device__ __forceinline__ void cf_produce(const FixedCompressArgs& a, uint8_t* smem, uint64_t* full, uint64_t* empty,
-                                           int64_t* s_stile, int* s_shead, int* s_scol) {
-  int64_t item = blockIdx.x;
-  for (int k = 0;; k++, item += gridDim.x) {
-    const int st = k % S;
-    if (k >= S && !mbar_wait_sleep(&empty[st], (uint32_t)((k / S) - 1) & 1u)) {
-      atomicExch(a.status, (unsigned long long)DEVERR_TIMEOUT);
-      s_stile[st] = -1;  // the compute warps stop at this stage (or time out on it)
-      mbar_arrive(&full[st]);
-      return;
-    }
-    if (item >= a.nitems) {
-      s_stile[st] = -1;
-      mbar_arrive(&full[st]);  // no copy: completes the phase, the compute warps see the end
-      return;
-    }
-    const int c = a.owner ? a.owner[item] : 0;
-    const CfColumn& col = a.cols ? a.cols[c] : a.single;
-    const int64_t e0 = (item - col.item_base) * kDecodeTile;
-    const int cnt = (int)((col.n - e0) < kDecodeTile ? (col.n - e0) : kDecodeTile);
-    const uintptr_t addr = reinterpret_cast<uintptr_t>(reinterpret_cast<const T*>(col.values) + e0);
-    const int head = (int)(addr & 15);
-    s_stile[st] = item;
-    s_shead[st] = head;
-    s_scol[st] = c;
-    // the copy covers the 16-byte blocks that hold the tile's values, never another page
-    const uint32_t bytes = (uint32_t)((head + (int64_t)cnt * (int64_t)sizeof(T) + 15) & ~15ll);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_arrive_expect_tx(&full[st], bytes);
-    tma_bulk_load(smem + (size_t)st * cf_stage_bytes<T>(), reinterpret_cast<const void*>(addr - head), bytes,
-                  &full[st]);
-  }
-}
-
 // ---- pieces of the compute warps -----------------------------------------------------------
-
-constexpr int kFtStride = 129;                        // transposed fields: field f of 32-value group G at f * 129 + G
-constexpr int kFtWords = 32 * kFtStride;
 
 // Per value, for the range tests of the partition: uint64 keeps the max of the high words, above
 // 2^21 when some value exceeds 2^53 (direct copy; exactly 2^21 is decided by a rescan of the
@@ -114,17 +59,17 @@ template <typename T> __device__ __forceinline__ void value_flag(uint32_t& f, T 
     else f = hi > f ? hi : f;
   }
 }
-// Whether a uint64 partition whose largest high word is exactly 2^21 holds a value above 2^53.
-template <typename T> __device__ __noinline__ bool cf_any_above_2_53(const T* __restrict__ xp, int len) {
-  for (int i = 0; i < len; i++)
-    if ((uint64_t)xp[i] > (1ull << 53)) return true;
-  return false;
-}
-// Direct copy for the range flag of a partition (the reference copies a uint64 partition with a
-// value above 2^53 directly).
-template <typename T> __device__ __forceinline__ bool cf_overflows(uint32_t flag, const T* __restrict__ xp, int len) {
+// Direct copy for the range flag of the partition whose `len` values start at value j0 of the tile (the
+// reference copies a uint64 partition with a value above 2^53 directly): a largest high word of exactly
+// 2^21 is decided by its values.
+template <typename T> __device__ __forceinline__ bool cg_overflows(uint32_t flag, const uint8_t* stage, int j0, int len) {
   if (TypeTraits<T>::is_signed || sizeof(T) != 8) return false;
-  return flag > 0x200000u || (flag == 0x200000u && cf_any_above_2_53<T>(xp, len));
+  bool over = flag > 0x200000u;
+  if (flag == 0x200000u) {
+#pragma unroll 1
+    for (int j = j0; j < j0 + len && !over; j++) over = (uint64_t)*reinterpret_cast<const T*>(stage + cg_at<T>(j)) > (1ull << 53);
+  }
+  return over;
 }
 
 // K + y as a double from the bits of y (|y| <= 2^51).
@@ -138,8 +83,6 @@ template <typename T> __device__ __forceinline__ double magic_of(T y) {
     return __hiloint2double(0x43380000, (int)(uint32_t)y);
   }
 }
-__device__ __forceinline__ uint32_t low_field(double d) { return (uint32_t)__double2loint(__dadd_rn(d, kMagic)); }
-
 __device__ __forceinline__ uint64_t madw_u(uint32_t a, uint32_t b, uint64_t c) {
   uint64_t d;
   asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
@@ -149,216 +92,6 @@ __device__ __forceinline__ int64_t madw_s(int32_t a, int32_t b, int64_t c) {
   int64_t d;
   asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
   return d;
-}
-
-// The HalfSums of a thread's values y_m = xp[r + g m] (m < 16), without the index per value:
-// sum (r + g m) y_m = r sum y_m + g sum m y_m, each sum accumulated by one 32 x 32 -> 64-bit
-// multiply-add per value and half (m is a compile-time constant); every partial stays below 2^48.
-template <typename T, bool FULL>
-__device__ __forceinline__ void cf_sums(const T* __restrict__ xp, int r, int g, int len, HalfSums<T>& hs,
-                                        uint32_t& flag) {
-  typedef typename HalfSums<T>::Acc Acc;
-  Acc s_lo = 0, s_hi = 0, t_lo = 0, t_hi = 0;
-  const T* p = xp + r;
-#pragma unroll
-  for (int m = 0; m < kCfPerThread; m++) {
-    if (FULL || r + g * m < len) {
-      const T y = p[g * m];
-      value_flag<T>(flag, y);
-      if (sizeof(T) == 8) {
-        const uint32_t yl = (uint32_t)(uint64_t)y, yh = (uint32_t)((uint64_t)y >> 32);
-        s_lo = (Acc)madw_u(yl, 1u, (uint64_t)s_lo);
-        if (m) t_lo = (Acc)madw_u(yl, (uint32_t)m, (uint64_t)t_lo);
-        if (TypeTraits<T>::is_signed) {
-          s_hi = (Acc)madw_s((int32_t)yh, 1, (int64_t)s_hi);
-          if (m) t_hi = (Acc)madw_s((int32_t)yh, m, (int64_t)t_hi);
-        } else {
-          s_hi = (Acc)madw_u(yh, 1u, (uint64_t)s_hi);
-          if (m) t_hi = (Acc)madw_u(yh, (uint32_t)m, (uint64_t)t_hi);
-        }
-      } else if (TypeTraits<T>::is_signed) {
-        s_lo = (Acc)madw_s((int32_t)y, 1, (int64_t)s_lo);
-        if (m) t_lo = (Acc)madw_s((int32_t)y, m, (int64_t)t_lo);
-      } else {
-        s_lo = (Acc)madw_u((uint32_t)y, 1u, (uint64_t)s_lo);
-        if (m) t_lo = (Acc)madw_u((uint32_t)y, (uint32_t)m, (uint64_t)t_lo);
-      }
-    }
-  }
-  hs.s_lo += s_lo;
-  hs.s_hi += s_hi;
-  hs.x_lo += (Acc)r * s_lo + (Acc)g * t_lo;
-  hs.x_hi += (Acc)r * s_hi + (Acc)g * t_hi;
-}
-
-template <typename T, bool FULL, bool NEG>
-__device__ __forceinline__ unsigned long long cf_resid_sign(const T* __restrict__ xp, int r, int g, int len,
-                                                            double t0, double t1, uint32_t (&fl)[kCfPerThread]) {
-  double dm = 0.0, xd = (double)r;
-  const double gd = (double)g;
-#pragma unroll
-  for (int m = 0; m < kCfPerThread; m++) {
-    const int i = r + g * m;
-    fl[m] = 0u;
-    if (FULL || i < len) {
-      const double yc = magic_of<T>(xp[i]);
-      const double x = __fma_rn(t1, xd, t0);
-      double d;
-      if (!NEG) {
-        d = __dsub_rn(yc, __dadd_rz(__dadd_rn(x, kHalfBias), kMagic));  // (K + y) - (K + pred)
-      } else {
-        d = __dadd_rn(__dsub_rn(yc, 2.0 * kMagic), __dadd_rz(__dsub_rn(kHalfBias, x), kMagic));  // (y - K) + (K - pred)
-      }
-      dm = fmax(dm, fabs(d));
-      fl[m] = low_field(d);
-    }
-    xd = __dadd_rn(xd, gd);
-  }
-  return (unsigned long long)dm;
-}
-
-template <typename T, bool FULL>
-__device__ __forceinline__ bool cf_resid_offset(const T* __restrict__ xp, int r, int g, int len, double t0,
-                                                double t1, double c, long long ci, uint32_t (&fl)[kCfPerThread],
-                                                unsigned long long& mx) {
-  double dm = 0.0, xd = (double)r;
-  const double gd = (double)g;
-  uint32_t range = 0u;
-#pragma unroll
-  for (int m = 0; m < kCfPerThread; m++) {
-    const int i = r + g * m;
-    fl[m] = 0u;
-    if (FULL || i < len) {
-      const uint64_t yo = (uint64_t)xp[i] - (uint64_t)ci;  // y - c
-      const uint32_t yh = (uint32_t)(yo >> 32);
-      range |= yh ^ (uint32_t)((int32_t)yh >> 31);
-      const double yk = __hiloint2double((int)(yh + 0x43380000u), (int)(uint32_t)yo);  // K + (y - c)
-      const double v = __dadd_rn(__dsub_rn(__fma_rn(t1, xd, t0), c), 0.5);          // x - c + 0.5
-      const double d = __dsub_rn(yk, __dadd_rz(v, kMagic));                          // - (K + pred - c)
-      dm = fmax(dm, fabs(d));
-      fl[m] = low_field(d);
-    }
-    xd = __dadd_rn(xd, gd);
-  }
-  mx = (unsigned long long)dm;
-  return range < 0x80000u;  // every |y - c| below 2^51 (y - c in [-2^51, 2^51))
-}
-
-template <typename T>
-__device__ __forceinline__ unsigned long long cf_resid_general(const T* __restrict__ xp, int r, int g, int len,
-                                                               double t0, double t1, uint32_t (&fl)[kCfPerThread]) {
-  unsigned long long mx = 0;
-#pragma unroll
-  for (int m = 0; m < kCfPerThread; m++) {
-    const int i = r + g * m;
-    fl[m] = 0u;
-    if (i < len) {
-      const long long d = calc_delta<T>(xp[i], predict_from<T>(__fma_rn(t1, (double)i, t0)));
-      fl[m] = (uint32_t)d;
-      const unsigned long long ad = (unsigned long long)abs_ref(d);
-      mx = ad > mx ? ad : mx;
-    }
-  }
-  return mx;
-}
-
-// Packs the 32 fields of one group (width B, 1..31, at fg[f * kFtStride]) into B words at staged
-// word o onward (staged word k at stg[k + k / 32]).
-template <int B>
-__device__ __forceinline__ void cf_pack_group(const uint32_t* __restrict__ fg, uint32_t* __restrict__ stg, int o) {
-  constexpr uint32_t kMask = (1u << B) - 1u;
-  uint32_t w = 0u;
-#pragma unroll
-  for (int f = 0; f < 32; f++) {
-    const uint32_t v = fg[f * kFtStride] & kMask;
-    const int sh = (f * B) & 31;
-    w |= v << sh;
-    if (sh + B >= 32) {
-      const int k = o + ((f * B) >> 5);
-      stg[k + (k >> 5)] = w;
-      w = sh + B > 32 ? v >> (32 - sh) : 0u;
-    }
-  }
-}
-
-__device__ __forceinline__ void cf_pack_dispatch(int b, const uint32_t* __restrict__ fg, uint32_t* __restrict__ stg,
-                                              int o) {
-  switch (b) {
-#define GLC_CF_PACK(B) \
-  case B: cf_pack_group<B>(fg, stg, o); break;
-    GLC_CF_PACK(1) GLC_CF_PACK(2) GLC_CF_PACK(3) GLC_CF_PACK(4) GLC_CF_PACK(5) GLC_CF_PACK(6) GLC_CF_PACK(7)
-    GLC_CF_PACK(8) GLC_CF_PACK(9) GLC_CF_PACK(10) GLC_CF_PACK(11) GLC_CF_PACK(12) GLC_CF_PACK(13) GLC_CF_PACK(14)
-    GLC_CF_PACK(15) GLC_CF_PACK(16) GLC_CF_PACK(17) GLC_CF_PACK(18) GLC_CF_PACK(19) GLC_CF_PACK(20)
-    GLC_CF_PACK(21) GLC_CF_PACK(22) GLC_CF_PACK(23) GLC_CF_PACK(24) GLC_CF_PACK(25) GLC_CF_PACK(26)
-    GLC_CF_PACK(27) GLC_CF_PACK(28) GLC_CF_PACK(29) GLC_CF_PACK(30) GLC_CF_PACK(31)
-#undef GLC_CF_PACK
-    default: break;  // width 0: no words
-  }
-}
-
-// The words of a partition of width b (1..64) whose exact residuals are rp[0, len), one thread per
-// word: word w holds the partition's bits [32 w, 32 w + 32), from the field holding bit 32 w and
-// the following ones (fields past len are zero).  One routine for every width (the wide-field path
-// is taken by a few tiles; a copy per width made the kernels' code several times larger than the
-// instruction cache).
-__device__ __noinline__ void cf_words_dispatch(int b, const long long* rp, int len, uint32_t* __restrict__ out,
-                                               int tid) {
-  if (b <= 0) return;
-  const int nwp = (int)(((long long)len * b + 31) >> 5);
-  const uint32_t mb = 0xffffffffu / (uint32_t)b + 1u;  // 32 w / b by a multiply-high (32 w < 2^18)
-  const uint64_t mask = b >= 64 ? ~0ull : ((1ull << b) - 1ull);
-  for (int w = tid; w < nwp; w += kCfThreads) {
-    int j = b > 1 ? (int)__umulhi((uint32_t)(32 * w), mb) : 32 * w;
-    const int s = 32 * w - j * b;
-    uint64_t v = ((uint64_t)rp[j] & mask) >> s;
-    int have = b - s;
-    while (have < 32 && ++j < len) {
-      v |= ((uint64_t)rp[j] & mask) << have;
-      have += b;
-    }
-    out[w] = (uint32_t)v;
-  }
-}
-
-// The exact residuals of one thread's values (value i of its partition at xp[i], written to rp[i];
-// for 8-byte types rp is xp, each value read before its residual replaces it).  The FP64 modes give
-// y - pred as an exact integer-valued double, converted once; the others use the integer formula.
-template <typename T>
-__device__ __forceinline__ void cf_store_resid(const T* xp, long long* rp, int r, int g, int len, int mode, double t0,
-                                               double t1) {
-  for (int m = 0; m < kCfPerThread; m++) {
-    const int i = r + g * m;
-    if (i >= len) break;
-    const T y = xp[i];
-    long long d;
-    if (mode == CF_DIRECT) {
-      d = (long long)(uint64_t)y;  // the field is the value itself (zero-extended)
-    } else if (mode == CF_NONNEG) {
-      const double x = __fma_rn(t1, (double)i, t0);
-      d = __double2ll_rn(__dsub_rn(magic_of<T>(y), __dadd_rz(__dadd_rn(x, kHalfBias), kMagic)));
-    } else if (TypeTraits<T>::is_signed && mode == CF_NONPOS) {
-      const double x = __fma_rn(t1, (double)i, t0);
-      d = __double2ll_rn(
-          __dadd_rn(__dsub_rn(magic_of<T>(y), 2.0 * kMagic), __dadd_rz(__dsub_rn(kHalfBias, x), kMagic)));
-    } else {
-      d = calc_delta<T>(y, predict_from<T>(__fma_rn(t1, (double)i, t0)));
-    }
-    rp[i] = d;
-  }
-}
-
-// The length choice's CTA: eight compute warps, the producer warp and the solver warp.  Per step
-// k the compute warps take the sums of tile k + 1 and the residuals, widths and words of tile k,
-// while the solver warp fits the lines of tile k + 1 and the producer stages the next tile as soon
-// as a stage is free: the fit's long dependency chain (128-bit arithmetic, two divisions) runs
-// beside the compute warps instead of between two of their barriers.  Every wait is bounded.  Three
-// stages at two CTAs per SM (two stages at three CTAs per SM fit its registers too, but measured 3 %
-// slower).
-constexpr int kCfChooseStages = 3;
-constexpr int kCfFixCTA = kCfThreads + 64;
-
-template <typename T> __host__ __device__ constexpr int cf_fix_smem_bytes(int stages) {
-  return stages * cf_stage_bytes<T>() + (sizeof(T) == 4 ? kCfWorkBytes : 0);
 }
 
 // ---- the compress kernel ---------------------------------------------------------------------
@@ -522,13 +255,7 @@ fixed_compress_kernel(const __grid_constant__ FixedCompressArgs a) {
       flag = TypeTraits<T>::is_signed ? (flag | s_flag[s]) : (s_flag[s] > flag ? s_flag[s] : flag);
     }
     const int len = (cnt - tid * L) < L ? (cnt - tid * L) : L;
-    bool ovf = false;  // a uint64 value above 2^53: direct copy
-    if (!TypeTraits<T>::is_signed && sizeof(T) == 8) {
-      ovf = flag > 0x200000u;
-      if (flag == 0x200000u)
-        for (int j = tid * L; j < tid * L + len && !ovf; j++)
-          ovf = (uint64_t)*reinterpret_cast<const T*>(stage + cg_at<T>(j)) > (1ull << 53);
-    }
+    const bool ovf = cg_overflows<T>(flag, stage, tid * L, len);  // a value above 2^53: direct copy
     const bool vsafe = sizeof(T) == 4 || flag < 0x80000u;
     double t0 = 0.0, t1 = 0.0, c = 0.0;
     long long ci = 0;
@@ -659,318 +386,268 @@ const double c = s_c[p];
   }
 }
 
-// The partition-length choice of the batched compress, one tile per step with the CTA layout of
-// fixed_compress_kernel (eight compute warps, a producer warp staging tiles three ahead, a solver
-// warp): the tile's four 1024-value quarters, its two halves and the whole tile are fitted from
-// exact per-quarter sums (the index offsets of a half or the tile added exactly) by the solver warp
-// while the compute warps measure the previous tile; every value's residual is measured against the
-// three lines that cover it (with the residual modes of fixed_compress_kernel), and the bits of each
-// candidate length are added into the column's choice_bits[0..2] (1024, 2048, 4096).  The widths
+// The largest |residual| of a group's `len` values against one line, in mode MODE (0 where it is a
+// direct copy): in 32 bits, or again in 64 where one does not fit.
+template <typename T, int MODE>
+__device__ __forceinline__ unsigned long long cg_max(const uint8_t* __restrict__ row, int len, int i0, double t0, double t1,
+                                                     double c, long long ci) {
+  int mn = 0, mx = 0;
+  uint32_t wide = 0u;
+  double xi = (double)i0;
+#pragma unroll 4
+  for (int f = 0; f < len; f++) {
+    const long long d = cg_field<T>(*reinterpret_cast<const T*>(row + f * (int)sizeof(T)), xi, MODE, t0, t1, c, ci);
+    xi = __dadd_rn(xi, 1.0);
+    const int lo = (int)(uint32_t)(unsigned long long)d;
+    wide |= (uint32_t)((unsigned long long)d >> 32) ^ (uint32_t)(lo >> 31);
+    mn = min(mn, lo);
+    mx = max(mx, lo);
+  }
+  if (!wide) return max((uint32_t)mx, 0u - (uint32_t)mn);
+  unsigned long long m = 0;
+  xi = (double)i0;
+#pragma unroll 1
+  for (int f = 0; f < len; f++) {
+    const unsigned long long ad = (unsigned long long)abs_ref(
+        cg_field<T>(*reinterpret_cast<const T*>(row + f * (int)sizeof(T)), xi, MODE, t0, t1, c, ci));
+    xi = __dadd_rn(xi, 1.0);
+    m = ad > m ? ad : m;
+  }
+  return m;
+}
+template <typename T>
+__device__ __forceinline__ unsigned long long cg_max_mode(const uint8_t* __restrict__ row, int len, int i0, int mode, double t0,
+                                                          double t1, double c, long long ci) {
+  if (mode == CF_DIRECT) return 0;
+  if (mode == CF_NONNEG) return cg_max<T, CF_NONNEG>(row, len, i0, t0, t1, c, ci);
+  if (TypeTraits<T>::is_signed && mode == CF_NONPOS) return cg_max<T, CF_NONPOS>(row, len, i0, t0, t1, c, ci);
+  if (sizeof(T) == 8 && mode == CF_OFFSET) return cg_max<T, CF_OFFSET>(row, len, i0, t0, t1, c, ci);
+  return cg_max<T, CF_GENERAL>(row, len, i0, t0, t1, c, ci);
+}
+
+// A full group against the quarter's, the half's and the tile's line, all of them CF_NONNEG (the usual
+// case), each value read once.  A width needs only the bit length of the largest |residual|, i.e. its
+// FP64 exponent: the largest high word of |d| for the lines that only count bits.  With PACK the
+// tile's line keeps its fields and exact maximum, as cg_resid does (false: one does not fit 32 bits).
+template <typename T, bool PACK>
+__device__ __forceinline__ bool cg_three(const uint8_t* __restrict__ row, const double (&t0)[3], const double (&t1)[3],
+                                         const int (&i0)[3], uint32_t (&fl)[32], unsigned long long (&m)[3]) {
+  constexpr long long kBits = 0x4338000000000000ll;
+  double xd[3];
+  uint32_t mh[3] = {0u, 0u, 0u}, wide = 0u;
+  int mn = 0, mx = 0;
+#pragma unroll
+  for (int c = 0; c < 3; c++) xd[c] = (double)i0[c];
+#pragma unroll
+  for (int k = 0; k < 32 / CgVec<T>::N; k++) {
+    const CgVec<T> vec(row + 16 * k);
+#pragma unroll
+    for (int u = 0; u < CgVec<T>::N; u++) {
+      const int f = k * CgVec<T>::N + u;
+      const double yc = magic_of<T>(vec.v[u]);  // K + y
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double pm = __dadd_rz(__dadd_rn(__fma_rn(t1[c], xd[c], t0[c]), kHalfBias), kMagic);  // K + pred
+        xd[c] = __dadd_rn(xd[c], 1.0);
+        if (PACK && c == 2) {
+          const uint64_t y = TypeTraits<T>::is_signed ? (uint64_t)(long long)vec.v[u] : (uint64_t)vec.v[u];
+          const uint64_t d = y - (uint64_t)(__double_as_longlong(pm) - kBits);
+          const int lo = (int)(uint32_t)d;
+          fl[f] = (uint32_t)d;
+          wide |= (uint32_t)(d >> 32) ^ (uint32_t)(lo >> 31);
+          mn = min(mn, lo);
+          mx = max(mx, lo);
+        } else {
+          const uint32_t h = (uint32_t)__double2hiint(__dsub_rn(yc, pm)) & 0x7fffffffu;
+          mh[c] = max(mh[c], h);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++) m[c] = mh[c] ? (1ull << ((mh[c] >> 20) - 1023)) : 0ull;  // the same bit length
+  if (PACK) m[2] = max((uint32_t)mx, 0u - (uint32_t)mn);
+  return wide == 0u;
+}
+
+// The partition-length choice of the batched compress, a CTA of 128 threads per tile as in
+// fixed_compress_kernel, a warp per 1024-value quarter: the tile's quarters, its two halves and the
+// whole tile are fitted from exact per-quarter sums (the index offsets of a half or the tile added
+// exactly); every value's residual is measured against the three lines that cover it, and the bits of
+// each candidate length are added into the column's choice_bits[0..2] (1024, 2048, 4096).  The widths
 // are the ones the compress at that length computes, so the column's size is exact.  With PACK the
 // tile is also compressed at length 4096 -- the usual choice -- exactly as fixed_compress_kernel
 // would (the tile's line from the same exact sums, the same residual modes and packing): its words
 // into its slot, its descriptor and max error into tdesc / terr, its bits into tile_bits.
-template <typename T, bool PACK> __global__ void __launch_bounds__(kCfFixCTA, 2)
+// Bound by instruction issue (three lines per value).  169M values of 1024 int32, int64 and uint64
+// columns: 1068 -> 620 us in all, against persistent CTAs of 256 compute threads that staged the fields.
+template <typename T, bool PACK> __global__ void __launch_bounds__(kCgThreads, 5)
 choose_lengths_kernel(const __grid_constant__ FixedCompressArgs a) {
-  constexpr int S = kCfChooseStages;
-  extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ __align__(8) uint64_t full[S], empty[S], sums[S], lines[S];
-  __shared__ int64_t s_stile[S];
-  __shared__ int s_shead[S];
-  __shared__ int s_scol[S];
-  __shared__ long long s_acc[S][8][4];
-  __shared__ uint32_t s_flag[S][8];
-  __shared__ double s_t0[S][7], s_t1[S][7], s_c[S][7];
-  __shared__ long long s_ci[S][7];
-  __shared__ int s_mode[S][7], s_len[S][7];
-  __shared__ unsigned long long s_m[8][3];
-  __shared__ int s_ok, s_b0;
-  if (threadIdx.x == 0) {
-    for (int st = 0; st < S; st++) {
-      mbar_init(&full[st], 1);
-      mbar_init(&empty[st], 1);
-      mbar_init(&sums[st], kCfThreads / 32);
-      mbar_init(&lines[st], 1);
+  extern __shared__ __align__(128) uint8_t stage[];
+  __shared__ long long s_acc[4][4];  // per quarter: exact partial sums and range flags
+  __shared__ uint32_t s_flag[4];
+  __shared__ double s_t0[7], s_t1[7], s_c[7];  // line 0 the tile, 1-2 its halves, 3-6 its quarters
+  __shared__ long long s_ci[7];
+  __shared__ int s_mode[7], s_len[7];
+  __shared__ unsigned long long s_m[4][3];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t item = blockIdx.x;
+  const CfColumn& col = a.cols[a.owner[item]];
+  const int64_t e0 = (item - col.item_base) * kDecodeTile, left = col.n - e0;
+  const int cnt = (int)(left < kDecodeTile ? left : kDecodeTile);
+  const int glen = cnt - 32 * tid < 32 ? cnt - 32 * tid : 32;  // values of the group (<= 0: none)
+  uint8_t* row = stage + tid * cg_row_bytes<T>();
+  cg_load<T>(stage, reinterpret_cast<const T*>(col.values) + e0, cnt, tid);
+  cg_load_wait();
+  __syncthreads();
+  {  // exact sums per quarter and the range flags
+    HalfSums<T> hs;
+    uint32_t flag = 0;
+    cg_sums<T>(row, 32 * lane, hs, flag);
+    const long long c0 = seg_sum48((long long)hs.s_lo, 32);
+    const long long c1 = sizeof(T) == 8 ? seg_sum48((long long)hs.s_hi, 32) : 0;
+    const long long c2 = seg_sum48((long long)hs.x_lo, 32);
+    const long long c3 = sizeof(T) == 8 ? seg_sum48((long long)hs.x_hi, 32) : 0;
+    flag = TypeTraits<T>::is_signed ? seg_or_u32(flag, 32) : seg_max_u32(flag, 32);
+    if (lane == 0) {
+      s_acc[warp][0] = c0;
+      s_acc[warp][1] = c1;
+      s_acc[warp][2] = c2;
+      s_acc[warp][3] = c3;
+      s_flag[warp] = flag;
     }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid >= kCfThreads + 32) {  // ---- solver warp: line l = 0 the tile, 1-2 its halves, 3-6 its quarters ----
-    for (int k = 0;; k++) {
-      const int st = k % S;
-      int ok = 1;
-      if (lane == 0) {
-        ok = mbar_wait_sleep(&sums[st], (uint32_t)(k / S) & 1u);
-        if (!ok) atomicExch(a.status, (unsigned long long)DEVERR_TIMEOUT);
-      }
-      if (!__shfl_sync(FULL_MASK, ok, 0)) return;
-      const int64_t item = s_stile[st];
-      if (item < 0) return;
-      if (lane < 7) {
-        const CfColumn& col = a.cols[s_scol[st]];
-        const int64_t e0 = (item - col.item_base) * kDecodeTile;
-        const int cnt = (int)((col.n - e0) < kDecodeTile ? (col.n - e0) : kDecodeTile);
-        const int l = lane;
-        const int q0 = l == 0 ? 0 : (l < 3 ? (l - 1) * 2 : l - 3);
-        const int q1 = l == 0 ? 4 : (l < 3 ? q0 + 2 : q0 + 1);
-        i128 sy = 0, sxy = 0;
-        uint32_t flag = 0;
-        for (int qq = q0; qq < q1; qq++) {
-          long long a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-          for (int w = 2 * qq; w < 2 * qq + 2; w++) {
-            a0 += s_acc[st][w][0];
-            a1 += s_acc[st][w][1];
-            a2 += s_acc[st][w][2];
-            a3 += s_acc[st][w][3];
-            flag = TypeTraits<T>::is_signed ? (flag | s_flag[st][w]) : (s_flag[st][w] > flag ? s_flag[st][w] : flag);
-          }
-          const i128 qy = (i128)a0 + (i128)a1 * ((i128)1 << 32);
-          sy += qy;
-          sxy += (i128)a2 + (i128)a3 * ((i128)1 << 32) + (i128)(1024 * (qq - q0)) * qy;  // quarter index -> line index
+  if (tid < 7) {  // the lines
+    const int l = tid;
+    const int q0 = l == 0 ? 0 : (l < 3 ? (l - 1) * 2 : l - 3);
+    const int q1 = l == 0 ? 4 : (l < 3 ? q0 + 2 : q0 + 1);
+    i128 sy = 0, sxy = 0;
+    uint32_t flag = 0;
+    for (int q = q0; q < q1; q++) {
+      flag = TypeTraits<T>::is_signed ? (flag | s_flag[q]) : (s_flag[q] > flag ? s_flag[q] : flag);
+      const i128 qy = (i128)s_acc[q][0] + (i128)s_acc[q][1] * ((i128)1 << 32);
+      sy += qy;
+      sxy += (i128)s_acc[q][2] + (i128)s_acc[q][3] * ((i128)1 << 32) + (i128)(1024 * (q - q0)) * qy;  // quarter index -> line index
+    }
+    int len = cnt - 1024 * q0;
+    len = len < 0 ? 0 : (len < 1024 * (q1 - q0) ? len : 1024 * (q1 - q0));
+    const bool ovf = len > 0 && cg_overflows<T>(flag, stage, 1024 * q0, len);
+    const bool vsafe = sizeof(T) == 4 || flag < 0x80000u;
+    double t0 = 0.0, t1 = 0.0, c = 0.0;
+    long long ci = 0;
+    int mode = CF_DIRECT;
+    if (len > 0 && !ovf) {
+      solve_line(len, sy, sxy, t0, t1);
+      mode = cf_mode<T>(t0, t1, len, vsafe, c, ci);
+    }
+    s_t0[l] = t0;
+    s_t1[l] = t1;
+    s_c[l] = c;
+    s_ci[l] = ci;
+    s_mode[l] = mode;
+    s_len[l] = len;
+  }
+  __syncthreads();
+  uint32_t fl[32];  // PACK: the low 32 bits of each value's residual against the tile's line
+  bool slow = false;
+  {  // max |residual| of each value against its quarter's, its half's and the tile's line
+    const int ls[3] = {3 + warp, 1 + (warp >> 1), 0};
+    const int i0[3] = {32 * lane, 32 * (tid & 63), 32 * tid};
+    unsigned long long mx[3] = {0, 0, 0};
+    if (glen > 0) {
+      bool fused = glen == 32, tile_done = false;
+#pragma unroll
+      for (int c = 0; c < 3; c++) fused = fused && s_mode[ls[c]] == CF_NONNEG;
+      if (fused) {
+        const double t0[3] = {s_t0[ls[0]], s_t0[ls[1]], s_t0[ls[2]]}, t1[3] = {s_t1[ls[0]], s_t1[ls[1]], s_t1[ls[2]]};
+        tile_done = cg_three<T, PACK>(row, t0, t1, i0, fl, mx);
+        slow = PACK && !tile_done;
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < 2; c++) {  // (one body for both lines)
+          const int l = c ? 1 + (warp >> 1) : 3 + warp, i = c ? 32 * (tid & 63) : 32 * lane;
+          const unsigned long long m = cg_max_mode<T>(row, glen, i, s_mode[l], s_t0[l], s_t1[l], s_c[l], s_ci[l]);
+          if (c) mx[1] = m;
+          else mx[0] = m;
         }
-        int len = cnt - 1024 * q0;
-        len = len < 0 ? 0 : (len < 1024 * (q1 - q0) ? len : 1024 * (q1 - q0));
-        const T* x = reinterpret_cast<const T*>(smem + (size_t)st * cf_stage_bytes<T>() + s_shead[st]);
-        const bool ovf = len > 0 && cf_overflows<T>(flag, x + 1024 * q0, len);
-        const bool vsafe = sizeof(T) == 4 || flag < 0x80000u;
-        double t0 = 0.0, t1 = 0.0, c = 0.0;
-        long long ci = 0;
-        int mode = CF_DIRECT;
-        if (len > 0 && !ovf) {
-          solve_line(len, sy, sxy, t0, t1);
-          mode = cf_mode<T>(t0, t1, len, vsafe, c, ci);
+        if (PACK && glen == 32) {
+          const int mode = s_mode[0];
+          uint32_t mag = 0u;
+          if (mode == CF_NONNEG) tile_done = cg_resid<T, CF_NONNEG>(row, i0[2], s_t0[0], s_t1[0], 0.0, 0, fl, mag);
+          else if (TypeTraits<T>::is_signed && mode == CF_NONPOS)
+            tile_done = cg_resid<T, CF_NONPOS>(row, i0[2], s_t0[0], s_t1[0], 0.0, 0, fl, mag);
+          else if (sizeof(T) == 8 && mode == CF_OFFSET)
+            tile_done = cg_resid<T, CF_OFFSET>(row, i0[2], s_t0[0], s_t1[0], s_c[0], s_ci[0], fl, mag);
+          mx[2] = mag;
         }
-        s_t0[st][l] = t0;
-        s_t1[st][l] = t1;
-        s_c[st][l] = c;
-        s_ci[st][l] = ci;
-        s_mode[st][l] = mode;
-        s_len[st][l] = len;
+        slow = PACK && !tile_done;
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&lines[st]);
+      if (!tile_done) mx[2] = cg_max_mode<T>(row, glen, i0[2], s_mode[0], s_t0[0], s_t1[0], s_c[0], s_ci[0]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) mx[c] = seg_max_u64(mx[c], 32);
+    if (lane == 0) {
+      s_m[warp][0] = mx[0];
+      s_m[warp][1] = mx[1];
+      s_m[warp][2] = mx[2];
     }
   }
-  if (tid >= kCfThreads) {  // ---- producer ----
-    if (tid == kCfThreads) cf_produce<T, S>(a, smem, full, empty, s_stile, s_shead, s_scol);
+  slow = __syncthreads_or(slow);
+  // lane l < 7 (of every warp): line l's width and bits; the three lengths' sums by shuffles
+  unsigned long long add[3] = {0, 0, 0}, m_line = 0;
+  int b_line = 0;
+  if (lane < 7 && s_len[lane] > 0) {
+    const int l = lane;
+    const int c = l == 0 ? 2 : (l < 3 ? 1 : 0);                  // index into s_m's lines
+    const int w0 = l == 0 ? 0 : (l < 3 ? 2 * (l - 1) : l - 3);   // the line's quarters
+    const int w1 = l == 0 ? 4 : (l < 3 ? w0 + 2 : w0 + 1);
+    for (int w = w0; w < w1; w++) m_line = s_m[w][c] > m_line ? s_m[w][c] : m_line;
+    b_line = s_mode[l] == CF_DIRECT ? (int)sizeof(T) * 8 : bits_for((long long)m_line);
+    add[c] = (unsigned long long)s_len[l] * (unsigned long long)b_line;
+  }
+  if (warp == 0) {
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) add[c] += __shfl_xor_sync(FULL_MASK, add[c], o);  // lanes 0-7
+  }
+  if (tid == 0) {
+    for (int c = 0; c < 3; c++)
+      if (add[c]) atomicAdd(col.choice_bits + c, add[c]);
+    if (PACK) {  // the tile as one partition of 4096 (line 0): width, descriptor, max error, bits
+      const bool direct = s_mode[0] == CF_DIRECT;
+      PartDesc d;
+      d.theta0 = s_t0[0];
+      d.theta1 = s_t1[0];
+      d.bit_off = 0;
+      d.start = (int32_t)e0;
+      d.bits_type = (b_line & 0xff) | ((direct ? MODEL_DIRECT_COPY : MODEL_LINEAR) << 8);
+      a.tdesc[item] = d;
+      a.terr[item] = direct ? 0 : (long long)m_line;
+      a.tile_bits[item] = (int64_t)cnt * b_line;
+      if (b_line > 0) atomicMax(col.stats + 1, (unsigned long long)b_line);
+    }
+  }
+  if (!PACK) return;
+  const int b = __shfl_sync(FULL_MASK, b_line, 0);
+  uint32_t* out = a.slots + item * a.slot_words;
+  if (!slow && b <= 31) {  // each warp's groups, staged over its rows and copied (fixed_compress_kernel)
+    uint32_t* stg = reinterpret_cast<uint32_t*>(stage + (tid & ~31) * cg_row_bytes<T>());
+    if (glen > 0) cg_pack_dispatch(b, fl, stg + lane * (b | 1));
+    __syncwarp();
+    const int groups = __popc(__ballot_sync(FULL_MASK, glen > 0));
+    cg_copy_words<true>(stg, out + 32 * warp * b, groups * b, b, lane);
     return;
   }
-  // ---- compute warps: thread tid measures values r + 64 m of quarter q ----
-  const int q = tid >> 6, r = tid & 63;
-  auto stage_sums = [&](int st) {  // exact sums per quarter (two warps each) and the range flags
-    const int64_t item = s_stile[st];
-    if (item >= 0) {
-      const CfColumn& col = a.cols[s_scol[st]];
-      const int64_t e0 = (item - col.item_base) * kDecodeTile;
-      const int cnt = (int)((col.n - e0) < kDecodeTile ? (col.n - e0) : kDecodeTile);
-      const int qlen = (cnt - 1024 * q) < 0 ? 0 : ((cnt - 1024 * q) < 1024 ? (cnt - 1024 * q) : 1024);
-      const T* xq = reinterpret_cast<const T*>(smem + (size_t)st * cf_stage_bytes<T>() + s_shead[st]) + 1024 * q;
-      HalfSums<T> hs;
-      uint32_t flag = 0;
-      if (qlen == 1024) cf_sums<T, true>(xq, r, 64, 1024, hs, flag);
-      else if (qlen > 0) cf_sums<T, false>(xq, r, 64, qlen, hs, flag);
-      const long long c0 = seg_sum48((long long)hs.s_lo, 32);
-      const long long c1 = sizeof(T) == 8 ? seg_sum48((long long)hs.s_hi, 32) : 0;
-      const long long c2 = seg_sum48((long long)hs.x_lo, 32);
-      const long long c3 = sizeof(T) == 8 ? seg_sum48((long long)hs.x_hi, 32) : 0;
-      flag = TypeTraits<T>::is_signed ? seg_or_u32(flag, 32) : seg_max_u32(flag, 32);
-      if (lane == 0) {
-        s_acc[st][warp][0] = c0;
-        s_acc[st][warp][1] = c1;
-        s_acc[st][warp][2] = c2;
-        s_acc[st][warp][3] = c3;
-        s_flag[st][warp] = flag;
-      }
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sums[st]);
-  };
-
-  if (tid == 0) {
-    s_ok = mbar_wait_sleep(&full[0], 0);
-    if (!s_ok) {
-      atomicExch(a.status, (unsigned long long)DEVERR_TIMEOUT);
-      mbar_wait_bounded(&full[0], 0);  // a copy in flight lands before the CTA exits
-    }
-  }
-  cf_sync();
-  if (!s_ok) return;
-  mbar_try_wait(&full[0], 0);
-  if (s_stile[0] < 0) return;
-  stage_sums(0);
-
-  for (int k = 0;; k++) {
-    const int st = k % S, st1 = (k + 1) % S;
-    const uint32_t par = (uint32_t)(k / S) & 1u, par1 = (uint32_t)((k + 1) / S) & 1u;
-    if (tid == 0) {
-      s_ok = mbar_wait_sleep(&full[st1], par1);
-      if (!s_ok) {
-        atomicExch(a.status, (unsigned long long)DEVERR_TIMEOUT);
-        mbar_wait_bounded(&full[st1], par1);  // a copy in flight lands before the CTA exits
-      } else {
-        s_ok = mbar_wait_sleep(&lines[st], par);
-        if (!s_ok) atomicExch(a.status, (unsigned long long)DEVERR_TIMEOUT);
-      }
-    }
-    cf_sync();
-    if (!s_ok) return;
-    mbar_try_wait(&full[st1], par1);
-    mbar_try_wait(&lines[st], par);
-    const int64_t item1 = s_stile[st1];
-    stage_sums(st1);
-
-    const int64_t item = s_stile[st];
-    const CfColumn& col = a.cols[s_scol[st]];
-    const int64_t e0 = (item - col.item_base) * kDecodeTile;
-    const int cnt = (int)((col.n - e0) < kDecodeTile ? (col.n - e0) : kDecodeTile);
-    const T* x = reinterpret_cast<const T*>(smem + (size_t)st * cf_stage_bytes<T>() + s_shead[st]);
-    const int qlen = (cnt - 1024 * q) < 0 ? 0 : ((cnt - 1024 * q) < 1024 ? (cnt - 1024 * q) : 1024);
-    const T* xq = x + 1024 * q;
-    uint32_t fl[kCfPerThread];  // PACK: the low 32 bits of each value's residual against the tile's line
-#pragma unroll
-    for (int m = 0; m < kCfPerThread; m++) fl[m] = 0u;
-    {  // max |residual| of each value against its quarter's, its half's and the tile's line
-      const int ls[3] = {3 + q, 1 + (q >> 1), 0};
-      const int off[3] = {0, 1024 * (q & 1), 1024 * q};
-      unsigned long long mx[3] = {0, 0, 0};
-      if (qlen > 0) {
-        if (s_mode[st][ls[0]] == CF_NONNEG && s_mode[st][ls[1]] == CF_NONNEG && s_mode[st][ls[2]] == CF_NONNEG) {
-          // the common case in one pass: each value read once, K + y shared by the three lines.  A
-          // width needs only the bit length of the largest |residual|, i.e. its FP64 exponent: the
-          // largest high word of |d| (sign cleared) for the lines that only count bits; the tile's
-          // line keeps the exact maximum when it is packed (its max error is stored)
-          double t0[3], t1[3], xd[3], dm = 0.0;
-          uint32_t mh[3] = {0u, 0u, 0u};
-#pragma unroll
-          for (int c = 0; c < 3; c++) {
-            t0[c] = s_t0[st][ls[c]];
-            t1[c] = s_t1[st][ls[c]];
-            xd[c] = (double)(r + off[c]);
-          }
-#pragma unroll
-          for (int m = 0; m < kCfPerThread; m++) {
-            const int i = r + 64 * m;
-            if (i < qlen) {
-              const double yc = magic_of<T>(xq[i]);
-#pragma unroll
-              for (int c = 0; c < 3; c++) {
-                const double d = __dsub_rn(yc, __dadd_rz(__dadd_rn(__fma_rn(t1[c], xd[c], t0[c]), kHalfBias), kMagic));
-                if (PACK && c == 2) {
-                  dm = fmax(dm, fabs(d));
-                  fl[m] = low_field(d);
-                } else {
-                  const uint32_t h = (uint32_t)__double2hiint(d) & 0x7fffffffu;
-                  mh[c] = h > mh[c] ? h : mh[c];
-                }
-              }
-            }
-#pragma unroll
-            for (int c = 0; c < 3; c++) xd[c] = __dadd_rn(xd[c], 64.0);
-          }
-#pragma unroll
-          for (int c = 0; c < 3; c++) {
-            // an integer with the same bit length as the largest |residual| (|d| < 2^53, integral)
-            mx[c] = mh[c] ? (1ull << ((mh[c] >> 20) - 1023)) : 0ull;
-          }
-          if (PACK) mx[2] = (unsigned long long)dm;
-        } else {
-#pragma unroll
-          for (int c = 0; c < 3; c++) {
-            // the line's index of value i of the quarter is i + off: read through a pointer moved back by off
-            const int l = ls[c], mode = s_mode[st][l];
-            const T* xl = xq - off[c];
-            const int rl = r + off[c], ll = qlen + off[c];
-            const double t0 = s_t0[st][l], t1 = s_t1[st][l];
-            uint32_t fd[kCfPerThread];  // the quarter's and the half's fields are not kept
-            uint32_t (&f)[kCfPerThread] = (PACK && c == 2) ? fl : fd;
-            bool general = mode == CF_GENERAL;
-            if (mode == CF_NONNEG) {
-              mx[c] = cf_resid_sign<T, false, false>(xl, rl, 64, ll, t0, t1, f);
-            } else if (TypeTraits<T>::is_signed && mode == CF_NONPOS) {
-              mx[c] = cf_resid_sign<T, false, true>(xl, rl, 64, ll, t0, t1, f);
-            } else if (sizeof(T) == 8 && mode == CF_OFFSET) {
-              general = !cf_resid_offset<T, false>(xl, rl, 64, ll, t0, t1, s_c[st][l], s_ci[st][l], f, mx[c]);
-            }
-            if (general) mx[c] = cf_resid_general<T>(xl, rl, 64, ll, t0, t1, f);
-          }
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < 3; c++) mx[c] = seg_max_u64(mx[c], 32);
-      if (lane == 0) {
-        s_m[warp][0] = mx[0];
-        s_m[warp][1] = mx[1];
-        s_m[warp][2] = mx[2];
-      }
-    }
-    cf_sync();
-    if (tid < 32) {  // lane l < 7: line l's width and bits; the three lengths' sums by shuffles
-      const int l = lane;
-      unsigned long long add[3] = {0, 0, 0};
-      int b_line = 0;
-      unsigned long long m_line = 0;
-      if (l < 7 && s_len[st][l] > 0) {
-        const int c = l == 0 ? 2 : (l < 3 ? 1 : 0);                      // index into s_m's lines
-        const int w0 = l == 0 ? 0 : (l < 3 ? 4 * (l - 1) : 2 * (l - 3));  // the line's warps
-        const int w1 = l == 0 ? 8 : (l < 3 ? w0 + 4 : w0 + 2);
-        for (int w = w0; w < w1; w++) m_line = s_m[w][c] > m_line ? s_m[w][c] : m_line;
-        b_line = s_mode[st][l] == CF_DIRECT ? (int)sizeof(T) * 8 : bits_for((long long)m_line);
-        add[c] = (unsigned long long)s_len[st][l] * (unsigned long long)b_line;
-      }
-#pragma unroll
-      for (int c = 0; c < 3; c++)
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) add[c] += __shfl_xor_sync(FULL_MASK, add[c], o);  // lanes 0-7
-      if (lane == 0) {
-        for (int c = 0; c < 3; c++)
-          if (add[c]) atomicAdd(col.choice_bits + c, add[c]);
-        if (PACK) {  // the tile as one partition of 4096 (line 0): width, descriptor, max error, bits
-          const bool direct = s_mode[st][0] == CF_DIRECT;
-          const int b = b_line;
-          PartDesc d;
-          d.theta0 = s_t0[st][0];
-          d.theta1 = s_t1[st][0];
-          d.bit_off = 0;
-          d.start = (int32_t)e0;
-          d.bits_type = (b & 0xff) | ((direct ? MODEL_DIRECT_COPY : MODEL_LINEAR) << 8);
-          a.tdesc[item] = d;
-          a.terr[item] = direct ? 0 : (long long)m_line;
-          a.tile_bits[item] = (int64_t)cnt * b;
-          if (b > 0) atomicMax(col.stats + 1, (unsigned long long)b);
-          s_b0 = b;
-        }
-      }
-    }
-    cf_sync();  // every compute thread is done with s_m (and, without PACK, with stage st)
-    if (PACK) {  // the tile's words at length 4096 into its slot (as fixed_compress_kernel)
-      const int b = s_b0;
-      uint8_t* stage = smem + (size_t)st * cf_stage_bytes<T>();
-      uint8_t* work = sizeof(T) == 8 ? stage : smem + (size_t)S * cf_stage_bytes<T>();
-      uint32_t* out = a.slots + item * a.slot_words;
-      if (b <= 31) {
-        uint32_t* fT = reinterpret_cast<uint32_t*>(work);
-        uint32_t* stg = fT + kFtWords;
-        uint32_t* fp = fT + lane * kFtStride + ((1024 * q + r) >> 5);  // position 1024 q + r + 64 m: j % 32 = lane
-#pragma unroll
-        for (int m = 0; m < kCfPerThread; m++) fp[2 * m] = fl[m];
-        cf_sync();
-        if (tid < ((cnt + 31) >> 5)) cf_pack_dispatch(b, fT + tid, stg, tid * b);
-        cf_sync();
-        const int nw = (int)(((long long)cnt * b + 31) >> 5);
-        for (int w = tid; w < nw; w += kCfThreads) out[w] = stg[w + (w >> 5)];
-      } else {
-        long long* res = sizeof(T) == 8 ? reinterpret_cast<long long*>(const_cast<T*>(x))
-                                        : reinterpret_cast<long long*>(work);
-        if (qlen > 0)
-          cf_store_resid<T>(x, res, 1024 * q + r, 64, cnt, s_mode[st][0], s_t0[st][0], s_t1[st][0]);
-        cf_sync();
-        cf_words_dispatch(b, res, cnt, out, tid);
-      }
-      cf_sync();  // every compute thread is done with stage st and the work area
-    }
-    if (tid == 0) mbar_arrive(&empty[st]);
-    if (item1 < 0) return;
+  if (glen > 0 && b > 0) cg_pack_slow<T>(row, glen, 32 * tid, b, s_mode[0], s_t0[0], s_t1[0], s_c[0], s_ci[0]);
+  __syncwarp();
+  for (int l = 0; l < 32; l++) {
+    const int gl = __shfl_sync(FULL_MASK, glen, l);
+    if (gl <= 0) break;
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(stage + ((tid & ~31) + l) * cg_row_bytes<T>());
+    const int nw = (gl * b + 31) >> 5;
+    for (int w = lane; w < nw; w += 32) out[(32 * warp + l) * b + w] = q[w];
   }
 }
 
@@ -1136,26 +813,8 @@ static cudaError_t launch_fixed_compress_dt(glc_dtype dt, const FixedCompressArg
   return cudaErrorInvalidValue;
 }
 
-template <typename T, bool PACK> static cudaError_t launch_choose_t(const FixedCompressArgs& a, int num_sms, cudaStream_t s) {
-  constexpr int smem = PACK ? cf_fix_smem_bytes<T>(kCfChooseStages) : kCfChooseStages * cf_stage_bytes<T>();
-  static PerDeviceFlag attr_set;
-  const int dev = current_device();
-  cudaError_t e;
-  if (!attr_set.test(dev)) {
-    if ((e = cudaFuncSetAttribute(choose_lengths_kernel<T, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  smem)) != cudaSuccess)
-      return e;
-    attr_set.set(dev);
-  }
-  int per_sm = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, choose_lengths_kernel<T, PACK>, kCfFixCTA, smem)) !=
-      cudaSuccess)
-    return e;
-  if (per_sm < 1) per_sm = 1;
-  int64_t grid = (int64_t)per_sm * num_sms;
-  if (grid > a.nitems) grid = a.nitems;
-  if (grid < 1) grid = 1;
-  choose_lengths_kernel<T, PACK><<<(unsigned)grid, kCfFixCTA, smem, s>>>(a);
+template <typename T, bool PACK> static cudaError_t launch_choose_t(const FixedCompressArgs& a, cudaStream_t s) {
+  choose_lengths_kernel<T, PACK><<<(unsigned)a.nitems, kCgThreads, cg_stage_bytes<T>(), s>>>(a);
   return cudaGetLastError();
 }
 
@@ -1177,10 +836,10 @@ cudaError_t launch_choose_lengths(glc_dtype dt, const CfColumn* cols, const int3
     a.terr = terr;
   }
   switch (dt) {
-    case GLC_I32: return pack ? launch_choose_t<int32_t, true>(a, num_sms, s) : launch_choose_t<int32_t, false>(a, num_sms, s);
-    case GLC_I64: return pack ? launch_choose_t<int64_t, true>(a, num_sms, s) : launch_choose_t<int64_t, false>(a, num_sms, s);
-    case GLC_U64: return pack ? launch_choose_t<uint64_t, true>(a, num_sms, s) : launch_choose_t<uint64_t, false>(a, num_sms, s);
-    case GLC_U32: return pack ? launch_choose_t<uint32_t, true>(a, num_sms, s) : launch_choose_t<uint32_t, false>(a, num_sms, s);
+    case GLC_I32: return pack ? launch_choose_t<int32_t, true>(a, s) : launch_choose_t<int32_t, false>(a, s);
+    case GLC_I64: return pack ? launch_choose_t<int64_t, true>(a, s) : launch_choose_t<int64_t, false>(a, s);
+    case GLC_U64: return pack ? launch_choose_t<uint64_t, true>(a, s) : launch_choose_t<uint64_t, false>(a, s);
+    case GLC_U32: return pack ? launch_choose_t<uint32_t, true>(a, s) : launch_choose_t<uint32_t, false>(a, s);
   }
   return cudaErrorInvalidValue;
 }
