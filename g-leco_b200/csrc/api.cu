@@ -291,6 +291,7 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
   // the column synchronises the device first, so a free behaves as cudaFree does.
   c->pool = ctx->pool;
   c->sync_free = true;
+  int32_t* unit_first = nullptr;  // V6: the first partition of each unit of kFitShort values
   if (mode == GLC_PART_FIXED) {
     c->P = (n + fixed_len - 1) / fixed_len;
     c->fixed_len = fixed_len;
@@ -299,6 +300,7 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
     PartOut po;
     po.column = c;
     po.alloc = alloc_meta;
+    po.unit_first = &unit_first;
     cudaError_t e = launch_partition_v6(ctx, dtype, dev_values, n, kV6Base, po, s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "GPU partitioner (V6)");
   } else {
@@ -342,15 +344,16 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
   }
   cudaError_t e = cudaSuccess;
   if (mode != GLC_PART_VARIABLE) {
-    // V6 partitions hold at most 4 * kV6Base values: one CTA fits each
-    static_assert(4 * kV6Base <= kFitShort, "V6 partitions are short");
+    // V6 partitions hold 1, 2, 4 or 8 times 1024 values, in blocks of 16,384: none crosses a unit
+    static_assert(4 * kV6Base == kFitShort, "a unit is the largest V6 partition");
     const bool brief = mode == GLC_PART_VARIABLE_V6;
     const size_t sb = brief ? fit_short_scratch_bytes(c->P) : fit_scratch_bytes(nullptr, n, c->P);
     void* scratch = nullptr;
     CK(pool_alloc(ctx, &scratch, sb, s), "compress: scratch allocation");
-    e = brief ? launch_fit_short(dtype, dev_values, c, scratch, ctx->d_stats, s)
+    e = brief ? launch_fit_short(dtype, dev_values, c, unit_first, scratch, ctx->d_stats, s)
               : launch_fit(dtype, dev_values, c, scratch, sb, ctx->d_stats, s);
     cudaFreeAsync(scratch, s);
+    if (unit_first) cudaFreeAsync(unit_first, s);
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -524,24 +524,27 @@ cudaError_t launch_fit(glc_dtype dt, const void* values, glc_column* c, void* sc
 }
 
 // ---------------------------------------------------------------------------------------
-// Partitions of at most kFitShort values: a CTA fits one, from its exact sums to its width, in one
-// launch.  The values are read twice, the second time from L1 or L2 (a partition is at most 64 KB);
-// no chunk tables, and so no scans before the fit.  The residuals are 64-bit integers against a
-// prediction rounded in FP64 (glc_group.cuh).  30M uint32 in V6 partitions: 11 launches and their
-// gaps, 170 us, become one launch of 77 us.  Bound by the latency of a CTA (two barriers and the solve
-// between its two short passes), with eight CTAs per SM.
+// Partitions that lie inside units of kFitShort = 8192 values: a CTA fits the 1 to 8 partitions of a
+// unit, from their exact sums to their widths, a group of its warps each, in one launch.  The values
+// are read twice, the second time from L1 or L2 (a unit is at most 64 KB); no chunk tables, and so no
+// scans before the fit.  The residuals are 64-bit integers against a prediction rounded in FP64
+// (glc_group.cuh).  30M uint32 in V6 partitions: 11 launches and their gaps, 170 us, became one launch
+// of 77 us with a CTA of 256 threads per partition, whose barriers and solve bound it where a
+// partition is 1024 values, and 44 us with a CTA per unit.
 // ---------------------------------------------------------------------------------------
 constexpr int kFsThreads = 256;
 constexpr int kFsWarps = kFsThreads / 32;
 
-// f(value, index) for this thread's values of a partition, 16 bytes at a time where they are aligned.
-template <typename T, typename F> __device__ __forceinline__ void fs_each(const T* __restrict__ v, int len, F f) {
+// f(value, index) for the values of a partition that thread `t` of a group of `threads` takes, 16 bytes
+// at a time where they are aligned.
+template <typename T, typename F>
+__device__ __forceinline__ void fs_each(const T* __restrict__ v, int len, int t, int threads, F f) {
   constexpr int N = CgVec<T>::N;
   int done = 0;
   if ((reinterpret_cast<uintptr_t>(v) & 15) == 0) {
     done = len / N * N;
 #pragma unroll 4
-    for (int j = threadIdx.x * N; j < done; j += kFsThreads * N) {
+    for (int j = t * N; j < done; j += threads * N) {
       const uint4 u = __ldg(reinterpret_cast<const uint4*>(v + j));
       T y[N];
       memcpy(y, &u, 16);
@@ -550,13 +553,13 @@ template <typename T, typename F> __device__ __forceinline__ void fs_each(const 
     }
   }
 #pragma unroll 4
-  for (int j = done + threadIdx.x; j < len; j += kFsThreads) f(__ldg(v + j), j);
+  for (int j = done + t; j < len; j += threads) f(__ldg(v + j), j);
 }
 
 // The largest |residual| of this thread's values: in 32 bits, or again in 64 where one does not fit.
 template <typename T>
-__device__ __forceinline__ unsigned long long fs_max(const T* __restrict__ v, int len, int mode, double t0, double t1,
-                                                     double c, long long ci) {
+__device__ __forceinline__ unsigned long long fs_max(const T* __restrict__ v, int len, int t, int threads, int mode,
+                                                     double t0, double t1, double c, long long ci) {
   int mn = 0, mx = 0;
   uint32_t wide = 0u;
   auto one = [&](T y, int j, int m) {
@@ -567,14 +570,14 @@ __device__ __forceinline__ unsigned long long fs_max(const T* __restrict__ v, in
     mx = max(mx, lo);
   };
   // (the mode a constant in each loop)
-  if (mode == CF_NONNEG) fs_each<T>(v, len, [&](T y, int j) { one(y, j, CF_NONNEG); });
-  else if (TypeTraits<T>::is_signed && mode == CF_NONPOS) fs_each<T>(v, len, [&](T y, int j) { one(y, j, CF_NONPOS); });
-  else if (sizeof(T) == 8 && mode == CF_OFFSET) fs_each<T>(v, len, [&](T y, int j) { one(y, j, CF_OFFSET); });
+  if (mode == CF_NONNEG) fs_each<T>(v, len, t, threads, [&](T y, int j) { one(y, j, CF_NONNEG); });
+  else if (TypeTraits<T>::is_signed && mode == CF_NONPOS) fs_each<T>(v, len, t, threads, [&](T y, int j) { one(y, j, CF_NONPOS); });
+  else if (sizeof(T) == 8 && mode == CF_OFFSET) fs_each<T>(v, len, t, threads, [&](T y, int j) { one(y, j, CF_OFFSET); });
   else wide = 1u;
   unsigned long long m = max((uint32_t)mx, 0u - (uint32_t)mn);
   if (wide) {
     m = 0;
-    fs_each<T>(v, len, [&](T y, int j) {
+    fs_each<T>(v, len, t, threads, [&](T y, int j) {
       const unsigned long long ad = (unsigned long long)abs_ref(cg_field<T>(y, (double)j, mode, t0, t1, c, ci));
       m = ad > m ? ad : m;
     });
@@ -583,61 +586,79 @@ __device__ __forceinline__ unsigned long long fs_max(const T* __restrict__ v, in
 }
 
 template <typename T> __global__ void __launch_bounds__(kFsThreads)
-fit_short_kernel(const T* __restrict__ values, const int32_t* __restrict__ starts, const int32_t* __restrict__ ends,
-                 int64_t P, int32_t* __restrict__ types, double* __restrict__ params, int32_t* __restrict__ bits,
-                 int64_t* __restrict__ err, int64_t* __restrict__ widths, unsigned long long* __restrict__ stats) {
+fit_short_kernel(const T* __restrict__ values, const int32_t* __restrict__ unit_first, const int32_t* __restrict__ starts,
+                 const int32_t* __restrict__ ends, int64_t P, int32_t* __restrict__ types, double* __restrict__ params,
+                 int32_t* __restrict__ bits, int64_t* __restrict__ err, int64_t* __restrict__ widths,
+                 unsigned long long* __restrict__ stats) {
   __shared__ long long s_acc[kFsWarps][4];
+  __shared__ int s_over[kFsWarps];
   __shared__ unsigned long long s_mx[kFsWarps];
-  __shared__ double s_line[3];
-  __shared__ long long s_ci;
-  __shared__ int s_mode;
+  __shared__ double s_line[kFsWarps][3];
+  __shared__ long long s_ci[kFsWarps];
+  __shared__ int s_mode[kFsWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t p = blockIdx.x;
-  const int s = starts[p], len = ends[p] - s;
+  const int p0 = unit_first[blockIdx.x], np = unit_first[blockIdx.x + 1] - p0;
+  if (np > kFsWarps) {  // not partitions for this kernel (of fewer than 1024 values each)
+    if (tid == 0) atomicExch(stats + 2, (unsigned long long)DEVERR_BOUNDS);
+    return;
+  }
+  const int per = np <= 1 ? 8 : np <= 2 ? 4 : np <= 4 ? 2 : 1;  // warps of a partition: [w0, w0 + per)
+  const int g = warp / per, w0 = g * per, t = tid - 32 * w0, threads = 32 * per;
+  const bool have = g < np;
+  const int64_t p = p0 + g;
+  const int s = have ? starts[p] : 0, len = have ? ends[p] - s : 0;
   const T* v = values + s;
   HalfSums<T> hs;
   bool over = false;
-  fs_each<T>(v, len, [&](T y, int j) {
+  fs_each<T>(v, len, t, threads, [&](T y, int j) {
     hs.add(y, j);
     over |= overflows_double<T>(y);
   });
   // (32 values a thread, j < 2^13, 32-bit halves: partials below 2^50)
   const long long c0 = seg_sum48((long long)hs.s_lo, 32), c1 = sizeof(T) == 8 ? seg_sum48((long long)hs.s_hi, 32) : 0;
   const long long c2 = seg_sum48((long long)hs.x_lo, 32), c3 = sizeof(T) == 8 ? seg_sum48((long long)hs.x_hi, 32) : 0;
+  over = __any_sync(FULL_MASK, over);
   if (lane == 0) {
     s_acc[warp][0] = c0;
     s_acc[warp][1] = c1;
     s_acc[warp][2] = c2;
     s_acc[warp][3] = c3;
+    s_over[warp] = over;
   }
-  over = __syncthreads_or(over);
-  if (tid == 0) {
+  __syncthreads();
+  if (have && t == 0) {
     long long a[4] = {0, 0, 0, 0};
-    for (int w = 0; w < kFsWarps; w++)
+    int ov = 0;
+    for (int w = w0; w < w0 + per; w++) {
       for (int k = 0; k < 4; k++) a[k] += s_acc[w][k];
+      ov |= s_over[w];
+    }
     double t0 = 0.0, t1 = 0.0, c = 0.0;
     long long ci = 0;
     int mode = CF_DIRECT;
-    if (!over) {
+    if (!ov) {
       solve_line(len, (i128)a[0] + (i128)a[1] * ((i128)1 << 32), (i128)a[2] + (i128)a[3] * ((i128)1 << 32), t0, t1);
       mode = cf_mode<T>(t0, t1, len, true, c, ci);  // (cg_field's differences need no bound on the values)
     }
-    s_line[0] = t0;
-    s_line[1] = t1;
-    s_line[2] = c;
-    s_ci = ci;
-    s_mode = mode;
+    s_line[g][0] = t0;
+    s_line[g][1] = t1;
+    s_line[g][2] = c;
+    s_ci[g] = ci;
+    s_mode[g] = mode;
   }
   __syncthreads();
-  unsigned long long m = over ? 0ull : seg_max_u64(fs_max<T>(v, len, s_mode, s_line[0], s_line[1], s_line[2], s_ci), 32);
+  const int mode = have ? s_mode[g] : CF_DIRECT;
+  unsigned long long m = 0;
+  if (mode != CF_DIRECT) m = fs_max<T>(v, len, t, threads, mode, s_line[g][0], s_line[g][1], s_line[g][2], s_ci[g]);
+  m = seg_max_u64(m, 32);
   if (lane == 0) s_mx[warp] = m;
   __syncthreads();
-  if (tid == 0) {
-    for (int w = 0; w < kFsWarps; w++) m = s_mx[w] > m ? s_mx[w] : m;
-    const int b = over ? (int)sizeof(T) * 8 : bits_for((long long)m);
-    types[p] = over ? MODEL_DIRECT_COPY : MODEL_LINEAR;
-    params[4 * p] = s_line[0];
-    params[4 * p + 1] = s_line[1];
+  if (have && t == 0) {
+    for (int w = w0; w < w0 + per; w++) m = s_mx[w] > m ? s_mx[w] : m;
+    const int b = mode == CF_DIRECT ? (int)sizeof(T) * 8 : bits_for((long long)m);
+    types[p] = mode == CF_DIRECT ? MODEL_DIRECT_COPY : MODEL_LINEAR;
+    params[4 * p] = s_line[g][0];
+    params[4 * p + 1] = s_line[g][1];
     params[4 * p + 2] = 0.0;
     params[4 * p + 3] = 0.0;
     bits[p] = b;
@@ -652,17 +673,18 @@ fit_short_kernel(const T* __restrict__ values, const int32_t* __restrict__ start
 
 size_t fit_short_scratch_bytes(int64_t P) { return sizeof(int64_t) * (size_t)(P + scan_num_tiles(P) + 4); }
 
-cudaError_t launch_fit_short(glc_dtype dt, const void* values, glc_column* c, void* scratch, int64_t* d_stats, cudaStream_t s) {
+cudaError_t launch_fit_short(glc_dtype dt, const void* values, glc_column* c, const int32_t* unit_first, void* scratch,
+                             int64_t* d_stats, cudaStream_t s) {
   const int64_t P = c->P;
   int64_t* widths = (int64_t*)scratch;
   int64_t* tmp = widths + ((P + 3) & ~3ll);
   cudaError_t e = cudaMemsetAsync(d_stats, 0, 4 * sizeof(int64_t), s);
   if (e != cudaSuccess) return e;
-  const unsigned g = (unsigned)P;
+  const unsigned g = (unsigned)((c->n + kFitShort - 1) / kFitShort);
   unsigned long long* st = (unsigned long long*)d_stats;
 #define GLC_FIT_SHORT(T)                                                                                              \
-  fit_short_kernel<T><<<g, kFsThreads, 0, s>>>((const T*)values, c->d_start, c->d_end, P, c->d_types, c->d_params, \
-                                               c->d_bits, c->d_err, widths, st)
+  fit_short_kernel<T><<<g, kFsThreads, 0, s>>>((const T*)values, unit_first, c->d_start, c->d_end, P, c->d_types,   \
+                                               c->d_params, c->d_bits, c->d_err, widths, st)
   switch (dt) {
     case GLC_I32: GLC_FIT_SHORT(int32_t); break;
     case GLC_I64: GLC_FIT_SHORT(int64_t); break;

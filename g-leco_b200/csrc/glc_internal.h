@@ -202,11 +202,12 @@ size_t fit_scratch_bytes(const int32_t* unused, int64_t n, int64_t P);
 // Fits every partition of c (starts/ends set); d_stats[0] = total bits, d_stats[1] = max bits.
 cudaError_t launch_fit(glc_dtype dt, const void* values, glc_column* c, void* scratch, size_t scratch_bytes,
                        int64_t* d_stats, cudaStream_t s);
-// The same for partitions of at most kFitShort values each (scratch:
-// fit_short_scratch_bytes).
+// The same for 1 to 8 partitions inside each unit of kFitShort values, none across two: unit_first[u] =
+// the first partition of unit u (units + 1 entries); scratch: fit_short_scratch_bytes.
 constexpr int kFitShort = 8192;
 size_t fit_short_scratch_bytes(int64_t P);
-cudaError_t launch_fit_short(glc_dtype dt, const void* values, glc_column* c, void* scratch, int64_t* d_stats, cudaStream_t s);
+cudaError_t launch_fit_short(glc_dtype dt, const void* values, glc_column* c, const int32_t* unit_first, void* scratch,
+                             int64_t* d_stats, cudaStream_t s);
 cudaError_t launch_desc_and_tiles(glc_column* c, cudaStream_t s);
 // compress_fixed.cu: one-pass compression of fixed partitions of L values, L a divisor of 4096 and >= 256
 // One column of a launch (its arrays are the column's own, or its slices of a batch's arrays).
@@ -395,6 +396,7 @@ struct PartOut {
   int32_t** starts = nullptr;
   int32_t** ends = nullptr;
   int64_t* P = nullptr;
+  int32_t** unit_first = nullptr;  // V6 with a column: launch_fit_short's, from pool_alloc
 };
 cudaError_t launch_partition_variable(glc_ctx* ctx, glc_dtype dt, const void* values, int64_t n, const PartOut& out,
                                       cudaStream_t s, std::string* err);

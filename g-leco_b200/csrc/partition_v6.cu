@@ -191,7 +191,7 @@ v6_select_kernel(const float* __restrict__ var, int64_t nb, int64_t n, int64_t b
 }
 
 __global__ void v6_emit_kernel(int64_t nb, const V6Plan* __restrict__ plan, int64_t n, int64_t base, int64_t P,
-                               int32_t* __restrict__ starts, int32_t* __restrict__ ends) {
+                               int32_t* __restrict__ starts, int32_t* __restrict__ ends, int32_t* __restrict__ unit_first) {
   const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= P) return;
   int64_t e[3];
@@ -204,6 +204,10 @@ __global__ void v6_emit_kernel(int64_t nb, const V6Plan* __restrict__ plan, int6
   const int64_t s = 8 * base * i + (o - v6_before(i, e)) * size;
   starts[o] = (int32_t)s;
   ends[o] = (int32_t)(s + size < end ? s + size : end);
+  if (unit_first) {  // (a block is a whole number of units, and every size divides it)
+    if (s % kFitShort == 0) unit_first[s / kFitShort] = (int32_t)o;
+    if (o == P - 1) unit_first[(n + kFitShort - 1) / kFitShort] = (int32_t)P;
+  }
 }
 
 template <typename T>
@@ -227,6 +231,7 @@ cudaError_t v6_typed(glc_ctx* ctx, const T* values, int64_t n, int64_t base, con
       if ((e = out.alloc(out.column, s)) == cudaSuccess) {
         starts = out.column->d_start;
         ends = out.column->d_end;
+        if (out.unit_first) e = pool_alloc(ctx, out.unit_first, 4 * (size_t)((n + kFitShort - 1) / kFitShort + 1), s);
       }
     } else {
       *out.P = P;
@@ -236,7 +241,8 @@ cudaError_t v6_typed(glc_ctx* ctx, const T* values, int64_t n, int64_t base, con
       }
     }
     if (e == cudaSuccess) {
-      v6_emit_kernel<<<(unsigned)((P + 255) / 256), 256, 0, s>>>(nb, plan, n, base, P, starts, ends);
+      v6_emit_kernel<<<(unsigned)((P + 255) / 256), 256, 0, s>>>(nb, plan, n, base, P, starts, ends,
+                                                                 out.unit_first ? *out.unit_first : nullptr);
       e = cudaGetLastError();
     }
   }
