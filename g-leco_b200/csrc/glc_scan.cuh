@@ -5,7 +5,7 @@
 // are usually that few, and each launch of a chain costs 3 to 5 us, its gap included: 13,725
 // widths took 14 us in three launches, 5 us in one).  More than that, where one SM's loads would
 // bound it, or wider items:
-// three launches: each 1024-thread CTA scans a tile of 4096 items and writes the tile total;
+// three launches: each 1024-thread CTA scans a tile of 4096 items (1024 of 32 bytes) and writes its total;
 // one CTA scans the tile totals (looping with a carry, so any count works); each CTA then adds
 // its tile's base.  The bit offsets of the bitstream are this scan over len * bits
 // (the reference computes each offset with an O(P) loop per partition,
@@ -62,22 +62,49 @@ template <typename V> __device__ V block_exclusive_scan(V x, V* total, V* s_warp
   return base + excl;
 }
 
+// One item, in one access where it is 32 bytes (and its array 32-byte aligned, as 32-byte items' are here).
+template <typename V> __device__ __forceinline__ V scan_load(const V* p) {
+  if constexpr (sizeof(V) == 32) {
+    const Bytes32 r = load32(p);
+    V v;
+    memcpy(&v, &r, 32);
+    return v;
+  } else {
+    return *p;
+  }
+}
+template <typename V> __device__ __forceinline__ void scan_store(V* p, const V& v) {
+  if constexpr (sizeof(V) == 32) {
+    Bytes32 r;
+    memcpy(&r, &v, 32);
+    store32(p, r);
+  } else {
+    *p = v;
+  }
+}
+
+// Items per thread of a tile: four of 8 bytes, one of 32 (a column of 3M values has 23,439 block sums of
+// 32 bytes, which six tiles of 4096 left to six SMs).
+template <typename V> __host__ __device__ constexpr int scan_items() { return sizeof(V) == 32 ? 1 : kScanItems; }
+template <typename V> __host__ __device__ constexpr int scan_tile() { return kScanThreads * scan_items<V>(); }
+
 template <typename V> __global__ void __launch_bounds__(kScanThreads)
 scan_tiles_kernel(const V* __restrict__ in, V* __restrict__ out, int64_t count, V* __restrict__ tile_totals) {
   __shared__ V s_warp[32];
-  const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
-  V items[kScanItems];
+  constexpr int kItems = scan_items<V>();
+  const int64_t base = (int64_t)blockIdx.x * scan_tile<V>() + (int64_t)threadIdx.x * kItems;
+  V items[kItems];
   V sum = V();
 #pragma unroll
-  for (int k = 0; k < kScanItems; k++) {
-    items[k] = (base + k < count) ? in[base + k] : V();
+  for (int k = 0; k < kItems; k++) {
+    items[k] = (base + k < count) ? scan_load(in + base + k) : V();
     sum = sum + items[k];
   }
   V total;
   V ex = block_exclusive_scan(sum, &total, s_warp);
 #pragma unroll
-  for (int k = 0; k < kScanItems; k++) {
-    if (base + k < count) out[base + k] = ex;
+  for (int k = 0; k < kItems; k++) {
+    if (base + k < count) scan_store(out + base + k, ex);
     ex = ex + items[k];
   }
   if (threadIdx.x == 0) tile_totals[blockIdx.x] = total;
@@ -116,11 +143,12 @@ scan_totals_kernel(V* __restrict__ totals, int64_t ntiles, V* __restrict__ grand
 
 template <typename V> __global__ void __launch_bounds__(kScanThreads)
 scan_add_kernel(V* __restrict__ out, int64_t count, const V* __restrict__ tile_bases) {
+  constexpr int kItems = scan_items<V>();
   const V b = tile_bases[blockIdx.x];
-  const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
+  const int64_t base = (int64_t)blockIdx.x * scan_tile<V>() + (int64_t)threadIdx.x * kItems;
 #pragma unroll
-  for (int k = 0; k < kScanItems; k++)
-    if (base + k < count) out[base + k] = out[base + k] + b;
+  for (int k = 0; k < kItems; k++)
+    if (base + k < count) scan_store(out + base + k, scan_load(out + base + k) + b);
 }
 
 // The whole scan in one CTA: up to four chunks of 4 items per thread, all of them loaded before the
@@ -202,7 +230,7 @@ scan_one_kernel(const V* in, V* out, int count, V* grand_total) {
   if (threadIdx.x == 0 && grand_total) *grand_total = before;
 }
 
-inline int64_t scan_num_tiles(int64_t count) { return (count + kScanTile - 1) / kScanTile; }
+template <typename V = int64_t> int64_t scan_num_tiles(int64_t count) { return (count + scan_tile<V>() - 1) / scan_tile<V>(); }
 
 // Scratch: one V per tile.  in and out may alias.  *grand_total (device) may be null.
 template <typename V>
@@ -219,7 +247,7 @@ cudaError_t exclusive_scan(const V* in, V* out, int64_t count, V* grand_total, V
       return cudaGetLastError();
     }
   }
-  int64_t nt = scan_num_tiles(count);
+  int64_t nt = scan_num_tiles<V>(count);
   scan_tiles_kernel<V><<<(unsigned)nt, kScanThreads, 0, s>>>(in, out, count, tile_scratch);
   scan_totals_kernel<V><<<1, kScanThreads, 0, s>>>(tile_scratch, nt, grand_total);
   scan_add_kernel<V><<<(unsigned)nt, kScanThreads, 0, s>>>(out, count, tile_scratch);

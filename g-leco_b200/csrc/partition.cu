@@ -1078,7 +1078,7 @@ static cudaError_t partition_typed(glc_ctx* ctx, const T* v, int64_t n, const Pa
                        // [4] partitions left, [5] list, [6] DEVERR_*
   unsigned* counters;  // right after dsc: cleared together
   split.want(&pre, nb + 1);
-  split.want(&ptiles, scan_num_tiles(nb) + 1);
+  split.want(&ptiles, scan_num_tiles<SumPair>(nb) + 1);
   split.want(&nb_next, nb);
   split.want(&nb_err, nb);
   split.want(&ovf, sizeof(T) == 8 && !TypeTraits<T>::is_signed ? nb : 1);
