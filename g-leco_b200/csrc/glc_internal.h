@@ -372,6 +372,7 @@ glc_status attach_column(glc_ctx* ctx, glc_dtype dtype, const void* blob, uint64
 struct RAColumn {
   const PartDesc* desc;
   const int32_t* starts;
+  const TileInfo* tiles;
   const uint32_t* words;
   int64_t P, n;
   int32_t fixed_len;  // > 0: partition = pos / fixed_len

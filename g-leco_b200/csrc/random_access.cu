@@ -8,9 +8,9 @@
 // Per lookup: the position, one 32-byte partition descriptor (theta0, theta1, bit offset,
 // start, bits|type -- a single DRAM sector instead of the reference's four arrays), and the
 // words that hold the field (or the 8-byte pre-unpacked residual).  Partition lookup is
-// pos / L for fixed partitions; for variable partitions a sample of every k-th start lives in
-// shared memory, a binary search there narrows the range to k partitions, and a short search
-// over the (L2-resident) start array finishes it.  Each thread carries several independent
+// pos / L for fixed partitions; for variable partitions the decode table gives the first and last
+// partition of the position's 4096-value tile (one 8-byte load), and a search between them, rarely of
+// more than two steps, finishes it.  Each thread carries several independent
 // lookups through the load stages so their DRAM latencies overlap.
 // Positions outside [0, n) yield 0, as the reference's variable-partition kernels do; the
 // fixed variants use the same rule here instead of reading past the metadata.
@@ -22,11 +22,11 @@
 namespace glc {
 
 constexpr int kRAThreads = 256;
-constexpr int kRASample = 4096;
 
 struct RAArgs {
   const PartDesc* desc;
   const int32_t* starts;
+  const TileInfo* tiles;
   const uint32_t* words;
   const int64_t* plain;
   int64_t P, n;
@@ -35,9 +35,18 @@ struct RAArgs {
   void* out;
   int32_t fixed_len;
   int32_t fixed_shift;   // >= 0 when fixed_len is a power of two
-  int32_t sample_stride;
-  int32_t nsample;
 };
+
+// The partition of a position in a column of variable partitions.
+__device__ __forceinline__ int32_t find_partition(const TileInfo* __restrict__ tiles, const int32_t* __restrict__ starts, int32_t pos) {
+  const int2 t = __ldg(reinterpret_cast<const int2*>(tiles + pos / kDecodeTile) + 1);  // p_first, p_last
+  int32_t lo = t.x, hi = t.y;
+  while (lo < hi) {
+    const int32_t mid = (lo + hi + 1) >> 1;
+    if (__ldg(starts + mid) <= pos) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
 
 // The words holding a field come from one aligned 16-byte load (one sector, one request); a
 // second load is needed only when the field continues past that granule.  The word array is
@@ -76,11 +85,6 @@ __device__ __forceinline__ PartDesc load_desc(const PartDesc* __restrict__ d) {
 // the register budget is sized for.
 template <typename T, bool PLAIN, int MODE, int kRAQueries, int MINB>
 __global__ void __launch_bounds__(kRAThreads, MINB) random_access_kernel(RAArgs a) {
-  __shared__ int32_t s_sample[MODE == 2 ? kRASample : 1];  // fixed modes leave L1 to descriptors
-  if (MODE == 2) {
-    for (int k = threadIdx.x; k < a.nsample; k += kRAThreads) s_sample[k] = a.starts[(int64_t)k * a.sample_stride];
-    __syncthreads();
-  }
   T* out = reinterpret_cast<T*>(a.out);
   const int64_t chunk = (int64_t)kRAThreads * kRAQueries;
   const int64_t stride = (int64_t)gridDim.x * chunk;
@@ -123,19 +127,7 @@ __global__ void __launch_bounds__(kRAThreads, MINB) random_access_kernel(RAArgs 
         p[k] = pos[k] / a.fixed_len;
         p[k] = p[k] < last_p ? p[k] : last_p;
       } else {
-        int lo = 0, hi = a.nsample - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (s_sample[mid] <= pos[k]) lo = mid; else hi = mid - 1;
-        }
-        int32_t plo = lo * a.sample_stride;
-        int32_t phi = plo + a.sample_stride - 1;
-        if (phi > last_p) phi = last_p;
-        while (plo < phi) {
-          const int32_t mid = (plo + phi + 1) >> 1;
-          if (__ldg(a.starts + mid) <= pos[k]) plo = mid; else phi = mid - 1;
-        }
-        p[k] = plo;
+        p[k] = find_partition(a.tiles, a.starts, pos[k]);
       }
     }
     double2 th[kRAQueries];  // theta0, theta1
@@ -177,12 +169,13 @@ static cudaError_t ra_shape(glc_ctx* ctx, const RAArgs& a, int mode, cudaStream_
                                 : random_access_kernel<T, PLAIN, 2, QPT, MINB>;
   int per_sm = 0;
   cudaError_t e;
-  if (mode != 2) {  // no shared memory in the fixed modes: prefer the largest L1 for descriptors
+  {  // no shared memory: prefer the largest L1 for descriptors
     static PerDeviceFlag carveout_set;  // per instantiation and device
     const int dev = current_device();
     if (!carveout_set.test(dev)) {
       cudaFuncSetAttribute(random_access_kernel<T, PLAIN, 0, QPT, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
       cudaFuncSetAttribute(random_access_kernel<T, PLAIN, 1, QPT, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
+      cudaFuncSetAttribute(random_access_kernel<T, PLAIN, 2, QPT, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
       carveout_set.set(dev);
     }
   }
@@ -232,6 +225,7 @@ cudaError_t launch_random_access_shape(glc_ctx* ctx, const glc_column* c, int pl
   RAArgs a;
   a.desc = c->d_desc;
   a.starts = c->d_start;
+  a.tiles = c->d_tiles;
   a.words = c->d_words;
   a.plain = c->d_plain;
   a.P = c->P;
@@ -253,9 +247,6 @@ cudaError_t launch_random_access_shape(glc_ctx* ctx, const glc_column* c, int pl
       a.fixed_shift = __builtin_ctz((unsigned)fixed_len);
     }
   }
-  a.sample_stride = (int32_t)((c->P + kRASample - 1) / kRASample);
-  if (a.sample_stride < 1) a.sample_stride = 1;
-  a.nsample = (int32_t)((c->P + a.sample_stride - 1) / a.sample_stride);
   switch (c->dtype) {
     case GLC_I32: return plain_src ? ra_typed<int32_t, true>(ctx, a, mode, shape, s) : ra_typed<int32_t, false>(ctx, a, mode, shape, s);
     case GLC_I64: return plain_src ? ra_typed<int64_t, true>(ctx, a, mode, shape, s) : ra_typed<int64_t, false>(ctx, a, mode, shape, s);
@@ -279,12 +270,7 @@ __device__ __forceinline__ void lookup_one(const RAColumn& c, int64_t pos, uint8
       p = pos / c.fixed_len;
       p = p < c.P ? p : c.P - 1;
     } else {
-      int64_t lo = 0, hi = c.P - 1;
-      while (lo < hi) {
-        const int64_t mid = (lo + hi + 1) >> 1;
-        if ((int64_t)__ldg(c.starts + mid) <= pos) lo = mid; else hi = mid - 1;
-      }
-      p = lo;
+      p = find_partition(c.tiles, c.starts, (int32_t)pos);
     }
     const PartDesc d = load_desc(c.desc + p);
     const int bits = d.bits_type & 0xff, type = d.bits_type >> 8;

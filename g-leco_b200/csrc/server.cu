@@ -466,6 +466,7 @@ void fill_views(SrvColumn& sc) {
   const glc_column* c = sc.col;
   sc.ra.desc = c->d_desc;
   sc.ra.starts = c->d_start;
+  sc.ra.tiles = c->d_tiles;
   sc.ra.words = c->d_words;
   sc.ra.P = c->P;
   sc.ra.n = c->n;
