@@ -349,7 +349,11 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
     const bool brief = mode == GLC_PART_VARIABLE_V6;
     const size_t sb = brief ? fit_short_scratch_bytes(c->P) : fit_scratch_bytes(nullptr, n, c->P);
     void* scratch = nullptr;
-    CK(pool_alloc(ctx, &scratch, sb, s), "compress: scratch allocation");
+    e = pool_alloc(ctx, &scratch, sb, s);
+    if (e != cudaSuccess) {
+      if (unit_first) cudaFreeAsync(unit_first, s);
+      return cuda_fail(ctx, e, "compress: scratch allocation");
+    }
     e = brief ? launch_fit_short(dtype, dev_values, c, unit_first, scratch, ctx->d_stats, s)
               : launch_fit(dtype, dev_values, c, scratch, sb, ctx->d_stats, s);
     cudaFreeAsync(scratch, s);
