@@ -746,6 +746,7 @@ struct MergeArgs {
 };
 constexpr int kMaxMergeRounds = 64;
 constexpr int kMergeThreads = 512;
+constexpr int kMergeShort = 16384;    // partitions of a list that every CTA counts for itself
 constexpr int kMergeUnitMost = 4096;  // values of a pair that one warp scans, at most
 // counters: [0] grid barrier, then per round: pairs taken, queue length, pairs rejected
 constexpr int kMergeCounters = 4 + 4 * kMaxMergeRounds;
@@ -780,7 +781,8 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned& arrived, i
 // their further units in a queue that all warps empty together after the others.
 //
 // 200M piecewise uint64 values: 3343 us of error passes and ~450 us of bookkeeping launches -> 1320 us;
-// 3M int64 timestamps: 57 + ~170 -> 120 us.  Bound by the values read (about four passes at 5 TB/s) and,
+// 3M int64 timestamps: 57 + ~170 -> 86 us (95 with a third barrier per round for the counts of a short
+// list).  Bound by the values read (about four passes at 5 TB/s) and,
 // on short columns, by the barriers.  Units of 32,768 values measured 1829 us (the last warps of a
 // round scan alone), 8192: 1420, 4096: 1346; 1024 threads with eight loads in flight per lane 1925
 // (64 registers: spills).
@@ -905,23 +907,33 @@ merge_kernel(const T* __restrict__ v, RangeSums rs, MergeArgs a) {
     // ---- compact: a CTA takes a stretch of the list ----
     const int seg = (m + gridDim.x - 1) / gridDim.x, k0 = min(m, (int)blockIdx.x * seg), k1 = min(m, k0 + seg);
     auto merges = [&](int k) { return k >= odd && ((k + round) & 1) == 0 && k + 1 < m && a.selected[k]; };
-    int heads = 0;
-    for (int k = k0 + threadIdx.x; k < k1; k += kMergeThreads) heads += !merges(k - 1);
-    heads = __reduce_add_sync(FULL_MASK, heads);
-    if (lane == 0) s_scan[warp] = heads;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int t = 0;
-      for (int w = 0; w < kMergeThreads / 32; w++) t += s_scan[w];
-      a.cta_heads[blockIdx.x] = t;
-    }
-    if (!grid_barrier(a.counters, arrived, a.out + 2)) return;
-    // heads before this CTA, and all of them
+    // heads before this CTA, and all of them: counted by every CTA for itself where the list is short
+    // (a barrier costs more than m / 512 loads per thread), else by the CTAs' own counts
     int before = 0, all = 0;
-    for (int c = threadIdx.x; c < (int)gridDim.x; c += kMergeThreads) {
-      const int h = *(volatile int32_t*)(a.cta_heads + c);
-      all += h;
-      if (c < (int)blockIdx.x) before += h;
+    if (m <= kMergeShort) {
+#pragma unroll 4
+      for (int k = threadIdx.x; k < m; k += kMergeThreads) {
+        const int h = !merges(k - 1);
+        all += h;
+        before += k < k0 ? h : 0;
+      }
+    } else {
+      int heads = 0;
+      for (int k = k0 + threadIdx.x; k < k1; k += kMergeThreads) heads += !merges(k - 1);
+      heads = __reduce_add_sync(FULL_MASK, heads);
+      if (lane == 0) s_scan[warp] = heads;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        int t = 0;
+        for (int w = 0; w < kMergeThreads / 32; w++) t += s_scan[w];
+        a.cta_heads[blockIdx.x] = t;
+      }
+      if (!grid_barrier(a.counters, arrived, a.out + 2)) return;
+      for (int c = threadIdx.x; c < (int)gridDim.x; c += kMergeThreads) {
+        const int h = *(volatile int32_t*)(a.cta_heads + c);
+        all += h;
+        if (c < (int)blockIdx.x) before += h;
+      }
     }
     before = __reduce_add_sync(FULL_MASK, before);
     all = __reduce_add_sync(FULL_MASK, all);
