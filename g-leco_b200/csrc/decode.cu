@@ -13,7 +13,8 @@
 // bit and first/last partition; no per-value search is needed.
 //
 // CTA = 1 producer warp + 8 consumer warps, persistent (grid = resident CTAs on all SMs):
-//   producer (one lane): claims the next tile from a global counter (work stealing), waits until
+//   producer (one lane): claims the next tile from a global counter (work stealing; its first tile is
+//     its CTA's number), waits until
 //     the consumers released the ring stage, then issues 1-D TMA bulk copies (cp.async.bulk,
 //     non-multicast) of the tile's packed words (or pre-unpacked residuals) AND of the tile's
 //     32-byte partition descriptors into that stage, completing on the stage's "full" mbarrier.
@@ -326,7 +327,9 @@ __global__ void __launch_bounds__(CW * 32 + 32) decode_kernel(DecodeArgs a) {
         break;
       }
       StageInfo si;
-      si.tile = a.counter ? a.t_begin + atomicAdd(a.counter, 1) : (k == 0 ? a.t_begin + (int64_t)blockIdx.x : a.t_end);
+      // the first tile by the CTA's number (the grid has no more CTAs than tiles), further ones claimed
+      si.tile = k == 0 ? a.t_begin + (int64_t)blockIdx.x
+                       : a.counter ? a.t_begin + (int64_t)gridDim.x + atomicAdd(a.counter, 1) : a.t_end;
       if (si.tile >= a.t_end) {
         s_info[s] = si;
         mbar_arrive(&full[s]);  // no copy: completes the phase, consumers see the end
