@@ -71,6 +71,12 @@ glc_status cuda_fail(glc_ctx* ctx, cudaError_t e, const char* where) {
   return fail(ctx, GLC_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
 }
 
+// A partitioner's failure: `what` where it is its own (cudaErrorLaunchTimeout then: a wait gave up).
+glc_status partition_fail(glc_ctx* ctx, cudaError_t e, const std::string& what, const char* where) {
+  if (what.empty()) return cuda_fail(ctx, e, where);
+  return fail(ctx, e == cudaErrorLaunchTimeout ? GLC_ERR_TIMEOUT : GLC_ERR_CUDA, what);
+}
+
 #define CK(call, where)                                  \
   do {                                                   \
     cudaError_t e_ = (call);                             \
@@ -208,6 +214,7 @@ glc_status glc_create(glc_ctx** out, int device) {
   tune_defaults(ctx);
   const char* expire = getenv("GLC_TEST_EXPIRE_FIRST_WAIT");  // test hook: see glc_ctx::expire_next_wait
   if (expire && expire[0] == '1') ctx->expire_next_wait.store(1);
+  if (expire && expire[0] == '2') ctx->expire_next_merge.store(1);
   const char* cache = getenv("GLC_TUNE_CACHE");  // results of an earlier glc_autotune, if they fit
   if (cache && *cache) tune_load(ctx, cache);
   *out = ctx;
@@ -311,7 +318,7 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
     po.alloc = alloc_meta;
     po.stats = ctx->d_stats;
     cudaError_t e = launch_partition_variable(ctx, dtype, dev_values, n, po, s, &perr);
-    if (e != cudaSuccess) return perr.empty() ? cuda_fail(ctx, e, "variable partitioner") : fail(ctx, GLC_ERR_CUDA, perr);
+    if (e != cudaSuccess) return partition_fail(ctx, e, perr, "variable partitioner");
   }
   if (mode == GLC_PART_FIXED) CK(alloc_meta(c, s), "compress: metadata allocation");
   if (mode == GLC_PART_FIXED && fixed_compress_supported(n, fixed_len)) {
@@ -467,7 +474,7 @@ static glc_status partition_only(glc_ctx* ctx, glc_dtype dtype, const void* valu
   cudaError_t e = v6_base > 0 ? launch_partition_v6(ctx, dtype, dev_values, n, v6_base, po, s)
                               : launch_partition_variable(ctx, dtype, dev_values, n, po, s, &perr);
   if (staged) cudaFreeAsync(staged, s);
-  if (e != cudaSuccess) return perr.empty() ? cuda_fail(ctx, e, "partition") : fail(ctx, GLC_ERR_CUDA, perr);
+  if (e != cudaSuccess) return partition_fail(ctx, e, perr, "partition");
   *num_partitions = P;
   glc_status st = GLC_OK;
   if (P > cap || !starts || !ends) {

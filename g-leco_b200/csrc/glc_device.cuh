@@ -307,9 +307,16 @@ __device__ __forceinline__ long long warp_max_ll(long long v) {
   return v;
 }
 
-// Bounded spin limit for every wait in these kernels (an mbarrier phase); after it the kernel
-// records an error code and returns instead of spinning forever.
+// Limits of every wait in these kernels (an mbarrier phase, a grid barrier), in tests and in wall time;
+// after them the kernel records an error code and returns instead of spinning forever.
 constexpr long long kSpinLimit = 1ll << 26;
+constexpr uint64_t kWaitLimitNs = 2000000000ull;
+
+__device__ __forceinline__ uint64_t global_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
 
 enum : int { DEVERR_NONE = 0, DEVERR_TIMEOUT = 1, DEVERR_BOUNDS = 2 };
 

@@ -76,6 +76,9 @@ struct glc_ctx {
   // test hook (GLC_TEST_EXPIRE_FIRST_WAIT=1 at glc_create): the next decode launch's consumers give
   // up their first wait at once, so that launch reports GLC_ERR_TIMEOUT on a healthy copy
   std::atomic<int> expire_next_wait{0};
+  // test hook (GLC_TEST_EXPIRE_FIRST_WAIT=2): the CTAs of the next merge launch wait for one arrival
+  // more than there are, for a millisecond
+  std::atomic<int> expire_next_merge{0};
   std::string err;
   glc::TuneEntry tune[4][glc::kTuneBuckets][2];  // [dtype][bucket][pre-unpacked source]
   std::mutex stats_mu;                     // held by calls that read results back through h_stats
@@ -399,6 +402,7 @@ struct PartOut {
   int64_t* P = nullptr;
   int32_t** unit_first = nullptr;  // V6 with a column: launch_fit_short's, from pool_alloc
 };
+// (cudaErrorLaunchTimeout: a device-side wait gave up.)
 cudaError_t launch_partition_variable(glc_ctx* ctx, glc_dtype dt, const void* values, int64_t n, const PartOut& out,
                                       cudaStream_t s, std::string* err);
 // partition_v6.cu: the reference's GPU partitioner boundaries, into starts/ends from pool_alloc or a

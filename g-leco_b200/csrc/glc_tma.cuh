@@ -55,12 +55,6 @@ __device__ __forceinline__ bool mbar_test_n(uint64_t* bar, uint32_t parity, int 
   return false;
 }
 
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
 // try_wait with a suspend-time hint: the thread may sleep in the barrier up to `ns` nanoseconds
 // (woken when the phase completes) instead of returning at once.
 __device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parity, uint32_t ns) {
@@ -73,13 +67,13 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parit
   return ok != 0;
 }
 
-// Wait for the phase of parity `parity` on `bar`, giving up after ~2 s of wall time.
+// Wait for the phase of parity `parity` on `bar`, giving up after kWaitLimitNs of wall time.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = global_ns();
   for (long long it = 0; it < kSpinLimit; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 255) == 0 && global_ns() - t0 > 2000000000ull) return false;
+    if ((it & 255) == 0 && global_ns() - t0 > kWaitLimitNs) return false;
   }
   return false;
 }

@@ -743,6 +743,8 @@ struct MergeArgs {
   int32_t* cta_heads;    // per CTA
   unsigned* counters;    // kMergeCounters, zero
   int64_t* out;          // [0] partitions left, [1] 1 when they are in b, [2] DEVERR_*
+  unsigned absent;       // arrivals that the barriers wait for in vain (0; 1 lets the first one run out)
+  uint64_t wait_ns;      // limit of a barrier's wait
 };
 constexpr int kMaxMergeRounds = 64;
 constexpr int kMergeThreads = 512;
@@ -752,21 +754,24 @@ constexpr int kMergeUnitMost = 4096;  // values of a pair that one warp scans, a
 constexpr int kMergeCounters = 4 + 4 * kMaxMergeRounds;
 
 // Barrier of all CTAs of a cooperative launch (a counter that only grows); false when the bounded wait
-// gave up.
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned& arrived, int64_t* status) {
+// gave up.  A CTA that gave up arrives no more: the others' next wait runs out too.
+__device__ __forceinline__ bool grid_barrier(const MergeArgs& a, unsigned& arrived) {
   __shared__ int s_ok;
   __syncthreads();
   arrived += gridDim.x;
   if (threadIdx.x == 0) {
     __threadfence();
-    atomicAdd(bar, 1u);
-    long long spins = 0;
-    unsigned seen;
-    do {
-      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-    } while ((int)(seen - arrived) < 0 && ++spins < kSpinLimit);
-    s_ok = (int)(seen - arrived) >= 0;
-    if (!s_ok) atomicExch((unsigned long long*)status, (unsigned long long)DEVERR_TIMEOUT);
+    atomicAdd(a.counters, 1u);
+    const uint64_t t0 = global_ns();
+    bool ok = false;
+    for (long long spins = 0; spins < kSpinLimit; spins++) {
+      unsigned seen;
+      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(a.counters) : "memory");
+      ok = (int)(seen - (arrived + a.absent)) >= 0;
+      if (ok || ((spins & 255) == 255 && global_ns() - t0 > a.wait_ns)) break;
+    }
+    s_ok = ok;
+    if (!ok) atomicExch((unsigned long long*)(a.out + 2), (unsigned long long)DEVERR_TIMEOUT);
   }
   __syncthreads();
   return s_ok != 0;
@@ -815,7 +820,7 @@ merge_kernel(const T* __restrict__ v, RangeSums rs, MergeArgs a) {
     }
     cur.err[k] = err;
   }
-  if (!grid_barrier(a.counters, arrived, a.out + 2)) return;
+  if (!grid_barrier(a, arrived)) return;
   bool flipped = false;
   for (int round = 0; round < kMaxMergeRounds && m >= 2; round++) {
     unsigned* taken = a.counters + 4 + 4 * round;
@@ -882,7 +887,7 @@ merge_kernel(const T* __restrict__ v, RangeSums rs, MergeArgs a) {
         }
       }
     }
-    if (!grid_barrier(a.counters, arrived, a.out + 2)) return;
+    if (!grid_barrier(a, arrived)) return;
     const unsigned nq = *(volatile unsigned*)queued;
     if (nq) {
       for (unsigned i = gwarp; i < nq; i += nwarps) {
@@ -902,7 +907,7 @@ merge_kernel(const T* __restrict__ v, RangeSums rs, MergeArgs a) {
           }
         }
       }
-      if (!grid_barrier(a.counters, arrived, a.out + 2)) return;
+      if (!grid_barrier(a, arrived)) return;
     }
     // ---- compact: a CTA takes a stretch of the list ----
     const int seg = (m + gridDim.x - 1) / gridDim.x, k0 = min(m, (int)blockIdx.x * seg), k1 = min(m, k0 + seg);
@@ -928,7 +933,7 @@ merge_kernel(const T* __restrict__ v, RangeSums rs, MergeArgs a) {
         for (int w = 0; w < kMergeThreads / 32; w++) t += s_scan[w];
         a.cta_heads[blockIdx.x] = t;
       }
-      if (!grid_barrier(a.counters, arrived, a.out + 2)) return;
+      if (!grid_barrier(a, arrived)) return;
       for (int c = threadIdx.x; c < (int)gridDim.x; c += kMergeThreads) {
         const int h = *(volatile int32_t*)(a.cta_heads + c);
         all += h;
@@ -986,7 +991,7 @@ merge_kernel(const T* __restrict__ v, RangeSums rs, MergeArgs a) {
     }
     rej = __reduce_add_sync(FULL_MASK, rej);
     if (lane == 0 && rej) atomicAdd(nrej, (unsigned)rej);
-    if (!grid_barrier(a.counters, arrived, a.out + 2)) return;
+    if (!grid_barrier(a, arrived)) return;
     const PartList t = cur;
     cur = nxt;
     nxt = t;
@@ -1175,6 +1180,12 @@ static cudaError_t partition_typed(glc_ctx* ctx, const T* v, int64_t n, const Pa
   ma.m = (int32_t)m;
   ma.counters = counters;
   ma.out = dsc + 4;
+  ma.absent = 0;
+  ma.wait_ns = kWaitLimitNs;
+  if (ctx->expire_next_merge.load() > 0 && ctx->expire_next_merge.exchange(0) > 0) {
+    ma.absent = 1;
+    ma.wait_ns = 1000000;
+  }
   chain_emit_kernel<<<(unsigned)nr, 32, (sizeof(int32_t) + sizeof(uint16_t)) * rb, s>>>(nb_next, nb_err, entries, base, rg, n,
                                                                                          ma.a.start, ma.a.end, ma.a.err);
   // one CTA per SM, all resident; fewer when the list is short (a cheaper barrier)
@@ -1186,8 +1197,12 @@ static cudaError_t partition_typed(glc_ctx* ctx, const T* v, int64_t n, const Pa
       (e = cudaStreamSynchronize(s)) != cudaSuccess)
     return e;
   const int64_t P = ctx->h_stats[0];
+  if (ctx->h_stats[2] == DEVERR_TIMEOUT) {
+    if (err) *err = "a device-side wait of the partitioner gave up";
+    return cudaErrorLaunchTimeout;
+  }
   if (ctx->h_stats[2] != DEVERR_NONE || P <= 0 || P > m) {
-    if (err) *err = ctx->h_stats[2] == DEVERR_TIMEOUT ? "a device-side wait of the partitioner gave up" : "partitioner produced an invalid merge";
+    if (err) *err = "partitioner produced an invalid merge";
     return cudaErrorUnknown;
   }
   const PartList fin = ctx->h_stats[1] ? ma.b : ma.a;
