@@ -369,7 +369,8 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
   if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "compress: fit");
-  if (ctx->h_stats[2] != DEVERR_NONE) return fail(ctx, GLC_ERR_TIMEOUT, "compress: a device-side wait of the fit gave up");
+  if (ctx->h_stats[2] == DEVERR_TIMEOUT) return fail(ctx, GLC_ERR_TIMEOUT, "compress: a device-side wait of the fit gave up");
+  if (ctx->h_stats[2] != DEVERR_NONE) return fail(ctx, GLC_ERR_CUDA, "compress: partitions beyond the fit's units");
   c->total_bits = ctx->h_stats[0];
   c->max_bits = (int32_t)ctx->h_stats[1];
   set_word_counts(c);
