@@ -77,6 +77,15 @@ glc_status partition_fail(glc_ctx* ctx, cudaError_t e, const std::string& what, 
   return fail(ctx, e == cudaErrorLaunchTimeout ? GLC_ERR_TIMEOUT : GLC_ERR_CUDA, what);
 }
 
+// A block of the temporaries' pool, given back in the stream's order on every way out.
+struct PoolGuard {
+  void** p;
+  cudaStream_t s;
+  ~PoolGuard() {
+    if (*p) cudaFreeAsync(*p, s);
+  }
+};
+
 #define CK(call, where)                                  \
   do {                                                   \
     cudaError_t e_ = (call);                             \
@@ -299,6 +308,7 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
   c->pool = ctx->pool;
   c->sync_free = true;
   int32_t* unit_first = nullptr;  // V6: the first partition of each unit of kFitShort values
+  PoolGuard unit_guard{reinterpret_cast<void**>(&unit_first), s};
   if (mode == GLC_PART_FIXED) {
     c->P = (n + fixed_len - 1) / fixed_len;
     c->fixed_len = fixed_len;
@@ -357,14 +367,10 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
     const size_t sb = brief ? fit_short_scratch_bytes(c->P) : fit_scratch_bytes(nullptr, n, c->P);
     void* scratch = nullptr;
     e = pool_alloc(ctx, &scratch, sb, s);
-    if (e != cudaSuccess) {
-      if (unit_first) cudaFreeAsync(unit_first, s);
-      return cuda_fail(ctx, e, "compress: scratch allocation");
-    }
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "compress: scratch allocation");
     e = brief ? launch_fit_short(dtype, dev_values, c, unit_first, scratch, ctx->d_stats, s)
               : launch_fit(dtype, dev_values, c, scratch, sb, ctx->d_stats, s);
     cudaFreeAsync(scratch, s);
-    if (unit_first) cudaFreeAsync(unit_first, s);
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -457,14 +463,15 @@ static glc_status partition_only(glc_ctx* ctx, glc_dtype dtype, const void* valu
   if (n > 0 && !values) return fail(ctx, GLC_ERR_INVALID_ARG, "null values");
   const void* dev_values = values;
   void* staged = nullptr;
+  int32_t* ds = nullptr;
+  int32_t* de = nullptr;
+  PoolGuard guards[3] = {{&staged, s}, {reinterpret_cast<void**>(&ds), s}, {reinterpret_cast<void**>(&de), s}};
   if (flags & GLC_HOST_IN) {
     const size_t bytes = (size_t)n * dtype_size(dtype);
     CK(pool_alloc(ctx, &staged, bytes, s), "partition: upload");
     CK(host_upload(ctx, staged, values, bytes, s), "partition: upload");
     dev_values = staged;
   }
-  int32_t* ds = nullptr;
-  int32_t* de = nullptr;
   int64_t P = 0;
   std::string perr;
   std::unique_lock<std::mutex> stats_lock(ctx->stats_mu);  // partition counts come back through h_stats
@@ -474,7 +481,6 @@ static glc_status partition_only(glc_ctx* ctx, glc_dtype dtype, const void* valu
   po.P = &P;
   cudaError_t e = v6_base > 0 ? launch_partition_v6(ctx, dtype, dev_values, n, v6_base, po, s)
                               : launch_partition_variable(ctx, dtype, dev_values, n, po, s, &perr);
-  if (staged) cudaFreeAsync(staged, s);
   if (e != cudaSuccess) return partition_fail(ctx, e, perr, "partition");
   *num_partitions = P;
   glc_status st = GLC_OK;
@@ -486,8 +492,6 @@ static glc_status partition_only(glc_ctx* ctx, glc_dtype dtype, const void* valu
     if (e == cudaSuccess) e = cudaMemcpyAsync(ends, de, 4 * P, k, s);
     if (e != cudaSuccess) st = cuda_fail(ctx, e, "partition: copy out");
   }
-  cudaFreeAsync(ds, s);
-  cudaFreeAsync(de, s);
   if (flags & GLC_HOST_OUT) CK(cudaStreamSynchronize(s), "partition: sync");
   return st;
 }
