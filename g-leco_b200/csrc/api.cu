@@ -141,6 +141,7 @@ cudaError_t alloc_meta(glc_column* c, cudaStream_t s) {
   cudaError_t e = col_alloc(c, &m, off[9], s);
   if (e != cudaSuccess) return e;
   c->meta = m;
+  c->meta_bytes = off[9];
   c->d_start = (int32_t*)(m + off[0]);
   c->d_end = (int32_t*)(m + off[1]);
   c->d_types = (int32_t*)(m + off[2]);
@@ -156,6 +157,13 @@ cudaError_t alloc_meta(glc_column* c, cudaStream_t s) {
 void set_word_counts(glc_column* c) {
   c->nwords = (c->total_bits + 31) / 32;
   c->nwords_alloc = ((c->nwords + 3) & ~3ll) + 8;  // decoders read up to 3 words past a field
+}
+
+// The word array, of c's word counts; `room`: with the slack that lets a freed column's block fit the next.
+cudaError_t alloc_words(glc_column* c, bool room, cudaStream_t s) {
+  const uint64_t bytes = 4 * (uint64_t)c->nwords_alloc;
+  c->words_bytes = room ? words_alloc_bytes(bytes) : bytes;
+  return col_alloc(c, &c->d_words, c->words_bytes, s);
 }
 
 // Private pools that keep freed memory, so that columns and per-call temporaries (host-output
@@ -348,7 +356,7 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
       c->total_bits = ctx->h_stats[0];
       c->max_bits = (int32_t)ctx->h_stats[1];
       set_word_counts(c);
-      e = col_alloc(c, &c->d_words, words_alloc_bytes(4 * c->nwords_alloc), s);
+      e = alloc_words(c, true, s);
     }
     if (e == cudaSuccess) e = launch_fixed_place(dtype, c, fixed_len, scratch, st, s);
     cudaFreeAsync(scratch, s);
@@ -380,7 +388,7 @@ static glc_status compress_impl(glc_ctx* ctx, glc_dtype dtype, const void* dev_v
   c->total_bits = ctx->h_stats[0];
   c->max_bits = (int32_t)ctx->h_stats[1];
   set_word_counts(c);
-  CK(col_alloc(c, &c->d_words, words_alloc_bytes(4 * c->nwords_alloc), s), "compress: word allocation");
+  CK(alloc_words(c, true, s), "compress: word allocation");
   const int64_t parts_per_tile = ctx->h_stats[3];
   CK(launch_desc_and_tiles(c, s), "compress: tables");
   // the partitioners' starts are multiples of 128 and of kV6Base / 2
@@ -789,7 +797,7 @@ glc_status glc::deserialize_column(glc_ctx* ctx, glc_dtype dtype, const void* bl
   cudaError_t e = alloc_meta(c, s);
   if (e != cudaSuccess) return bail(cuda_fail(ctx, e, "deserialize: allocation"));
   set_word_counts(c);
-  if ((e = col_alloc(c, &c->d_words, 4 * c->nwords_alloc, s)) != cudaSuccess)
+  if ((e = alloc_words(c, false, s)) != cudaSuccess)
     return bail(cuda_fail(ctx, e, "deserialize: allocation"));
   const cudaMemcpyKind k = host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
   const uint8_t* b = (const uint8_t*)blob;

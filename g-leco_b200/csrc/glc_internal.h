@@ -102,6 +102,8 @@ struct glc_column {
   int64_t reported_size = 0;
   // reference SoA (CompressedData<T>)
   void* meta = nullptr;      // one allocation that holds d_start .. d_err, d_desc and d_tiles (null: views)
+  uint64_t meta_bytes = 0;   // its size
+  uint64_t words_bytes = 0;  // the size of d_words' allocation
   int32_t* d_start = nullptr;
   int32_t* d_end = nullptr;
   int32_t* d_types = nullptr;

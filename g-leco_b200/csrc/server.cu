@@ -42,14 +42,10 @@ int64_t now_ns() {
 // bits, bit offset, error bound), the partition descriptors, the tile table, the padded
 // bitstream and the optional pre-unpacked residuals.
 uint64_t column_device_bytes(const glc_column* c) {
-  const uint64_t P = (uint64_t)c->P;
+  const uint64_t plain = c->d_plain ? 8ull * (uint64_t)c->n + 16 : 0;
   if (c->blob_view)  // an attached blob: the blob (or its bitstream) it holds and its derived tables
-    return c->owned_bytes + P * sizeof(PartDesc) + sizeof(TileInfo) * (uint64_t)(c->ntiles + 1) +
-           (c->d_plain ? 8ull * (uint64_t)c->n + 16 : 0);
-  uint64_t b = P * (4 + 4 + 4 + 32 + 4 + 8 + 8) + P * sizeof(PartDesc) + sizeof(TileInfo) * (uint64_t)(c->ntiles + 1);
-  if (c->d_words) b += 4ull * (uint64_t)c->nwords_alloc;
-  if (c->d_plain) b += 8ull * (uint64_t)c->n + 16;
-  return b;
+    return c->owned_bytes + (uint64_t)c->P * sizeof(PartDesc) + sizeof(TileInfo) * (uint64_t)(c->ntiles + 1) + plain;
+  return c->meta_bytes + (c->d_words ? c->words_bytes : 0) + plain;  // as allocated, paddings included
 }
 
 constexpr int kMaxSlots = 16;

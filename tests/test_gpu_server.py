@@ -172,6 +172,29 @@ def test_everything_submitted_at_once_shares_launches():
     server.close()
 
 
+@pytest.mark.parametrize("n", [4096, 200_003, 5_000_000])
+def test_resident_bytes_are_what_a_compressed_column_allocates(n):
+    """The words' block is rounded up to 1/32 of its size and the metadata lies in one block with each
+    array from a 256-byte boundary: the budget counts both as allocated."""
+    ctx = glc.Context(0)
+    v = _values(glc.I64, n, 5)
+    col = glc.compress_device(ctx, glc.I64, v.ctypes.data, n, glc.FIXED, host=True)
+    info = col.info()
+    words = 4 * ((((info.total_bits + 31) // 32 + 3) & ~3) + 8)
+    if words >= 1 << 20:
+        step = 1 << 15
+        while step * 64 <= words:
+            step *= 2
+        words = -(-words // step) * step
+    P, tiles = info.num_partitions, -(-n // 4096) + 1
+    meta = sum(-(-b // 256) * 256 for b in (4 * P, 4 * P, 4 * P, 32 * P, 4 * P, 8 * P, 8 * P, 32 * P, 16 * tiles))
+    server = glc.Server(ctx, budget_bytes=1 << 40)
+    server.admit(col)
+    assert server.stats().resident_bytes == words + meta
+    server.close()
+    ctx.close()
+
+
 def test_admission_budget_and_lru_eviction():
     ctx = glc.Context(0)
     v = _values(glc.I64, 500_000, 1)
