@@ -167,8 +167,11 @@ cudaError_t alloc_words(glc_column* c, bool room, cudaStream_t s) {
 }
 
 // Private pools that keep freed memory, so that columns and per-call temporaries (host-output
-// staging, scratch) cost no fresh device allocation after the first call: the columns' with release
-// threshold = max, the temporaries' up to 8 GB.
+// staging, scratch) cost no fresh device allocation after the first call: the compressed columns' with
+// release threshold = max, the temporaries' up to 8 GB.  Deserialized columns, which cudaFree gave back
+// to the device, keep no more than kLoadKeep for the next one.
+constexpr uint64_t kLoadColumn = 256ull << 20;  // the largest blob whose column comes from the pool
+constexpr uint64_t kLoadKeep = 2 * kLoadColumn;
 cudaError_t create_pools(glc_ctx* ctx) {
   cudaMemPoolProps props = {};
   props.allocType = cudaMemAllocationTypePinned;
@@ -176,10 +179,12 @@ cudaError_t create_pools(glc_ctx* ctx) {
   props.location.id = ctx->device;
   cudaError_t e = cudaMemPoolCreate(&ctx->pool, &props);
   if (e != cudaSuccess) return e;
-  uint64_t keep = ~0ull, keep_temp = 8ull << 30;
+  uint64_t keep = ~0ull, keep_temp = 8ull << 30, keep_load = kLoadKeep;
   if ((e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) return e;
   if ((e = cudaMemPoolCreate(&ctx->temp_pool, &props)) != cudaSuccess) return e;
-  return cudaMemPoolSetAttribute(ctx->temp_pool, cudaMemPoolAttrReleaseThreshold, &keep_temp);
+  if ((e = cudaMemPoolSetAttribute(ctx->temp_pool, cudaMemPoolAttrReleaseThreshold, &keep_temp)) != cudaSuccess) return e;
+  if ((e = cudaMemPoolCreate(&ctx->load_pool, &props)) != cudaSuccess) return e;
+  return cudaMemPoolSetAttribute(ctx->load_pool, cudaMemPoolAttrReleaseThreshold, &keep_load);
 }
 
 int64_t reported_size(int64_t P, int64_t total_bits) {  // api/G-LeCo.cuh:589-603
@@ -249,9 +254,9 @@ glc_status glc_destroy(glc_ctx* ctx) {
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   for (cudaStream_t a : ctx->aux_stream)
     if (a) cudaStreamDestroy(a);
-  if (ctx->pool || ctx->temp_pool) cudaDeviceSynchronize();
-  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
-  if (ctx->temp_pool) cudaMemPoolDestroy(ctx->temp_pool);
+  if (ctx->pool || ctx->temp_pool || ctx->load_pool) cudaDeviceSynchronize();
+  for (cudaMemPool_t q : {ctx->pool, ctx->temp_pool, ctx->load_pool})
+    if (q) cudaMemPoolDestroy(q);
   delete ctx;
   return GLC_OK;
 }
@@ -722,9 +727,9 @@ glc_status glc_serialize(glc_ctx* ctx, const glc_column* c, void* blob, uint64_t
 
 glc_status glc_deserialize(glc_ctx* ctx, glc_dtype dtype, const void* blob, uint64_t size, int flags, int crc32c,
                            int pre_unpack, glc_column** out, glc_stream stream) {
-  // Columns of up to 256 MB come from the context's pool (a cudaMalloc and cudaFree per array cost 1.4 ms a
+  // Columns of up to kLoadColumn come from a pool (a cudaMalloc and cudaFree per array cost 1.4 ms a
   // column of 2M values); larger ones keep giving their memory back to the device when freed.
-  cudaMemPool_t pool = ctx && size <= (256ull << 20) && !pre_unpack ? ctx->pool : nullptr;
+  cudaMemPool_t pool = ctx && size <= kLoadColumn && !pre_unpack ? ctx->load_pool : nullptr;
   const glc_status st = glc::deserialize_column(ctx, dtype, blob, size, flags, crc32c, pre_unpack, out, stream, pool, false);
   if (st == GLC_OK && pool) (*out)->sync_free = true;  // freed as cudaFree frees
   return st;

@@ -69,6 +69,7 @@ struct glc_ctx {
   cudaStream_t aux_stream[2] = {nullptr, nullptr};  // streaming decode: download, upload (lazy)
   cudaMemPool_t pool = nullptr;  // private stream-ordered pool; keeps freed memory for reuse
   cudaMemPool_t temp_pool = nullptr;  // the same for memory that a call takes and gives back (pool_alloc)
+  cudaMemPool_t load_pool = nullptr;  // deserialized columns; keeps less
   int* d_flags = nullptr;      // [0, 64) decode work counters, [64] device error code
   int64_t* d_stats = nullptr;  // small readback area (total bits, max bits, ...)
   int64_t* h_stats = nullptr;  // pinned mirror of d_stats
