@@ -168,7 +168,10 @@ cudaError_t alloc_words(glc_column* c, bool room, cudaStream_t s) {
 
 // Private pools that keep freed memory, so that columns and per-call temporaries (host-output
 // staging, scratch) cost no fresh device allocation after the first call: the compressed columns' with
-// release threshold = max, the temporaries' up to 8 GB.  Deserialized columns, which cudaFree gave back
+// release threshold = max, the temporaries' up to a quarter of the device (a column of 2^31 8-byte values
+// that comes from the host takes 34 GB of them; what a call takes beyond it is mapped anew each time:
+// with 8 GB, 2 * 10^9 int64 values in fixed partitions took 92 ms instead of 9).  The driver takes
+// unused memory of a pool back before an allocation fails.  Deserialized columns, which cudaFree gave back
 // to the device, keep no more than kLoadKeep for the next one.
 constexpr uint64_t kLoadColumn = 256ull << 20;  // the largest blob whose column comes from the pool
 constexpr uint64_t kLoadKeep = 2 * kLoadColumn;
@@ -179,7 +182,9 @@ cudaError_t create_pools(glc_ctx* ctx) {
   props.location.id = ctx->device;
   cudaError_t e = cudaMemPoolCreate(&ctx->pool, &props);
   if (e != cudaSuccess) return e;
-  uint64_t keep = ~0ull, keep_temp = 8ull << 30, keep_load = kLoadKeep;
+  size_t free_bytes = 0, total_bytes = 0;
+  if ((e = cudaMemGetInfo(&free_bytes, &total_bytes)) != cudaSuccess) return e;
+  uint64_t keep = ~0ull, keep_temp = total_bytes / 4, keep_load = kLoadKeep;
   if ((e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) return e;
   if ((e = cudaMemPoolCreate(&ctx->temp_pool, &props)) != cudaSuccess) return e;
   if ((e = cudaMemPoolSetAttribute(ctx->temp_pool, cudaMemPoolAttrReleaseThreshold, &keep_temp)) != cudaSuccess) return e;
