@@ -770,7 +770,7 @@ glc_status glc_batch_compress(glc_ctx* ctx, const glc_dtype* dtypes, const void*
     return ee;
   };
   if ((e = dalloc(b, &d_fc, nc)) != cudaSuccess || (e = dalloc(b, &d_pb, nc + 1)) != cudaSuccess ||
-      (e = dalloc(b, &d_colbits, 3 * (size_t)nc + 1)) != cudaSuccess)
+      (e = dalloc(b, &d_colbits, 3 * (size_t)nc)) != cudaSuccess)
     return bail(bcuda(ctx, e, "batch compress: allocation"));
   // lengths 1024 / 2048 / 4096: the choice pass measures the exact bits of all three, and the
   // one-pass kernel compresses every column at its chosen length
@@ -779,7 +779,7 @@ glc_status glc_batch_compress(glc_ctx* ctx, const glc_dtype* dtypes, const void*
   std::vector<unsigned long long> hbits(3 * (size_t)nc);
   std::vector<PrePacked> pre;
   if (one_pass) {  // one read of every column measures all three candidate lengths
-    if ((e = cudaMemsetAsync(d_colbits, 0, sizeof(unsigned long long) * (3 * (size_t)nc + 1), s)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(d_colbits, 0, sizeof(unsigned long long) * 3 * (size_t)nc, s)) != cudaSuccess)
       return bail(bcuda(ctx, e, "batch compress: sizes"));
     // one launch per element type, which also packs every tile at length 4096 (kept by most
     // columns); the host tables stay alive until the stream is synchronised
@@ -838,8 +838,7 @@ glc_status glc_batch_compress(glc_ctx* ctx, const glc_dtype* dtypes, const void*
       if ((e = cudaMemcpyAsync(d_g, g.data(), sizeof(CfColumn) * g.size(), cudaMemcpyHostToDevice, s)) ||
           (e = cudaMemcpyAsync(d_ib, ib.data(), sizeof(int64_t) * ib.size(), cudaMemcpyHostToDevice, s)) ||
           (e = launch_pack_item_owner(d_ib, (int)g.size(), d_owner, s)) ||
-          (e = launch_choose_lengths(dt, d_g, d_owner, ib.back(), d_colbits + 3 * (size_t)nc, ctx->num_sms, s,
-                                     scratch, tdesc, terr)))
+          (e = launch_choose_lengths(dt, d_g, d_owner, ib.back(), s, scratch, tdesc, terr)))
         return release_pre(), bail(bcuda(ctx, e, "batch compress: length choice"));
     }
     // everything that does not depend on the lengths, while the choice runs on the device
@@ -849,15 +848,10 @@ glc_status glc_batch_compress(glc_ctx* ctx, const glc_dtype* dtypes, const void*
                                              fixed_partition_len ? fixed_partition_len : kCandidates[0], s, &prep);
       if (ps != GLC_OK) return release_pre(), bail(ps);
     }
-    unsigned long long choice_status = 0;
     if ((e = cudaMemcpyAsync(hbits.data(), d_colbits, sizeof(unsigned long long) * 3 * nc, cudaMemcpyDeviceToHost,
                              s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(&choice_status, d_colbits + 3 * (size_t)nc, sizeof(unsigned long long),
-                             cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
       return release_pre(), bail(bcuda(ctx, e, "batch compress: sizes"));
-    if (choice_status != DEVERR_NONE)
-      return release_pre(), bail(bfail(ctx, GLC_ERR_TIMEOUT, "batch compress: a device-side wait gave up"));
     // the smallest compressed size; within 0.1 % of it, the length the tuner found to decode
     // fastest for the element type and the column's mean field width (when the table holds one)
     for (int i = 0; i < nc && fixed_partition_len == 0; i++) {

@@ -22,7 +22,6 @@
 #include "glc_group.cuh"
 #include "glc_internal.h"
 #include "glc_scan.cuh"
-#include "glc_tma.cuh"
 
 namespace glc {
 
@@ -41,7 +40,7 @@ struct FixedCompressArgs {
   int64_t slot_words;
   int64_t* tile_bits;         // per item: bits of the tile (nitems + 1 entries: the scan's input)
   const int64_t* tile_first;  // per item: exclusive scan of tile_bits over the launch (nitems + 1)
-  unsigned long long* status; // DEVERR_* when a bounded wait gave up or a column's words overflow
+  unsigned long long* status; // the place: DEVERR_BOUNDS when a column's words would pass its array
   PartDesc* tdesc;            // the length choice that also packs at 4096: per item, the tile's one
   long long* terr;            // partition's descriptor (tile-relative offset) and max error
 };
@@ -292,7 +291,7 @@ fixed_compress_kernel(const __grid_constant__ FixedCompressArgs a) {
       slow = !ok;
       if (slow && mode != CF_DIRECT) {
         mx = 0;
-const double c = s_c[p];
+        const double c = s_c[p];
         const long long ci = s_ci[p];
         double xi = (double)i0;
 #pragma unroll 1
@@ -821,14 +820,12 @@ template <typename T, bool PACK> static cudaError_t launch_choose_t(const FixedC
 static void carve(FixedCompressArgs& a, glc_dtype dt, void* scratch);
 
 cudaError_t launch_choose_lengths(glc_dtype dt, const CfColumn* cols, const int32_t* owner, int64_t nitems,
-                                  unsigned long long* status, int num_sms, cudaStream_t s, void* scratch,
-                                  PartDesc* tdesc, long long* terr) {
+                                  cudaStream_t s, void* scratch, PartDesc* tdesc, long long* terr) {
   if (nitems <= 0) return cudaSuccess;
   FixedCompressArgs a{};
   a.cols = cols;
   a.owner = owner;
   a.nitems = nitems;
-  a.status = status;
   const bool pack = scratch != nullptr;
   if (pack) {
     carve(a, dt, scratch);
@@ -898,8 +895,8 @@ static cudaError_t place_pass(const FixedCompressArgs& a, int num_sms, cudaStrea
 // One column: values (n of dt, fixed partitions of L) into c's metadata arrays and tables
 // (allocated by the caller for P = ceil(n / L) partitions); scratch holds
 // fixed_compress_scratch_bytes(dt, ntiles) bytes.  Pass 1 leaves stats[0] = the column's total bits,
-// stats[1] = its widest field, stats[2] = a DEVERR_* code (stats[0..3] zeroed here); the caller
-// reads them, allocates the words and calls launch_fixed_place.
+// stats[1] = its widest field (stats[0..3] zeroed here); the caller reads them, allocates the words
+// and calls launch_fixed_place.
 cudaError_t launch_fixed_compress(glc_dtype dt, const void* values, glc_column* c, int32_t L, void* scratch,
                                   unsigned long long* stats, cudaStream_t s) {
   FixedCompressArgs a{};
@@ -922,7 +919,6 @@ cudaError_t launch_fixed_compress(glc_dtype dt, const void* values, glc_column* 
   col.tiles = c->d_tiles;
   col.stats = stats;
   a.nitems = c->ntiles;
-  a.status = stats + 2;
   cudaError_t e;
   if ((e = cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned long long), s)) != cudaSuccess) return e;
   // the total: the scan's grand total (the column is the whole launch)

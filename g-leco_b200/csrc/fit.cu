@@ -10,6 +10,7 @@
 // (64-bit atomicMax per partition), and a thread per partition sets the bit width.  The
 // bit offsets are an exclusive scan of len * bits.  All passes read the values once or twice
 // with coalesced loads; nothing here is a contraction, so the bound is HBM bandwidth.
+#include <algorithm>
 #include <type_traits>
 #include "glc_group.cuh"
 #include "glc_internal.h"
@@ -33,23 +34,6 @@ cudaError_t launch_fixed_partitions(int32_t* starts, int32_t* ends, int64_t n, i
   if (P <= 0) return cudaSuccess;
   fixed_partitions_kernel<<<(unsigned)((P + 255) / 256), 256, 0, s>>>(starts, ends, n, len, P);
   return cudaGetLastError();
-}
-
-__global__ void chunk_count_kernel(const int32_t* __restrict__ starts, const int32_t* __restrict__ ends, int64_t P,
-                                   int64_t* __restrict__ nch) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  int64_t len = (int64_t)ends[p] - starts[p];
-  nch[p] = len > 0 ? (len + kFitChunk - 1) / kFitChunk : 0;
-}
-
-// owner[c] = the partition of chunk c (one thread per partition writes its chunks), so a fit CTA
-// finds its partition with one load instead of a dependent binary search.
-__global__ void chunk_owner_kernel(const int64_t* __restrict__ base, const int64_t* __restrict__ nch, int64_t P,
-                                   int32_t* __restrict__ owner) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  for (int64_t c = base[p], e = base[p] + nch[p]; c < e; c++) owner[c] = (int32_t)p;
 }
 
 struct FitChunkArgs {
@@ -380,14 +364,6 @@ template <typename T> __global__ void fit_bits_kernel(const int32_t* __restrict_
 
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// nm[p] = chunks of p when p is longer than one chunk (their maximum error takes a second pass).
-__global__ void multi_count_kernel(const int32_t* __restrict__ starts, const int32_t* __restrict__ ends,
-                                   const int64_t* __restrict__ nch, int64_t P, int64_t* __restrict__ nm) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  nm[p] = ((int64_t)ends[p] - starts[p]) > kFitChunk ? nch[p] : 0;
-}
-
 // Fixed partitions of length L (the last one n - (P - 1) L): the chunk tables in closed form, in
 // one launch -- chunks per partition, each partition's first chunk, chunk -> partition, and the
 // chunk counts of the two fit passes.  Partitions longer than one chunk are all the full ones
@@ -417,15 +393,15 @@ __global__ void fixed_chunk_setup_kernel(int64_t n, int64_t L, int64_t P, int64_
   }
 }
 
-size_t fit_scratch_bytes(const int32_t*, int64_t n, int64_t P) {
+size_t fit_scratch_bytes(int64_t n, int64_t P) {
   int64_t ncmax = n / kFitChunk + P + 1;
   size_t b = 0;
-  b += align_up(sizeof(int64_t) * (P + 1), 256) * 4;                  // nch, chunk_base, nm, mbase
+  b += align_up(sizeof(int64_t) * (P + 1), 256) * 2;                  // nch, chunk_base
   b += align_up(sizeof(int64_t) * (scan_num_tiles(P) + 1), 256);      // scan tiles
   b += align_up(sizeof(int64_t) * 2, 256) * 2;                        // chunk count, long-partition chunk count
   b += align_up(sizeof(i128) * ncmax, 256) * 2;                       // sy, sxy
   b += align_up(sizeof(int) * ncmax, 256);                            // ovf
-  b += align_up(sizeof(int32_t) * ncmax, 256) * 2;                    // owner, owner of the long-partition list
+  b += align_up(sizeof(int32_t) * ncmax, 256);                        // owner
   b += align_up(sizeof(int64_t) * (P + 1), 256);                      // widths
   return b;
 }
@@ -459,8 +435,6 @@ static cudaError_t fit_typed(const T* v, glc_column* c, void* scratch, int64_t* 
   auto take = [&](size_t bytes) { void* r = sp; sp += align_up(bytes, 256); return r; };
   int64_t* nch = (int64_t*)take(sizeof(int64_t) * (P + 1));
   int64_t* base = (int64_t*)take(sizeof(int64_t) * (P + 1));
-  int64_t* nm = (int64_t*)take(sizeof(int64_t) * (P + 1));
-  int64_t* mbase = (int64_t*)take(sizeof(int64_t) * (P + 1));
   int64_t* tiles = (int64_t*)take(sizeof(int64_t) * (scan_num_tiles(P) + 1));
   int64_t* nchunks = (int64_t*)take(sizeof(int64_t) * 2);
   int64_t* nmulti = (int64_t*)take(sizeof(int64_t) * 2);
@@ -468,7 +442,6 @@ static cudaError_t fit_typed(const T* v, glc_column* c, void* scratch, int64_t* 
   i128* sxy = (i128*)take(sizeof(i128) * ncmax);
   int* ovf = (int*)take(sizeof(int) * ncmax);
   int32_t* owner = (int32_t*)take(sizeof(int32_t) * ncmax);
-  int32_t* owner_m = (int32_t*)take(sizeof(int32_t) * ncmax);
   int64_t* widths = (int64_t*)take(sizeof(int64_t) * (P + 1));
   const unsigned pg = (unsigned)((P + 255) / 256);
   const int num_sms = c->ctx->num_sms;
@@ -477,32 +450,16 @@ static cudaError_t fit_typed(const T* v, glc_column* c, void* scratch, int64_t* 
   // partitions per 4096-value tile (without the last partition)
   if ((e = cudaMemsetAsync(d_stats, 0, 4 * sizeof(int64_t), s)) != cudaSuccess) return e;
 
-  if (c->fixed_len > 0) {  // fixed partitions: closed-form tables, one launch
-    const int64_t span = n / kFitChunk + P + 1;
-    int64_t grid = (span + 255) / 256;
-    if (grid > 4ll * num_sms) grid = 4ll * num_sms;
-    fixed_chunk_setup_kernel<<<(unsigned)grid, 256, 0, s>>>(n, c->fixed_len, P, nch, base, owner, nchunks, nmulti);
-    owner_m = owner;  // the second pass's chunks are a prefix of the first's
-    mbase = base;
-  } else {
-    chunk_count_kernel<<<pg, 256, 0, s>>>(c->d_start, c->d_end, P, nch);
-    if ((e = exclusive_scan<int64_t>(nch, base, P, nchunks, tiles, s)) != cudaSuccess) return e;
-    chunk_owner_kernel<<<pg, 256, 0, s>>>(base, nch, P, owner);
-    // the chunks of the second pass (partitions longer than one chunk)
-    multi_count_kernel<<<pg, 256, 0, s>>>(c->d_start, c->d_end, nch, P, nm);
-    if ((e = exclusive_scan<int64_t>(nm, mbase, P, nmulti, tiles, s)) != cudaSuccess) return e;
-    chunk_owner_kernel<<<pg, 256, 0, s>>>(mbase, nm, P, owner_m);
-  }
+  const int64_t grid = std::min<int64_t>((ncmax + 255) / 256, 4ll * num_sms);
+  fixed_chunk_setup_kernel<<<(unsigned)grid, 256, 0, s>>>(n, c->fixed_len, P, nch, base, owner, nchunks, nmulti);
 
   FitStreamArgs a{c->d_start, c->d_end, nchunks, owner, base, P, sy, sxy, ovf, base,
                   c->d_types, c->d_params, c->d_err, (unsigned long long*)(d_stats + 2)};
   if ((e = launch_fit_stream<T, 0>(v, a, num_sms, s)) != cudaSuccess) return e;
   FitChunkArgs fa{c->d_start, c->d_end, base, nchunks, owner, P, sy, sxy, ovf};
   fit_solve_kernel<T><<<pg, 256, 0, s>>>(fa, nch, c->d_types, c->d_params, c->d_err);
-  FitStreamArgs am = a;
+  FitStreamArgs am = a;  // (the second pass's chunks are a prefix of the first's)
   am.count = nmulti;
-  am.owner = owner_m;
-  am.base = mbase;
   if ((e = launch_fit_stream<T, 1>(v, am, num_sms, s)) != cudaSuccess) return e;
   fit_bits_kernel<T><<<pg, 256, 0, s>>>(c->d_start, c->d_end, c->d_types, c->d_err, c->d_bits, widths, P,
                                          (unsigned long long*)(d_stats + 1), (unsigned long long*)(d_stats + 3));

@@ -204,8 +204,8 @@ inline size_t words_alloc_bytes(size_t bytes) {
 // ---- kernel launchers (defined in the .cu files) -------------------------------------
 // fit.cu
 cudaError_t launch_fixed_partitions(int32_t* starts, int32_t* ends, int64_t n, int32_t len, int64_t P, cudaStream_t s);
-size_t fit_scratch_bytes(const int32_t* unused, int64_t n, int64_t P);
-// Fits every partition of c (starts/ends set); d_stats[0] = total bits, d_stats[1] = max bits.
+size_t fit_scratch_bytes(int64_t n, int64_t P);
+// Fits the fixed partitions of c (starts/ends set); d_stats[0] = total bits, d_stats[1] = max bits.
 cudaError_t launch_fit(glc_dtype dt, const void* values, glc_column* c, void* scratch, size_t scratch_bytes,
                        int64_t* d_stats, cudaStream_t s);
 // The same for 1 to 8 partitions inside each unit of kFitShort values, none across two: unit_first[u] =
@@ -256,8 +256,8 @@ cudaError_t launch_fixed_compress_batch(glc_dtype dt, const CfColumn* cols, cons
 // at length 4096: its words into its slot, its descriptor and max error into tdesc / terr (nitems
 // each); launch_place_prepacked then places the columns that keep length 4096.
 cudaError_t launch_choose_lengths(glc_dtype dt, const CfColumn* cols, const int32_t* owner, int64_t nitems,
-                                  unsigned long long* status, int num_sms, cudaStream_t s, void* scratch = nullptr,
-                                  PartDesc* tdesc = nullptr, long long* terr = nullptr);
+                                  cudaStream_t s, void* scratch = nullptr, PartDesc* tdesc = nullptr,
+                                  long long* terr = nullptr);
 cudaError_t launch_place_prepacked(glc_dtype dt, const CfColumn* cols, const int32_t* owner, int64_t nitems,
                                    void* scratch, PartDesc* tdesc, long long* terr, unsigned long long* status,
                                    int num_sms, cudaStream_t s);
