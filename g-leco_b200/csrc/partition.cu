@@ -754,7 +754,9 @@ constexpr int kMergeUnitMost = 4096;  // values of a pair that one warp scans, a
 constexpr int kMergeCounters = 4 + 4 * kMaxMergeRounds;
 
 // Barrier of all CTAs of a cooperative launch (a counter that only grows); false when the bounded wait
-// gave up.  A CTA that gave up arrives no more: the others' next wait runs out too.
+// gave up.  A CTA that gave up arrives no more: the others' next wait runs out too.  The limit is longer
+// than kWaitLimitNs: the last CTAs may first have to wait for a kernel of another stream to leave their SMs.
+constexpr uint64_t kGridWaitNs = 20000000000ull;
 __device__ __forceinline__ bool grid_barrier(const MergeArgs& a, unsigned& arrived) {
   __shared__ int s_ok;
   __syncthreads();
@@ -1181,7 +1183,7 @@ static cudaError_t partition_typed(glc_ctx* ctx, const T* v, int64_t n, const Pa
   ma.counters = counters;
   ma.out = dsc + 4;
   ma.absent = 0;
-  ma.wait_ns = kWaitLimitNs;
+  ma.wait_ns = kGridWaitNs;
   if (ctx->expire_next_merge.load() > 0 && ctx->expire_next_merge.exchange(0) > 0) {
     ma.absent = 1;
     ma.wait_ns = 1000000;
