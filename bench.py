@@ -587,14 +587,20 @@ def run_c1(args):
                      "algorithmic_bytes": algo},
         "e2e": {"value": round(4 * n / e2e_s / 1e9, 3), "unit": "GB/s", "h2d_bytes_per_step": 4 * n + 4 * q,
                 "d2h_bytes_per_step": 4 * n + 4 * q + 8},
-        "gpu_launches": (COMPRESS_LAUNCHES["fixed"] + 2) * args.steps, "clocks": clk, "cpu_baseline": cpu,
+        "gpu_launches": (compress_launches("fixed", n, info.num_partitions) + 2) * args.steps, "clocks": clk,
+        "cpu_baseline": cpu,
     }
     print(json.dumps(line), flush=True)
     ctx.close()
     return 0
 
 
-COMPRESS_LAUNCHES = {"fixed": 5, "v6": 29}  # kernels launched by one compress call (fixed: compress, 3 scan, place)
+def compress_launches(partitioning: str, n: int, partitions: int):
+    """Kernels launched by one compress call, or None where the data decide (variable partitions).  Fixed:
+    compress, scan of the tiles' bits, place.  V6: variances, thresholds, boundaries, fit, scan of the
+    partitions' bits, two tables, pack.  A scan is one launch up to 16,384 items, three beyond."""
+    scan = lambda items: 1 if items <= 16_384 else 3
+    return {"fixed": 2 + scan(-(-n // 4096)), "v6": 7 + scan(partitions)}.get(partitioning)
 
 
 def run_compress(args):
@@ -664,6 +670,7 @@ def run_compress(args):
             e2e.append(e0.elapsed_time(e1))
         c.free()
     e2e_ms = sum(e2e) / len(e2e)
+    launches = compress_launches(args.partitioning, n, info.num_partitions)
     cpu = None
     if not args.no_cpu_baseline and args.partitioning == "fixed":
         import oracle
@@ -687,7 +694,7 @@ def run_compress(args):
                      "algorithmic_bytes": in_bytes + comp},
         "e2e": {"value": round(in_bytes / (e2e_ms / 1e3) / 1e9, 2), "unit": "GB/s", "h2d_bytes_per_step": in_bytes,
                 "d2h_bytes_per_step": 8},
-        "gpu_launches": COMPRESS_LAUNCHES[args.partitioning] * args.steps if args.partitioning in COMPRESS_LAUNCHES else None,
+        "gpu_launches": None if launches is None else launches * args.steps,
         "clocks": clk, "cpu_baseline": cpu,
     }
     print(json.dumps(line), flush=True)
