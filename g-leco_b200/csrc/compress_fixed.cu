@@ -49,7 +49,7 @@ struct FixedCompressArgs {
 
 // Per value, for the range tests of the partition: uint64 keeps the max of the high words, above
 // 2^21 when some value exceeds 2^53 (direct copy; exactly 2^21 is decided by a rescan of the
-// partition, cf_any_above_2_53) and below 2^19 iff every value is below 2^51; int64 keeps the OR of
+// partition, cg_overflows) and below 2^19 iff every value is below 2^51; int64 keeps the OR of
 // hi ^ (hi >> 31), below 2^19 iff every value is in [-2^51, 2^51); 4-byte values always fit.
 template <typename T> __device__ __forceinline__ void value_flag(uint32_t& f, T y) {
   if (sizeof(T) == 8) {
@@ -228,11 +228,10 @@ fixed_compress_kernel(const __grid_constant__ FixedCompressArgs a) {
     HalfSums<T> hs;
     uint32_t flag = 0;
     cg_sums<T>(row, i0, hs, flag);
-    // a warp's sum by 24-bit limbs holds for partials below 2^50 (the high limb below 2^26 a lane)
-    const long long c0 = seg_sum48((long long)hs.s_lo, W);
-    const long long c1 = sizeof(T) == 8 ? seg_sum48((long long)hs.s_hi, W) : 0;
-    const long long c2 = seg_sum48((long long)hs.x_lo, W);
-    const long long c3 = sizeof(T) == 8 ? seg_sum48((long long)hs.x_hi, W) : 0;
+    const long long c0 = seg_sum50((long long)hs.s_lo, W);
+    const long long c1 = sizeof(T) == 8 ? seg_sum50((long long)hs.s_hi, W) : 0;
+    const long long c2 = seg_sum50((long long)hs.x_lo, W);
+    const long long c3 = sizeof(T) == 8 ? seg_sum50((long long)hs.x_hi, W) : 0;
     flag = TypeTraits<T>::is_signed ? seg_or_u32(flag, W) : seg_max_u32(flag, W);
     if ((tid & (W - 1)) == 0) {
       s_acc[seg][0] = c0;
@@ -503,10 +502,10 @@ choose_lengths_kernel(const __grid_constant__ FixedCompressArgs a) {
     HalfSums<T> hs;
     uint32_t flag = 0;
     cg_sums<T>(row, 32 * lane, hs, flag);
-    const long long c0 = seg_sum48((long long)hs.s_lo, 32);
-    const long long c1 = sizeof(T) == 8 ? seg_sum48((long long)hs.s_hi, 32) : 0;
-    const long long c2 = seg_sum48((long long)hs.x_lo, 32);
-    const long long c3 = sizeof(T) == 8 ? seg_sum48((long long)hs.x_hi, 32) : 0;
+    const long long c0 = seg_sum50((long long)hs.s_lo, 32);
+    const long long c1 = sizeof(T) == 8 ? seg_sum50((long long)hs.s_hi, 32) : 0;
+    const long long c2 = seg_sum50((long long)hs.x_lo, 32);
+    const long long c3 = sizeof(T) == 8 ? seg_sum50((long long)hs.x_hi, 32) : 0;
     flag = TypeTraits<T>::is_signed ? seg_or_u32(flag, 32) : seg_max_u32(flag, 32);
     if (lane == 0) {
       s_acc[warp][0] = c0;

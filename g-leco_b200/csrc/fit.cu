@@ -572,8 +572,8 @@ fit_short_kernel(const T* __restrict__ values, const int32_t* __restrict__ unit_
     over |= overflows_double<T>(y);
   });
   // (32 values a thread, j < 2^13, 32-bit halves: partials below 2^50)
-  const long long c0 = seg_sum48((long long)hs.s_lo, 32), c1 = sizeof(T) == 8 ? seg_sum48((long long)hs.s_hi, 32) : 0;
-  const long long c2 = seg_sum48((long long)hs.x_lo, 32), c3 = sizeof(T) == 8 ? seg_sum48((long long)hs.x_hi, 32) : 0;
+  const long long c0 = seg_sum50((long long)hs.s_lo, 32), c1 = sizeof(T) == 8 ? seg_sum50((long long)hs.s_hi, 32) : 0;
+  const long long c2 = seg_sum50((long long)hs.x_lo, 32), c3 = sizeof(T) == 8 ? seg_sum50((long long)hs.x_hi, 32) : 0;
   over = __any_sync(FULL_MASK, over);
   if (lane == 0) {
     s_acc[warp][0] = c0;

@@ -89,9 +89,10 @@ constexpr double kHalfBias = 0x1.fffffffffffffp-2;    // 0.5 - 2^-54
 // low 32 bits (the low bits of (y - pred) + K), which is all the packing of a width <= 31 reads.
 enum : int { CF_DIRECT = 0, CF_NONNEG = 1, CF_NONPOS = 2, CF_GENERAL = 3, CF_OFFSET = 4 };
 
-// Exact sum over a reduction segment of W lanes (32, or 16 at L = 256) of values |v| < 2^48: for a
-// whole warp two redux sums of the 24-bit limbs (each limb's sum stays below 2^29).
-__device__ __forceinline__ long long seg_sum48(long long v, int W) {
+// Exact sum over a reduction segment of W lanes (32; 16 where a partition is 16 groups, 8 where it is
+// eight): for a whole warp two redux sums of 24-bit limbs.  Any |v| < 2^50 will do: 32 low limbs stay
+// below 2^29, 32 high limbs (below 2^26 each) below 2^31.
+__device__ __forceinline__ long long seg_sum50(long long v, int W) {
   if (W == 32) {
     const unsigned lo = __reduce_add_sync(FULL_MASK, (unsigned)v & 0xFFFFFFu);
     const int hi = __reduce_add_sync(FULL_MASK, (int)(v >> 24));

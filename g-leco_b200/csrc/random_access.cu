@@ -67,8 +67,8 @@ __device__ __forceinline__ uint64_t read_field_global(const uint32_t* __restrict
 
 // A descriptor is one 32-byte access (the arrays are 32-byte aligned): a warp's lookups land on
 // different lines, so every access costs the L1 a tag lookup per lane, and two 16-byte halves cost
-// two (100M lookups into 64M int64 values: 1038 -> 942 us).  The field's words stay with 16 bytes:
-// its whole sector in one access measured slower (997 us).
+// two (100M lookups into 64M int64 values: 1064 -> 1019 us a call).  The field's words stay with 16
+// bytes: its whole sector in one access measured 5 % slower.
 __device__ __forceinline__ PartDesc load_desc(const PartDesc* __restrict__ d) {
   const Bytes32 x = load32_nc(d);
   PartDesc r;
@@ -212,8 +212,11 @@ cudaError_t launch_random_access(glc_ctx* ctx, const glc_column* c, int plain_sr
                                  void* out, int32_t fixed_len, cudaStream_t s) {
   const char* v = getenv("GLC_RA_SHAPE");
   // A call that one lookup per thread spreads over no more than two CTAs per SM gains nothing from
-  // several lookups in a thread: their searches run one after another (10,007 lookups into a
-  // variable column: 6.8 us in shape 0, 3.3 in shape 5).
+  // several lookups in a thread: their searches run one after another.  Calls back to back in shape 0 /
+  // 4 / 5, into 30M-value columns: variable 10,000 lookups 8.2 / 6.2 / 4.8 us, 75,000 the same, 150,000
+  // 8.2 / 6.2 / 6.1, 600,000 10.3 each; fixed 75,000 6.2 / 4.8 / 4.8, 300,000 8.2 / 6.2 / 6.2.  Beyond the
+  // line shape 5 is never far ahead of the tuned one, and pre-unpacked columns lose by it (600,000: 9.7
+  // / 10.2 / 10.3, shape 3 9.5).
   const bool small = q <= 2ll * kRAThreads * ctx->num_sms;
   const int shape = (v && *v) ? atoi(v) : small ? 5 : tune_entry(ctx, c->dtype, c->max_bits, plain_src).ra_shape;
   return launch_random_access_shape(ctx, c, plain_src, pos, q, out, fixed_len, shape, s);
